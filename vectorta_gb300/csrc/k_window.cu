@@ -1015,32 +1015,25 @@ __global__ void k_percentile(PnrArgs a) {
     const int c0 = blockIdx.y * kPnrChunk;
     const int c1 = min(c0 + kPnrChunk, a.n);
     if (c0 >= a.n) return;
-    // windows of at most 64 values: the register window, sized by the
-    // warp's longest window (warp-uniform); longer ones: the sorted array
-    {
-        const bool live = li < a.n_lanes;
-        const int len = live ? (a.layout == 0 ? a.lengths[li] : a.length) : 1;
-        const int wmax = __reduce_max_sync(0xffffffffu, len);
-        if (wmax <= 64) {
-            const int u0 = max(0, c0 - wmax + 1);
-            const float* x = a.layout == 0 ? a.x : a.x + (live ? li : 0);
-            const size_t stride = a.layout == 0 ? 1 : (size_t)a.cols;
-            const int f = a.layout == 0 ? a.first : (live ? a.first_tm[li] : 0);
-            const double pf = a.layout == 0 ? (live ? (double)a.pfrac[li] : 0.5) : (double)a.p_frac;
-            float* out = a.layout == 0 ? a.out + (size_t)(live ? li : 0) * a.n : a.out + (live ? li : 0);
-            const size_t ostride = a.layout == 0 ? 1 : (size_t)a.cols;
-            if (!live) return;  // after the warp-wide reduction
-            switch ((wmax + 7) / 8) {
-                case 1: case 2: pnr_lane_reg<16>(x, stride, f, len, pf, c0, c1, u0, out, ostride); break;
-                case 3: pnr_lane_reg<24>(x, stride, f, len, pf, c0, c1, u0, out, ostride); break;
-                case 4: pnr_lane_reg<32>(x, stride, f, len, pf, c0, c1, u0, out, ostride); break;
-                case 5: pnr_lane_reg<40>(x, stride, f, len, pf, c0, c1, u0, out, ostride); break;
-                case 6: pnr_lane_reg<48>(x, stride, f, len, pf, c0, c1, u0, out, ostride); break;
-                case 7: pnr_lane_reg<56>(x, stride, f, len, pf, c0, c1, u0, out, ostride); break;
-                default: pnr_lane_reg<64>(x, stride, f, len, pf, c0, c1, u0, out, ostride); break;
-            }
-            return;
+    // time-major windows of at most 64 values: the register window
+    if (a.layout != 0 && a.length <= 64) {
+        if (li >= a.n_lanes) return;
+        const int len = a.length, u0 = max(0, c0 - len + 1);
+        const float* x = a.x + li;
+        const size_t stride = (size_t)a.cols;
+        const int f = a.first_tm[li];
+        const double pf = (double)a.p_frac;
+        float* out = a.out + li;
+        switch ((len + 7) / 8) {
+            case 1: case 2: pnr_lane_reg<16>(x, stride, f, len, pf, c0, c1, u0, out, stride); break;
+            case 3: pnr_lane_reg<24>(x, stride, f, len, pf, c0, c1, u0, out, stride); break;
+            case 4: pnr_lane_reg<32>(x, stride, f, len, pf, c0, c1, u0, out, stride); break;
+            case 5: pnr_lane_reg<40>(x, stride, f, len, pf, c0, c1, u0, out, stride); break;
+            case 6: pnr_lane_reg<48>(x, stride, f, len, pf, c0, c1, u0, out, stride); break;
+            case 7: pnr_lane_reg<56>(x, stride, f, len, pf, c0, c1, u0, out, stride); break;
+            default: pnr_lane_reg<64>(x, stride, f, len, pf, c0, c1, u0, out, stride); break;
         }
+        return;
     }
     if (li >= a.n_lanes) return;
     float local[kPnrLocal];

@@ -1183,35 +1183,45 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
             return VTA_OK;
         }
         case I_PNR: {
-            const int nchunk = (n + 255) / 256;
-            const size_t sc = pmax > 64 ? (size_t)nchunk * nc * pmax : 0;
+            // p_frac = percentage * 0.01 (percentile_nearest_rank.rs:213)
+            for (int i = 0; i < nc; ++i) fa[i] = (float)(cs[i].a * 0.01);
+            // the rank-bitmap sweep up to its longest window (3,841 values),
+            // one sorted array per thread in scratch memory past it
+            const bool ranks = pnr_sweep_ok(n, pmax);
+            PnrPlan plan;
+            if (ranks) plan = pnr_plan(n, periods, fa, ctx->num_sms);
+            const size_t sc = ranks ? plan.work_bytes / sizeof(float) : (size_t)((n + 255) / 256) * nc * pmax;
             ar.need(sc * sizeof(float));
+            ar.need(plan.items.size() * sizeof(int4));
+            ar.need(plan.runs.size() * sizeof(int2));
             VTA_TRY(ar.commit());
-            int* d_per = ar.take<int>(nc);
-            ar.take<double>(nc);
-            ar.take<double>(nc);
-            float* d_fa = ar.take<float>(nc);
-            ar.take<float>(nc);
-            float* d_sc = sc ? ar.take<float>(sc) : nullptr;
-            std::vector<float> pf(nc);
-            // p_frac = percentage * 0.01 in f64 (percentile_nearest_rank.rs:213)
-            std::vector<double> pfd(nc);
-            for (int i = 0; i < nc; ++i) pf[i] = (float)(cs[i].a * 0.01);
-            VTA_TRY(upload(ctx, d_per, periods.data(), nc * sizeof(int)));
-            VTA_TRY(upload(ctx, d_fa, pf.data(), nc * sizeof(float)));
             PnrArgs a{};
             a.layout = 0;
             a.x = in.p[0];
             a.n = n;
             a.first = (int)first;
-            a.lengths = d_per;
-            a.pfrac = d_fa;
             a.length = pmax;
             a.n_lanes = nc;
             a.out = out[0];
-            a.scratch = d_sc;
-            ctx->last_kernel = "percentile_sorted_window";
-            return launch_percentile(a, st);
+            const int4* d_items = nullptr;
+            const int2* d_runs = nullptr;
+            int* per_slot = ar.take<int>(nc);
+            ar.take<double>(nc);
+            ar.take<double>(nc);
+            float* fa_slot = ar.take<float>(nc);
+            ar.take<float>(nc);
+            a.scratch = ar.take<float>(sc);
+            if (plan.grow) {
+                int4* item_slot = ar.take<int4>(plan.items.size());
+                VTA_TRY(const_upload(ctx, plan.items.data(), plan.items.size(), item_slot, &d_items));
+                VTA_TRY(const_upload(ctx, plan.runs.data(), plan.runs.size(), ar.take<int2>(plan.runs.size()), &d_runs));
+            } else {
+                VTA_TRY(const_upload(ctx, periods.data(), nc, per_slot, &a.lengths));
+                VTA_TRY(const_upload(ctx, fa.data(), nc, fa_slot, &a.pfrac));
+            }
+            ctx->last_kernel = !ranks ? "percentile_sorted_window"
+                             : plan.grow ? "percentile_ranks_grow" : "percentile_ranks_slide";
+            return ranks ? launch_pnr_sweep(a, plan, d_items, d_runs, ctx->num_sms, st) : launch_percentile(a, st);
         }
         default:
             return fail(VTA_ERR_NOT_IMPLEMENTED, "indicator not implemented");

@@ -509,6 +509,20 @@ struct PnrArgs {
     size_t scratch_floats;
 };
 vta_status launch_percentile(const PnrArgs& a, cudaStream_t st);
+// Batch sweeps whose longest window fits the rank bitmap (k_percentile.cu):
+// how a sweep runs, with the growing walk's work list (empty for the sliding one).
+struct PnrPlan {
+    bool grow = false;
+    int lmax = 0;
+    size_t work_bytes = 0;     // PnrArgs::scratch
+    std::vector<int4> items;   // by percentage and length: {length, row, full-window rank, f32 bits of the fraction}
+    std::vector<int2> runs;    // item ranges walked by one block each
+};
+bool pnr_sweep_ok(int n, int lmax);
+PnrPlan pnr_plan(int n, const std::vector<int>& lengths, const std::vector<float>& pfrac, int num_sms);
+// items / runs: the plan's lists on the device
+vta_status launch_pnr_sweep(const PnrArgs& a, const PnrPlan& plan, const int4* items, const int2* runs, int num_sms,
+                            cudaStream_t st);
 
 // One ATR (0) / ADX (1) / SuperTrend (2) / percentile (3) job of the plan
 // kernels over a rectangular time-major matrix, enqueued on st (vta_plan.cu).
