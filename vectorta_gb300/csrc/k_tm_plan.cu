@@ -290,49 +290,10 @@ __global__ void k_tm_fixup(PlanArgs a) {
     }
 }
 
-// First valid index per series within its own length: close alone and
-// high, low and close together (len[s] when there is none).
-// First valid row of each series: close alone (percentile) and high, low and
-// close together (the high/low/close jobs).  Rows are examined kFirstRows at a
-// time; the block's loads are all issued before any is tested (rows clamped
-// into the series, no short-circuit), so the NaN lead costs few memory round
-// trips.
-constexpr int kFirstRows = 16;
-
-__global__ void k_plan_first(PlanArgs a, int* first_hlc, int* first_c) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.cols) return;
-    const int L = a.len[s];
-    const TmIn in{a.h, a.l, a.c, (size_t)a.cols, (size_t)s};
-    int fc = L, fh = L;
-    for (int t0 = 0; t0 < L && fh == L; t0 += kFirstRows) {
-        float hv[kFirstRows], lv[kFirstRows], cv[kFirstRows];
-#pragma unroll
-        for (int j = 0; j < kFirstRows; ++j) {
-            const int t = min(t0 + j, L - 1);
-            cv[j] = in.C(t);
-            hv[j] = in.H(t);
-            lv[j] = in.L(t);
-        }
-        int bc = L, bh = L;  // first hit of this block
-#pragma unroll
-        for (int j = kFirstRows - 1; j >= 0; --j) {
-            const bool okc = (t0 + j < L) & !isnan(cv[j]);
-            if (okc) bc = t0 + j;
-            if (okc & !isnan(hv[j]) & !isnan(lv[j])) bh = t0 + j;
-        }
-        if (fc == L) fc = bc;
-        fh = bh;
-    }
-    first_c[s] = fc;
-    first_hlc[s] = fh;
-}
-
 }  // namespace
 
 vta_status launch_plan_first(const PlanArgs& a, int* first_hlc, int* first_c, cudaStream_t st) {
-    k_plan_first<<<(a.cols + 127) / 128, 128, 0, st>>>(a, first_hlc, first_c);
-    return check_launch("k_plan_first");
+    return launch_first_valid_tm_hlc(a.h, a.l, a.c, a.cols, a.rows, first_hlc, st, a.len, first_c);
 }
 
 int tm_plan_blocks(int num_sms) {

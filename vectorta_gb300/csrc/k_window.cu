@@ -437,13 +437,13 @@ k_prefix_window_batch(PrefixWinArgs a, int pmax, int cpb) {
 // ---------------------------------------------- prefix windows, time-major -
 constexpr int kTmChunk = 512;
 
-__global__ void k_prefix_window_tm(PrefixWinTmArgs a, const int* first_nan) {
+__global__ void k_prefix_window_tm(PrefixWinTmArgs a) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.cols) return;
     const int c0 = blockIdx.y * kTmChunk;
     const int c1 = min(c0 + kTmChunk, a.rows);
     const int f = a.first[s];
-    const int fn = first_nan[s];
+    const int fn = a.first_nan[s];
     const int p = a.period;
     const int warm = f + p - 1;
     const size_t S = a.cols;
@@ -481,16 +481,6 @@ __global__ void k_prefix_window_tm(PrefixWinTmArgs a, const int* first_nan) {
         a.out0[o] = r.o0;
         if (a.kind == WK_BB) { a.out1[o] = r.o1; a.out2[o] = r.o2; }
     }
-}
-
-// First NaN strictly after the first valid index, per time-major series.
-__global__ void k_first_nan_after_tm(const float* __restrict__ x, int cols, int rows,
-                                     const int* first, int* out) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= cols) return;
-    int t = first[s] + 1;
-    while (t < rows && !isnan(x[(size_t)t * cols + s])) ++t;
-    out[s] = t < rows ? t : rows;
 }
 
 // ------------------------------------------------- min/max, batch ----------
@@ -1098,14 +1088,10 @@ vta_status launch_prefix_window_batch(const PrefixWinArgs& a, int pmax, size_t s
     return check_launch("k_prefix_window_batch");
 }
 
-// first_nan scratch is carved by the caller right after `first`
 vta_status launch_prefix_window_tm(const PrefixWinTmArgs& a, cudaStream_t st) {
-    int* first_nan = const_cast<int*>(a.first) + a.cols;
-    k_first_nan_after_tm<<<ceil_div(a.cols, 128), 128, 0, st>>>(a.x_tm, a.cols, a.rows, a.first, first_nan);
-    VTA_TRY(check_launch("k_first_nan_after_tm"));
     dim3 grid(ceil_div(a.cols, 128), ceil_div(a.rows, kTmChunk));
     ktimer_begin(st);
-    k_prefix_window_tm<<<grid, 128, 0, st>>>(a, first_nan);
+    k_prefix_window_tm<<<grid, 128, 0, st>>>(a);
     ktimer_end(st);
     return check_launch("k_prefix_window_tm");
 }

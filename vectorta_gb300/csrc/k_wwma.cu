@@ -115,7 +115,7 @@ k_wwma_batch_plain(WwmaBatchArgs a) {
 constexpr int kTmT = 8;
 constexpr int kTmTiles = 8;  // tiles of 8 times per thread
 
-__global__ void k_wwma_tm(WwmaTmArgs a, const int* first_nan) {
+__global__ void k_wwma_tm(WwmaTmArgs a) {
     extern __shared__ float wsm[];
     for (int i = threadIdx.x; i < a.period; i += blockDim.x) wsm[i] = a.w[i];
     __syncthreads();
@@ -123,7 +123,7 @@ __global__ void k_wwma_tm(WwmaTmArgs a, const int* first_nan) {
     if (s >= a.cols) return;
     const size_t S = a.cols;
     const int p = a.period, f = a.first[s];
-    const int fn = first_nan ? first_nan[s] : a.rows;
+    const int fn = a.first_nan ? a.first_nan[s] : a.rows;
     for (int tile = 0; tile < kTmTiles; ++tile) {
         const int t0 = (blockIdx.y * kTmTiles + tile) * kTmT;
         if (t0 >= a.rows) return;
@@ -157,15 +157,6 @@ __global__ void k_wwma_tm(WwmaTmArgs a, const int* first_nan) {
     }
 }
 
-__global__ void k_first_nan_tm(const float* __restrict__ x, int cols, int rows, const int* first,
-                               int* out) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= cols) return;
-    int t = first[s] + 1;
-    while (t < rows && !isnan(x[(size_t)t * cols + s])) ++t;
-    out[s] = t < rows ? t : rows;
-}
-
 }  // namespace
 
 vta_status launch_wwma_batch_plain(const WwmaBatchArgs& a, cudaStream_t st) {
@@ -182,22 +173,14 @@ vta_status launch_wwma_batch_plain(const WwmaBatchArgs& a, cudaStream_t st) {
     return check_launch("k_wwma_batch_plain");
 }
 
-// first_nan scratch (cols ints) is carved by the caller right after `first`
 vta_status launch_wwma_tm(const WwmaTmArgs& a, cudaStream_t st) {
-    const int* fn = nullptr;
-    if (a.nan_mode == 1) {
-        int* first_nan = const_cast<int*>(a.first) + a.cols;
-        k_first_nan_tm<<<ceil_div(a.cols, 128), 128, 0, st>>>(a.x_tm, a.cols, a.rows, a.first, first_nan);
-        VTA_TRY(check_launch("k_first_nan_tm"));
-        fn = first_nan;
-    }
     dim3 grid(ceil_div(a.cols, 128), ceil_div(a.rows, kTmT * kTmTiles));
     const size_t smem = (size_t)a.period * sizeof(float);
     if (smem > 227 * 1024) return fail(VTA_ERR_LAUNCH_CONFIG_TOO_LARGE, "wwma tm: period too large");
     if (smem > 48 * 1024)
         VTA_CUDA_TRY(cudaFuncSetAttribute(k_wwma_tm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ktimer_begin(st);
-    k_wwma_tm<<<grid, 128, smem, st>>>(a, fn);
+    k_wwma_tm<<<grid, 128, smem, st>>>(a);
     ktimer_end(st);
     return check_launch("k_wwma_tm");
 }

@@ -1275,7 +1275,11 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
     double* d_ab = ar.take<double>(2);
     float* d_sc = pnr_sc ? ar.take<float>(pnr_sc) : nullptr;
 
-    if (kInfo[ind].in == IN_X) VTA_TRY(launch_first_valid_tm(in.p[0], C, R, d_first, st));
+    // the running-sum kinds hold a series' NaN for ever: they need its first one
+    const bool sums = ind == I_SMA || ind == I_STDDEV || ind == I_ZSCORE || ind == I_BB;
+    const bool wsums = ind == I_WMA || ind == I_SWMA || ind == I_TRIMA;
+    int* d_first_nan = sums || wsums ? d_first + C : nullptr;
+    if (kInfo[ind].in == IN_X) VTA_TRY(launch_first_valid_tm(in.p[0], C, R, d_first, st, d_first_nan));
     else if (ind == I_DONCHIAN) VTA_TRY(launch_first_valid_tm_hlc(in.p[0], in.p[1], in.p[1], C, R, d_first, st));
     else VTA_TRY(launch_first_valid_tm_hlc(in.p[0], in.p[1], in.p[2], C, R, d_first, st));
 
@@ -1296,7 +1300,8 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
         a.w = d_w;
         a.period = pw;
         a.warm_extra = wwma_warm_extra(ind, c);
-        a.nan_mode = (ind == I_WMA || ind == I_SWMA || ind == I_TRIMA) ? 1 : 0;
+        a.nan_mode = wsums ? 1 : 0;
+        a.first_nan = d_first_nan;
         a.out_tm = out[0];
         ctx->last_kernel = "wwma_tm_f32";
         return launch_wwma_tm(a, st);
@@ -1343,6 +1348,7 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
             a.cols = C;
             a.rows = R;
             a.first = d_first;
+            a.first_nan = d_first_nan;
             a.period = p;
             a.k1 = (float)c.a;
             a.k2 = (float)c.b;

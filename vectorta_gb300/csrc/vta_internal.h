@@ -189,10 +189,15 @@ inline unsigned ceil_div(size_t a, size_t b) { return (unsigned)((a + b - 1) / b
 // Every launcher enqueues on `st` and returns the launch status.
 
 // First valid (non-NaN) index of each time-major series; rows if all NaN.
-vta_status launch_first_valid_tm(const float* x_tm, int cols, int rows, int* first, cudaStream_t st);
+// first_nan (may be null): the first NaN after it; rows if there is none.
+vta_status launch_first_valid_tm(const float* x_tm, int cols, int rows, int* first, cudaStream_t st,
+                                 int* first_nan = nullptr);
 // Same over the three HLC inputs (first index where all three are non-NaN).
+// len (may be null): per-series lengths in place of rows; first_c (may be
+// null): the first valid index of c alone.
 vta_status launch_first_valid_tm_hlc(const float* h, const float* l, const float* c, int cols,
-                                     int rows, int* first, cudaStream_t st);
+                                     int rows, int* first, cudaStream_t st, const int* len = nullptr,
+                                     int* first_c = nullptr);
 
 // Inclusive f64 prefix of f(x[i]) for i >= first (0 before first), with
 // f selected by `kind`; optionally packed to double-single float2.
@@ -243,6 +248,7 @@ struct WwmaTmArgs {
     int period;            // window length
     int warm_extra;        // first output of series s at first[s] + period - 1 + warm_extra
     int nan_mode;
+    const int* first_nan;  // nan_mode 1: first NaN after first[s] (rows: none)
     float* out_tm;
 };
 vta_status launch_wwma_tm(const WwmaTmArgs& a, cudaStream_t st);
@@ -443,6 +449,7 @@ struct PrefixWinTmArgs {
     const float* x_tm;
     int cols, rows;
     const int* first;
+    const int* first_nan;  // first NaN after first[s] (rows: none)
     int period;
     float k1, k2;
     float* out0;
