@@ -69,3 +69,22 @@ def test_periods(name, period):
     # running-sum NaN rule there)
     c, h, l = matrix(35, 700, seed=90, gaps=name in GAPS and (name, period) != ("sma", 1))
     check(name, c, h, l, dict(PARAMS[name], period=period))
+
+
+@pytest.mark.parametrize("name", ["sma", "stddev", "bollinger_bands"])
+def test_overflowing_values_poison_alike(name):
+    """The running sums restart every 512 rows; shorter chunks (few series)
+    poison the same outputs after an infinite or overflowing value as 512-row
+    chunks (many series) do."""
+    c, _, _ = matrix(32, 1029, seed=7, gaps=False)
+    for j, v in enumerate([np.inf, -np.inf, 3e38, 2e19, 1e30]):
+        c[400 + 70 * j, 3 * j] = v
+        c[511 + j, 3 * j + 1] = v
+    prm = dict(PARAMS[name], period=20)
+    few = run(name, c, c, c, prm)
+    many = run(name, np.tile(c, (1, 1600)), None, None, prm)
+    for a, b in zip(few, many):
+        b = b[:, :32]
+        assert np.array_equal(np.isnan(a), np.isnan(b))
+        ok = np.isfinite(b) & (np.abs(b) < 1e6)
+        assert np.allclose(a[ok], b[ok], rtol=1e-5, atol=1e-4 * (name != "sma"))

@@ -29,7 +29,7 @@ constexpr int kFvWarps = 32, kFvRows = 8;
 template <bool ALL>
 __global__ void __launch_bounds__(32 * kFvWarps)
 k_first_valid_tm(const float* __restrict__ h, const float* __restrict__ l, const float* __restrict__ c, int cols,
-                 int rows, const int* len, int* first, int* first_c, int* first_nan) {
+                 int rows, const int* len, int* first, int* first_c, int* first_nan, int* first_big) {
     __shared__ int fa[32], fc[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int s = blockIdx.x * 32 + lane;
@@ -66,35 +66,41 @@ k_first_valid_tm(const float* __restrict__ h, const float* __restrict__ l, const
         first[s] = fa[lane];
         if (first_c) first_c[s] = fc[lane];
         if (first_nan) first_nan[s] = rows;
+        if (first_big) first_big[s] = rows;
     }
 }
 
-// First NaN after each series' first valid row: first_nan[s] holds `rows` (set
-// by k_first_valid_tm) and is lowered to the row.  Blocks of 128 series x 64
-// rows read the whole matrix once (one thread per series walking its rows took
-// 1,073 us for 3,000 x 2,520; now 9).
+// First NaN after each series' first valid row, and first value of magnitude
+// above 2^60 (infinite ones too): first_nan[s] and first_big[s] (may be null)
+// hold `rows` (set by k_first_valid_tm) and are lowered to the row.  Blocks of
+// 128 series x 64 rows read the whole matrix once (one thread per series
+// walking its rows took 1,073 us for 3,000 x 2,520; now 11).
 constexpr int kFnRows = 64, kFnBatch = 16;
 
 __global__ void __launch_bounds__(128)
-k_first_nan_tm(const float* __restrict__ x, int cols, int rows, const int* __restrict__ first, int* first_nan) {
+k_first_nan_tm(const float* __restrict__ x, int cols, int rows, const int* __restrict__ first, int* first_nan,
+               int* first_big) {
     const int s = blockIdx.x * 128 + threadIdx.x;
     if (s >= cols) return;
     const int f = first[s];
-    int found = rows;
+    int found = rows, big = rows;
     for (long long t0 = (long long)blockIdx.y * kFnRows; t0 < rows; t0 += (long long)gridDim.y * kFnRows) {
         const int t1 = (int)min(t0 + kFnRows, (long long)rows);
-        if (t1 - 1 <= f) continue;
+        if (t1 - 1 < f) continue;
         for (int tb = (int)t0; tb < t1; tb += kFnBatch) {
             const int m = t1 - tb;
             float v[kFnBatch];
 #pragma unroll
             for (int j = 0; j < kFnBatch; ++j) v[j] = __ldg(x + (size_t)(tb + min(j, m - 1)) * cols + s);
 #pragma unroll
-            for (int j = 0; j < kFnBatch; ++j)
+            for (int j = 0; j < kFnBatch; ++j) {
                 if (j < m && tb + j > f && isnan(v[j])) found = min(found, tb + j);
+                if (j < m && fabsf(v[j]) > 0x1p60f) big = min(big, tb + j);
+            }
         }
     }
     if (found < rows) atomicMin(first_nan + s, found);
+    if (first_big && big < rows) atomicMin(first_big + s, big);
 }
 
 __device__ __forceinline__ double prefix_value(const float* x, int i, int first, int kind) {
@@ -212,20 +218,20 @@ __global__ void k_prefix_apply(const float* __restrict__ x, int n, int first, in
 }  // namespace
 
 vta_status launch_first_valid_tm(const float* x_tm, int cols, int rows, int* first, cudaStream_t st,
-                                 int* first_nan) {
+                                 int* first_nan, int* first_big) {
     k_first_valid_tm<false><<<ceil_div(cols, 32), 32 * kFvWarps, 0, st>>>(nullptr, nullptr, x_tm, cols, rows, nullptr,
-                                                                         first, nullptr, first_nan);
+                                                                         first, nullptr, first_nan, first_big);
     VTA_TRY(check_launch("k_first_valid_tm"));
     if (!first_nan) return VTA_OK;
     const unsigned ny = std::min(ceil_div(rows, kFnRows), 65535u);
-    k_first_nan_tm<<<dim3(ceil_div(cols, 128), ny), 128, 0, st>>>(x_tm, cols, rows, first, first_nan);
+    k_first_nan_tm<<<dim3(ceil_div(cols, 128), ny), 128, 0, st>>>(x_tm, cols, rows, first, first_nan, first_big);
     return check_launch("k_first_nan_tm");
 }
 
 vta_status launch_first_valid_tm_hlc(const float* h, const float* l, const float* c, int cols,
                                      int rows, int* first, cudaStream_t st, const int* len, int* first_c) {
     k_first_valid_tm<true><<<ceil_div(cols, 32), 32 * kFvWarps, 0, st>>>(h, l, c, cols, rows, len, first, first_c,
-                                                                        nullptr);
+                                                                        nullptr, nullptr);
     return check_launch("k_first_valid_tm_hlc");
 }
 

@@ -1250,7 +1250,7 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
                               ind == I_SUPERTREND ? out[1] : nullptr, st);
     }
     Arena ar(ctx);
-    ar.need(2 * cols * sizeof(int));  // first + first_nan
+    ar.need(3 * cols * sizeof(int));  // first, first_nan, first_big
     const bool recur = ind == I_EMA || ind == I_DEMA || ind == I_TEMA || ind == I_RSI || ind == I_WILDERS ||
                        ind == I_ATR;
     int chunk = 0, nch = 0;
@@ -1267,7 +1267,7 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
     const size_t pnr_sc = (ind == I_PNR && p > 64) ? (size_t)((R + 255) / 256) * cols * p : 0;
     ar.need(pnr_sc * sizeof(float));
     VTA_TRY(ar.commit());
-    int* d_first = ar.take<int>(2 * cols);
+    int* d_first = ar.take<int>(3 * cols);
     float* d_agg = recur ? ar.take<float>((size_t)nch * cols * 4) : nullptr;
     float* d_carry = recur ? ar.take<float>((size_t)nch * cols * 4) : nullptr;
     float* d_w = ar.take<float>(pw);
@@ -1279,7 +1279,8 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
     const bool sums = ind == I_SMA || ind == I_STDDEV || ind == I_ZSCORE || ind == I_BB;
     const bool wsums = ind == I_WMA || ind == I_SWMA || ind == I_TRIMA;
     int* d_first_nan = sums || wsums ? d_first + C : nullptr;
-    if (kInfo[ind].in == IN_X) VTA_TRY(launch_first_valid_tm(in.p[0], C, R, d_first, st, d_first_nan));
+    int* d_first_big = sums ? d_first_nan + C : nullptr;
+    if (kInfo[ind].in == IN_X) VTA_TRY(launch_first_valid_tm(in.p[0], C, R, d_first, st, d_first_nan, d_first_big));
     else if (ind == I_DONCHIAN) VTA_TRY(launch_first_valid_tm_hlc(in.p[0], in.p[1], in.p[1], C, R, d_first, st));
     else VTA_TRY(launch_first_valid_tm_hlc(in.p[0], in.p[1], in.p[2], C, R, d_first, st));
 
@@ -1349,13 +1350,14 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
             a.rows = R;
             a.first = d_first;
             a.first_nan = d_first_nan;
+            a.first_big = d_first_big;
             a.period = p;
             a.k1 = (float)c.a;
             a.k2 = (float)c.b;
             a.out0 = out[0];
             if (ind == I_BB) { a.out1 = out[1]; a.out2 = out[2]; }
             ctx->last_kernel = "prefix_window_tm";
-            return launch_prefix_window_tm(a, st);
+            return launch_prefix_window_tm(a, ctx->num_sms, st);
         }
         case I_DONCHIAN: case I_WILLR: {
             MinMaxTmArgs a{};
