@@ -358,6 +358,22 @@ static int pick_chunk(vta_ctx* ctx, int n, int lanes, int warps_per_sm = 64) {
     return (int)len;
 }
 
+// Time-major: the chunks are latency-bound while they leave warp slots free, so
+// 32 rows as long as that makes at most 64 warps per SM, 64 up to 128, else
+// 128 (us at 32 / 64 / 128 / 256 rows: RSI(14) of 3,000 series x 2,520 rows 62
+// / 76 / 110 / 116, 500 x 60,000 151 / 120 / 134 / 146; EMA(20) of 20,000 x
+// 1,000 95 / 91 / 105 / 123).
+static int pick_chunk_tm(vta_ctx* ctx, int rows, int cols) {
+    const int pol = ctx->policy.recur_chunk;
+    if (pol == 1) return ((rows + 31) / 32) * 32;
+    if (pol > 1) return pol;
+    const long lane_warps = (cols + 31) / 32;
+    auto warps_per_sm = [&](long len) { return lane_warps * ((rows + len - 1) / len) / ctx->num_sms; };
+    long len = warps_per_sm(32) <= 64 ? 32 : warps_per_sm(64) <= 128 ? 64 : 128;
+    while ((rows + len - 1) / len > 65535) len *= 2;
+    return (int)len;
+}
+
 // ------------------------------------------------------ sweep autotuner ---
 // The launch knobs of the batch sweeps are picked by timing: the first call
 // with a new (indicator, log2 length, log2 sweep size, knob) runs the sweep
@@ -1255,7 +1271,7 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
                        ind == I_ATR;
     int chunk = 0, nch = 0;
     if (recur) {
-        chunk = pick_chunk(ctx, R, C);
+        chunk = pick_chunk_tm(ctx, R, C);
         nch = (R + chunk - 1) / chunk;
         ar.need((size_t)nch * cols * 16);
         ar.need((size_t)nch * cols * 16);
