@@ -71,11 +71,13 @@ __device__ __forceinline__ float adx_dx_wide(float pdm, float mdm) {
     return fabsf(pdm - mdm) * rcp_approx_ftz(pdm + mdm) * 100.f;
 }
 
+// (Selects, no branches: the unrolled steps of a batch then form one block of
+// code whose divisions overlap.)
 __device__ __forceinline__ float adx_dx(float pdm, float mdm, float atr) {
-    if (atr == 0.f) return 0.f;
     const float s = pdm + mdm;
-    const float d = s != 0.f ? __fdividef(fabsf(pdm - mdm), s) * 100.f : 0.f;
-    return atr == atr ? d : qnan();
+    const float q = __fdividef(fabsf(pdm - mdm), s) * 100.f;
+    const float d = atr == atr ? (s != 0.f ? q : 0.f) : qnan();
+    return atr == 0.f ? 0.f : d;
 }
 
 // ATR: atr_compute_into_scalar (atr.rs:329-460); TR(f) = h - l, seed = mean
@@ -340,16 +342,13 @@ struct PSuperTrend {
         float cub = fmaf(fac, atr, hl2), clb = fmaf(-fac, atr, hl2);
         if (last_close <= pub) cub = fminf(cub, pub);
         if (last_close >= plb) clb = fmaxf(clb, plb);
-        float v0;
-        if (upper) {
-            if (cl <= cub) { v0 = cub; v1 = 0.f; }
-            else { v0 = clb; v1 = 1.f; upper = false; }
-        } else {
-            if (cl >= clb) { v0 = clb; v1 = 0.f; }
-            else { v0 = cub; v1 = 1.f; upper = true; }
-        }
+        // the band holds or the trend flips to the other one (selects: see adx_dx)
+        const bool up = cl <= cub, down = cl >= clb;
+        const bool hold = upper ? up : down;
+        upper = upper == hold;
+        v1 = hold ? 0.f : 1.f;
         pub = cub; plb = clb; last_close = cl;
-        return v0;
+        return upper ? cub : clb;
     }
 };
 

@@ -1,11 +1,14 @@
 // Many-series work-list kernels: several indicators over one set of ragged
 // time-major OHLC series in one persistent launch.
 //
-// Work items are (job, tile of 32 consecutive series, time chunk).  A warp
-// takes items from a global counter; lane l of the warp owns series
-// 32 * tile + l, so every load and store of a time step is one coalesced
-// 128-byte row segment.  Series of uneven length stop at their own length:
-// cells past it are neither read nor written.
+// Work items are (job, time chunk, up to 32 of the series that reach the
+// chunk).  A warp takes items from a global counter; its lanes own consecutive
+// entries of the chunk's list of series, which are adjacent series as long as
+// all of them reach it (every load and store of a time step is then one
+// 128-byte row segment) and skip the ones that have ended after that: with
+// lengths spread over [1,000, 20,000] fixed tiles of 32 series left half the
+// lanes idle.  Series of uneven length stop at their own length: cells past it
+// are neither read nor written.
 //
 // Recurrent jobs (ATR, ADX, SuperTrend) are cut into time chunks with a
 // verified warm restart.  Chunk k (c0 = k * chunk) that starts past the
@@ -20,6 +23,7 @@
 // The percentile job is exact per chunk by construction (its window is
 // rebuilt from the `length` inputs before c0).
 #include <cfloat>
+#include <climits>
 
 #include "vta_internal.h"
 #include "vta_plan.h"
@@ -50,14 +54,16 @@ using pnr::pick;
 using pnr::rank;
 
 // ------------------------------------------------ chunk runners -------------
-// Inputs are staged per warp in shared memory: a double buffer of kPB steps
-// x {high, low, close} x 32 lanes, filled with cp.async (4 bytes per lane and
-// value, so each step of a warp is one 128-byte row segment).  Each lane
-// copies and reads only its own column, so no cross-lane synchronisation is
-// needed; while a block is computed the next one is in flight, so a warp
-// waits for memory about once per kPB steps instead of once per step.
-constexpr int kPB = 16;
-constexpr int kStageFloats = 2 * 3 * kPB * 32;  // per warp
+// Inputs are staged per warp in shared memory: a ring of kPS blocks of kPB
+// steps x {high, low, close} x 32 lanes, filled with cp.async (4 bytes per lane
+// and value, so each step of a warp is one 128-byte row segment when its
+// series are adjacent).  Each lane copies and reads only its own column, so no
+// cross-lane synchronisation is needed; kPS - 1 blocks are in flight while one
+// is computed (the recurrences take about 20 issue slots a step, far less than
+// a memory round trip per block).
+constexpr int kPB = 8;
+constexpr int kPS = 4;
+constexpr int kStageFloats = kPS * 3 * kPB * 32;  // per warp
 constexpr size_t kPlanSmem = (size_t)kPlanWarps * kStageFloats * sizeof(float);
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
@@ -66,48 +72,128 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
 struct Stage {
-    float* base;  // this warp's [2][3][kPB][32]
+    float* base;  // this warp's [kPS][3][kPB][32]
     int lane;
-    __device__ float* at(int buf, int arr, int j) const { return base + ((buf * 3 + arr) * kPB + j) * 32 + lane; }
-    // copies of steps [tb, min(tb + kPB, tend)) of the given arrays into `buf`
-    __device__ void load(int buf, const float* a0, const float* a1, const float* a2, size_t cols, size_t s,
-                         int tb, int tend) const {
-        for (int j = 0; j < kPB && tb + j < tend; ++j) {
-            const size_t g = (size_t)(tb + j) * cols + s;
-            if (a0) cp_async4(at(buf, 0, j), a0 + g);
-            if (a1) cp_async4(at(buf, 1, j), a1 + g);
-            if (a2) cp_async4(at(buf, 2, j), a2 + g);
-        }
-        cp_async_commit();
+    __device__ __forceinline__ float* at(int buf, int arr, int j) const {
+        return base + ((buf * 3 + arr) * kPB + j) * 32 + lane;
     }
 };
 
-// Steps t in [t, tend); with `emit` writes the outputs of each step.
+// A lane's seeding: its state at run_from() and the outputs of the step before
+// it (every op's first ones).  rf: run_from(), or kNever for a series too short
+// to be seeded, whose outputs are all NaN.
+constexpr int kNever = INT_MAX;
+struct Seed {
+    int rf;
+    float y0, y1;
+};
+
+// Runs the seeding steps [f, run_from()) of every lane of the warp, each on
+// rows of its own: the step index relative to f is the warp's, so the lanes
+// pass the op's phases together whatever their first valid rows are.
 template <class Op>
-__device__ void run_span(Op& op, const TmIn& in, const Stage& sg, int t, int tend, bool emit, float* out0,
-                         float* out1) {
-    if (t >= tend) return;
-    const int rf = op.run_from();  // from here on the running update alone
-    sg.load(0, in.h, in.l, in.c, in.cols, in.s, t, tend);
-    int buf = 0;
-    for (int tb = t; tb < tend; tb += kPB, buf ^= 1) {
-        // next block in flight (an empty group at the end keeps the count)
-        sg.load(buf ^ 1, in.h, in.l, in.c, in.cols, in.s, tb + kPB, tend);
-        cp_async_wait1();
-        const int te = min(tb + kPB, tend);
-        for (int tt = tb; tt < te; ++tt) {
-            const int j = tt - tb;
-            float o1;
-            const float hv = *sg.at(buf, 0, j), lv = *sg.at(buf, 1, j), cv = *sg.at(buf, 2, j);
-            const float o0 = tt >= rf ? op.step_run(hv, lv, cv, o1) : op.stepv(tt, hv, lv, cv, o1);
-            if (emit) {
-                out0[(size_t)tt * in.cols + in.s] = o0;
-                if (Op::kTwo) out1[(size_t)tt * in.cols + in.s] = o1;
+__device__ Seed run_seed(Op& op, const TmIn& in, int f, int L) {
+    const int n = op.run_from() - f;  // (the same for all lanes)
+    const bool ok = f < L && n <= L - f;
+    Seed sd{ok ? f + n : kNever, qnan(), qnan()};
+    op.start_exact();
+    for (int r = 0; r < n; r += kPB) {
+        float hv[kPB], lv[kPB], cv[kPB];
+#pragma unroll
+        for (int j = 0; j < kPB; ++j) {
+            const int t = ok ? f + min(r + j, n - 1) : 0;
+            hv[j] = in.H(t);
+            lv[j] = in.L(t);
+            cv[j] = in.C(t);
+        }
+#pragma unroll
+        for (int j = 0; j < kPB; ++j)
+            if (r + j < n) sd.y0 = op.stepv(f + r + j, hv[j], lv[j], cv[j], sd.y1);
+    }
+    return sd;
+}
+
+// Steps t in [t, tend) of each lane; EMIT writes the outputs of each step.  t
+// is the same for the lanes of `mask` (all call); they run in step to the
+// latest tend.  A lane takes part from its sd.rf on, and past its own tend
+// computes on without storing (its state is not read again: tend is either the
+// warp's or the end of the lane's series).
+template <bool EMIT, class Op>
+__device__ void run_span(Op& op, const TmIn& in, const Stage& sg, unsigned mask, const Seed& sd, int t, int tend,
+                         float* out0, float* out1) {
+    const int te = __reduce_max_sync(mask, tend);
+    const int rf = __reduce_max_sync(mask, sd.rf == kNever ? INT_MIN : sd.rf);
+    if (t >= te) return;
+    const size_t row0 = (size_t)t * in.cols + in.s;
+    const float *gh = in.h + row0, *gl = in.l + row0, *gc = in.c + row0;  // next row to load
+    int tl = t;
+    auto load = [&](int buf) {  // (an empty group past the end keeps the count)
+#pragma unroll
+        for (int j = 0; j < kPB; ++j) {
+            if (tl + j < tend) {
+                cp_async4(sg.at(buf, 0, j), gh + (size_t)j * in.cols);
+                cp_async4(sg.at(buf, 1, j), gl + (size_t)j * in.cols);
+                cp_async4(sg.at(buf, 2, j), gc + (size_t)j * in.cols);
             }
         }
+        tl += kPB;
+        gh += kPB * in.cols;
+        gl += kPB * in.cols;
+        gc += kPB * in.cols;
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int q = 0; q < kPS - 1; ++q) load(q);
+    float* o0 = out0 + row0;
+    float* o1 = Op::kTwo ? out1 + row0 : nullptr;
+    int buf = 0;
+    for (int tb = t; tb < te; tb += kPB, buf = (buf + 1) & (kPS - 1)) {
+        load((buf + kPS - 1) & (kPS - 1));
+        cp_async_wait<kPS - 1>();
+        float hv[kPB], lv[kPB], cv[kPB];
+#pragma unroll
+        for (int j = 0; j < kPB; ++j) {
+            hv[j] = *sg.at(buf, 0, j);
+            lv[j] = *sg.at(buf, 1, j);
+            cv[j] = *sg.at(buf, 2, j);
+        }
+        auto put = [&](int j, float y0, float y1) {
+            if (EMIT && tb + j < tend) {
+                o0[(size_t)j * in.cols] = y0;
+                if (Op::kTwo) o1[(size_t)j * in.cols] = y1;
+            }
+        };
+        const bool never = sd.rf == kNever;
+        if (tb >= rf && tb + kPB <= te) {
+#pragma unroll
+            for (int j = 0; j < kPB; ++j) {
+                float y1 = qnan();
+                const float y0 = op.step_run(hv[j], lv[j], cv[j], y1);
+                put(j, never ? qnan() : y0, never ? qnan() : y1);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < kPB; ++j) {
+                const int tt = tb + j;
+                if (tt >= te) break;
+                float y0 = qnan(), y1 = qnan();
+                if (tt >= sd.rf) {
+                    y0 = op.step_run(hv[j], lv[j], cv[j], y1);
+                } else if (tt == sd.rf - 1) {
+                    y0 = sd.y0;
+                    y1 = sd.y1;
+                }
+                put(j, y0, y1);
+            }
+        }
+        o0 += kPB * in.cols;
+        if (Op::kTwo) o1 += kPB * in.cols;
     }
 }
 
@@ -144,7 +230,7 @@ __device__ void pnr_chunk(const TmIn& in, const Stage& sg, unsigned mask, int f,
     int buf = 0;
     for (int ub = tbeg; ub < tend; ub += kPB, buf ^= 1) {
         load(buf ^ 1, ub + kPB);
-        cp_async_wait1();
+        cp_async_wait<1>();
         const int ue = min(ub + kPB, tend);
         for (int u = ub; u < ue; ++u) {
             const int j = u - ub, uo = u - len;
@@ -156,39 +242,48 @@ __device__ void pnr_chunk(const TmIn& in, const Stage& sg, unsigned mask, int f,
                 out[(size_t)u * in.cols + in.s] = u < start ? qnan() : pick(w, wl, len, kfull, pf);
         }
     }
+    cp_async_wait<0>();
 }
 
+// One item of a recurrent job; `mask`: the lanes of the warp working on it
+// (all of them call).  The warm restart and the run from the series start give
+// the same bits, so one lane that cannot restart (its seeding is too near)
+// makes all of them run from their seeds rather than split the warp.
 template <class Op>
-__device__ void run_chunk(const PlanArgs& a, const PlanJob& J, int s, int k, const Stage& sg) {
+__device__ void run_chunk(const PlanArgs& a, const PlanJob& J, int s, int k, const Stage& sg, unsigned mask) {
     const int L = a.len[s];
     const int c0 = k * J.chunk;
+    const int f = a.first_hlc[s];
+    const unsigned live = __ballot_sync(mask, c0 < L);
     if (c0 >= L) return;
     const int c1 = min(c0 + J.chunk, L);
-    const int f = a.first_hlc[s];
     Op op;
     op.init(J.period, J.param, f);
     const TmIn in{a.h, a.l, a.c, (size_t)a.cols, (size_t)s};
     const size_t sidx = (size_t)k * a.cols + s;
+    // (a series without a valid bar has nothing to restart or compute)
+    const bool exact = __any_sync(live, k == 0 || (f < L && c0 - J.warm < op.run_from()));
+    Seed sd;
     int t;
-    bool exact = true;
-    if (k > 0 && f < L && c0 - J.warm >= op.run_from()) {
+    if (!exact) {
         t = c0 - J.warm;
-        op.start_warm(in, t);
-        exact = false;
-    } else {
-        t = min(f, c0);
+        sd = Seed{f < L ? t : kNever, qnan(), qnan()};
         op.start_exact();
+        if (f < L) op.start_warm(in, t);
+    } else {
+        sd = run_seed(op, in, f, L);
+        t = __reduce_min_sync(live, min(sd.rf, c0));
     }
-    run_span(op, in, sg, t, c0, false, J.out0, J.out1);
+    run_span<false>(op, in, sg, live, sd, t, c0, J.out0, J.out1);
     float w[8];
     if (k > 0) {
         op.save(w);
         float4* d = reinterpret_cast<float4*>(J.st_start + sidx * 8);
         d[0] = make_float4(w[0], w[1], w[2], w[3]);
         d[1] = make_float4(w[4], w[5], w[6], w[7]);
-        J.exact[sidx] = exact ? 1 : 0;
+        J.exact[sidx] = exact || f >= L ? 1 : 0;
     }
-    run_span(op, in, sg, c0, c1, true, J.out0, J.out1);
+    run_span<true>(op, in, sg, live, sd, c0, c1, J.out0, J.out1);
     op.save(w);
     float4* d = reinterpret_cast<float4*>(J.st_end + sidx * 8);
     d[0] = make_float4(w[0], w[1], w[2], w[3]);
@@ -202,45 +297,68 @@ __device__ void run_pnr(const PlanArgs& a, const PlanJob& J, int s, int k, const
     const int c1 = max(c0, min(c0 + J.chunk, L));
     const TmIn in{a.h, a.l, a.c, (size_t)a.cols, (size_t)s};
     const int f = a.first_c[s];
-    // window registers: the length rounded up to a multiple of 8
-    switch ((J.period + 7) >> 3) {
-        case 1: case 2: pnr_chunk<16>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
-        case 3: pnr_chunk<24>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
-        case 4: pnr_chunk<32>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
-        case 5: pnr_chunk<40>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
-        case 6: pnr_chunk<48>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
-        case 7: pnr_chunk<56>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+    // window registers: the length rounded up to a multiple of 4
+    switch (max(4, (J.period + 3) >> 2)) {
+        case 4: pnr_chunk<16>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 5: pnr_chunk<20>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 6: pnr_chunk<24>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 7: pnr_chunk<28>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 8: pnr_chunk<32>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 9: pnr_chunk<36>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 10: pnr_chunk<40>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 11: pnr_chunk<44>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 12: pnr_chunk<48>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 13: pnr_chunk<52>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 14: pnr_chunk<56>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
+        case 15: pnr_chunk<60>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
         default: pnr_chunk<64>(in, sg, mask, f, L, J.period, J.pfrac, c0, c1, J.out0); break;
     }
 }
 
 // Persistent work-list kernel: each warp takes items until the list is done.
+// A warp's first item is its rank in the order (warp of the block, block), so a
+// list shorter than the grid's warps is spread evenly over the SMs (blocks are
+// placed round-robin); the others come from the counter.
 __global__ void __launch_bounds__(kPlanWarps * 32) k_tm_plan(PlanArgs a) {
     extern __shared__ float plan_smem[];
-    const int lane = threadIdx.x & 31;
-    const Stage sg{plan_smem + (threadIdx.x >> 5) * kStageFloats, lane};
-    for (;;) {
-        int it = 0;
-        if (lane == 0) it = atomicAdd(a.counter, 1);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= a.n_items) break;
-        const int4 w = a.items[it];
-        const int s = w.y * 32 + lane;
-        const unsigned mask = __ballot_sync(0xffffffffu, s < a.cols);
-        if (s >= a.cols) continue;
-        const PlanJob& J = a.jobs[w.x];
-        switch (J.kind) {
-            case PJ_ATR: run_chunk<PAtr>(a, J, s, w.z, sg); break;
-            case PJ_ADX: run_chunk<PAdx>(a, J, s, w.z, sg); break;
-            case PJ_SUPERTREND: run_chunk<PSuperTrend>(a, J, s, w.z, sg); break;
-            default: run_pnr(a, J, s, w.z, sg, mask); break;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Stage sg{plan_smem + warp * kStageFloats, lane};
+    const int n_warps = gridDim.x * kPlanWarps;
+    int it = warp * gridDim.x + blockIdx.x;
+    while (it < a.n_items) {
+        const int4 w = a.items[it];  // {job, first entry of a.lanes, chunk, lanes}
+        const unsigned mask = __ballot_sync(0xffffffffu, lane < w.w);
+        if (lane < w.w) {
+            const int s = a.lanes[w.y + lane];
+            const PlanJob& J = a.jobs[w.x];
+            switch (J.kind) {
+                case PJ_ATR: run_chunk<PAtr>(a, J, s, w.z, sg, mask); break;
+                case PJ_ADX: run_chunk<PAdx>(a, J, s, w.z, sg, mask); break;
+                case PJ_SUPERTREND: run_chunk<PSuperTrend>(a, J, s, w.z, sg, mask); break;
+                default: run_pnr(a, J, s, w.z, sg, mask); break;
+            }
         }
+        __syncwarp();
+        if (lane == 0) it = n_warps + atomicAdd(a.counter, 1);
+        it = __shfl_sync(0xffffffffu, it, 0);
     }
 }
 
-// Fix-up: per (recurrent job, series), chunks in order; a warm-restarted
-// chunk whose recorded start state differs from the previous chunk's end
-// state is recomputed from that end state.
+// Fix-up of a (recurrent job, 32 series) block: its warps compare, over all
+// chunks at once, the recorded start state of each warm-restarted chunk with
+// the end state of the chunk before it.  Series with a mismatch (rare) then
+// take their chunks in order: one whose start state differs from the end state
+// that now stands before it is recomputed from that.
+constexpr int kFixWarps = 8;
+
+__device__ __forceinline__ bool same_state(const PlanJob& J, size_t sidx, size_t pidx) {
+    const uint4* ps = reinterpret_cast<const uint4*>(J.st_start + sidx * 8);
+    const uint4* pe = reinterpret_cast<const uint4*>(J.st_end + pidx * 8);
+    const uint4 s0 = ps[0], s1 = ps[1], e0 = pe[0], e1 = pe[1];
+    return s0.x == e0.x && s0.y == e0.y && s0.z == e0.z && s0.w == e0.w && s1.x == e1.x && s1.y == e1.y &&
+           s1.z == e1.z && s1.w == e1.w;
+}
+
 template <class Op>
 __device__ void fixup_series(const PlanArgs& a, const PlanJob& J, int s) {
     const int L = a.len[s];
@@ -249,12 +367,7 @@ __device__ void fixup_series(const PlanArgs& a, const PlanJob& J, int s) {
         const size_t sidx = (size_t)k * a.cols + s;
         if (J.exact[sidx]) continue;
         const size_t pidx = sidx - a.cols;
-        const uint4* ps = reinterpret_cast<const uint4*>(J.st_start + sidx * 8);
-        const uint4* pe = reinterpret_cast<const uint4*>(J.st_end + pidx * 8);
-        const uint4 s0 = ps[0], s1 = ps[1], e0 = pe[0], e1 = pe[1];
-        if (s0.x == e0.x && s0.y == e0.y && s0.z == e0.z && s0.w == e0.w && s1.x == e1.x && s1.y == e1.y &&
-            s1.z == e1.z && s1.w == e1.w)
-            continue;
+        if (same_state(J, sidx, pidx)) continue;
         const int c0 = k * J.chunk;
         const int c1 = min(c0 + J.chunk, L);
         Op op;
@@ -277,16 +390,25 @@ __device__ void fixup_series(const PlanArgs& a, const PlanJob& J, int s) {
     }
 }
 
-__global__ void k_tm_fixup(PlanArgs a) {
-    const long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = (int)(g / a.cols), s = (int)(g % a.cols);
-    if (j >= a.n_jobs) return;
-    const PlanJob& J = a.jobs[j];
+__global__ void __launch_bounds__(32 * kFixWarps) k_tm_fixup(PlanArgs a) {
+    const PlanJob& J = a.jobs[blockIdx.y];
+    if (J.kind == PJ_PERCENTILE) return;
+    __shared__ int need[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int s = blockIdx.x * 32 + lane;
+    const int L = s < a.cols ? a.len[s] : 0;
+    if (warp == 0) need[lane] = 0;
+    __syncthreads();
+    for (int k = 1 + warp; (long long)k * J.chunk < L; k += kFixWarps) {
+        const size_t sidx = (size_t)k * a.cols + s;
+        if (!J.exact[sidx] && !same_state(J, sidx, sidx - a.cols)) need[lane] = 1;
+    }
+    __syncthreads();
+    if (warp != 0 || !need[lane]) return;
     switch (J.kind) {
         case PJ_ATR: fixup_series<PAtr>(a, J, s); break;
         case PJ_ADX: fixup_series<PAdx>(a, J, s); break;
-        case PJ_SUPERTREND: fixup_series<PSuperTrend>(a, J, s); break;
-        default: break;
+        default: fixup_series<PSuperTrend>(a, J, s); break;
     }
 }
 
@@ -312,8 +434,7 @@ vta_status launch_tm_plan(const PlanArgs& a, int blocks, cudaStream_t st) {
 }
 
 vta_status launch_tm_fixup(const PlanArgs& a, cudaStream_t st) {
-    const long long n = (long long)a.n_jobs * a.cols;
-    k_tm_fixup<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(a);
+    k_tm_fixup<<<dim3((a.cols + 31) / 32, a.n_jobs), 32 * kFixWarps, 0, st>>>(a);
     return check_launch("k_tm_fixup");
 }
 

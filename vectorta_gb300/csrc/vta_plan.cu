@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <tuple>
 #include <vector>
 
@@ -27,7 +28,6 @@ struct vta_tm_plan {
     const float* c = nullptr;
     int cols = 0, rows = 0;
     std::vector<int> lens;      // host copy of the series lengths
-    std::vector<int> tile_max;  // longest series of each 32-series tile
     std::vector<PlanJob> jobs;  // device pointers inside
     std::vector<size_t> state_cap;  // chunks the state buffers of each job hold
     std::vector<void*> allocs;  // every device allocation of the plan
@@ -37,6 +37,8 @@ struct vta_tm_plan {
     PlanJob* d_jobs = nullptr;
     int4* d_items = nullptr;
     size_t items_cap = 0;
+    int* d_lanes = nullptr;  // series lists of the work items
+    size_t lanes_cap = 0;
     int n_items = 0;
     int* d_ctr = nullptr;   // [0] work-list head, [1] fix-up count
     int* h_stats = nullptr; // pinned copy of d_ctr after each run
@@ -90,20 +92,34 @@ vta_status plan_states(vta_tm_plan* P, int j, int chunk) {
 
 // Work list of the jobs in `which` (indices into P->jobs; the item's job field
 // is the position in `which`), ordered by chunk start so that the jobs and
-// tiles working on the same rows run together and share the inputs in L2.
+// series working on the same rows run together and share the inputs in L2.  A
+// chunk's items take the series that reach its start, 32 at a time.
 vta_status plan_items(vta_tm_plan* P, const std::vector<int>& which) {
     struct Key {
-        int c0, tile, job, k;
+        int c0, lane0, job, k, lanes;
     };
     std::vector<Key> keys;
+    std::vector<int> lanes;
+    std::map<int, std::pair<int, int>> lists;  // chunk start -> {first entry, entries}
+    const int maxlen = *std::max_element(P->lens.begin(), P->lens.end());
     for (size_t q = 0; q < which.size(); ++q) {
         const PlanJob& J = P->jobs[which[q]];
-        for (size_t g = 0; g < P->tile_max.size(); ++g)
-            for (int k = 0; (long long)k * J.chunk < P->tile_max[g]; ++k)
-                keys.push_back({k * J.chunk, (int)g, (int)q, k});
+        for (int k = 0; (long long)k * J.chunk < maxlen; ++k) {
+            const int c0 = k * J.chunk;
+            auto [l, fresh] = lists.try_emplace(c0, (int)lanes.size(), 0);
+            if (fresh) {
+                for (int s = 0; s < P->cols; ++s)
+                    if (P->lens[s] > c0) lanes.push_back(s);
+                if (lanes.size() > (size_t)INT32_MAX)
+                    return fail(VTA_ERR_LAUNCH_CONFIG_TOO_LARGE, "tm plan: too many work items");
+                l->second.second = (int)lanes.size() - l->second.first;
+            }
+            for (int i = 0; i < l->second.second; i += 32)
+                keys.push_back({c0, l->second.first + i, (int)q, k, std::min(32, l->second.second - i)});
+        }
     }
     std::sort(keys.begin(), keys.end(), [](const Key& a, const Key& b) {
-        return std::tie(a.c0, a.tile, a.job) < std::tie(b.c0, b.tile, b.job);
+        return std::tie(a.c0, a.lane0, a.job) < std::tie(b.c0, b.lane0, b.job);
     });
     if (keys.size() > (size_t)INT32_MAX) return fail(VTA_ERR_LAUNCH_CONFIG_TOO_LARGE, "tm plan: too many work items");
     if (keys.size() > P->items_cap) {
@@ -113,10 +129,20 @@ vta_status plan_items(vta_tm_plan* P, const std::vector<int>& which) {
         P->d_items = static_cast<int4*>(p);
         P->items_cap = keys.size();
     }
+    if (lanes.size() > P->lanes_cap) {
+        plan_free(P, P->d_lanes);
+        void* p = nullptr;
+        VTA_TRY(plan_alloc(P, lanes.size() * sizeof(int), &p));
+        P->d_lanes = static_cast<int*>(p);
+        P->lanes_cap = lanes.size();
+    }
     std::vector<int4> items(keys.size());
-    for (size_t i = 0; i < keys.size(); ++i) items[i] = make_int4(keys[i].job, keys[i].tile, keys[i].k, 0);
-    if (!items.empty())
+    for (size_t i = 0; i < keys.size(); ++i)
+        items[i] = make_int4(keys[i].job, keys[i].lane0, keys[i].k, keys[i].lanes);
+    if (!items.empty()) {
         VTA_CUDA_TRY(cudaMemcpy(P->d_items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+        VTA_CUDA_TRY(cudaMemcpy(P->d_lanes, lanes.data(), lanes.size() * sizeof(int), cudaMemcpyHostToDevice));
+    }
     P->n_items = (int)items.size();
     return VTA_OK;
 }
@@ -142,6 +168,7 @@ PlanArgs plan_args(const vta_tm_plan* P, int n_jobs) {
     a.jobs = P->d_jobs;
     a.n_jobs = n_jobs;
     a.items = P->d_items;
+    a.lanes = P->d_lanes;
     a.n_items = P->n_items;
     a.counter = P->d_ctr;
     a.stats = P->d_ctr + 1;
@@ -201,11 +228,11 @@ void tune_store_locked(const TuneKey& key, int chunk) {
 // Times job j alone with each candidate chunk length (second of two runs)
 // and returns the fastest.
 vta_status tune_job(vta_tm_plan* P, int j, int* best) {
-    static const int kRec[] = {1024, 2048, 4096, 8192, 16384};
+    static const int kRec[] = {256, 512, 1024, 2048, 4096, 8192, 16384};
     static const int kPnr[] = {128, 256, 512, 1024};
     const bool rec = plan_job_recurrent(P->jobs[j].kind);
     const int* cand = rec ? kRec : kPnr;
-    const int nc = rec ? 5 : 4;
+    const int nc = rec ? 7 : 4;
     const int maxlen = *std::max_element(P->lens.begin(), P->lens.end());
     cudaStream_t st = P->ctx->stream;
     cudaEvent_t e0, e1;
@@ -266,11 +293,6 @@ vta_status plan_create(vta_ctx* ctx, const float* h, const float* l, const float
         const size_t L = lengths ? lengths[s] : rows;
         if (L > rows) return fail(VTA_ERR_INVALID_INPUT, "tm plan: a series length exceeds rows");
         P->lens[s] = (int)L;
-    }
-    for (size_t g = 0; g < (cols + 31) / 32; ++g) {
-        int mx = 0;
-        for (size_t s = g * 32; s < std::min(cols, g * 32 + 32); ++s) mx = std::max(mx, P->lens[s]);
-        P->tile_max.push_back(mx);
     }
     for (size_t j = 0; j < n_jobs; ++j) {
         const vta_tm_job& in = jobs[j];
@@ -445,6 +467,7 @@ vta_status tm_job_enqueue(vta_ctx* ctx, int kind, int period, double param, cons
     ar.need(cols * sizeof(int));
     ar.need(sizeof(PlanJob));
     ar.need(n_items * sizeof(int4));
+    ar.need(cols * sizeof(int));
     ar.need(2 * sizeof(int));
     ar.need(states * 8 * sizeof(float));
     ar.need(states * 8 * sizeof(float));
@@ -455,6 +478,7 @@ vta_status tm_job_enqueue(vta_ctx* ctx, int kind, int period, double param, cons
     int* d_fc = ar.take<int>(cols);
     PlanJob* d_job = ar.take<PlanJob>(1);
     int4* d_items = ar.take<int4>(n_items);
+    int* d_lanes = ar.take<int>(cols);
     int* d_ctr = ar.take<int>(2);
     PlanJob J{};
     J.kind = kind;
@@ -472,8 +496,11 @@ vta_status tm_job_enqueue(vta_ctx* ctx, int kind, int period, double param, cons
     std::vector<int4> items;
     items.reserve(n_items);
     for (int k = 0; k < nch; ++k)
-        for (int g = 0; g < tiles; ++g) items.push_back(make_int4(0, g, k, 0));
+        for (int g = 0; g < tiles; ++g) items.push_back(make_int4(0, 32 * g, k, std::min(32, cols - 32 * g)));
+    std::vector<int> lanes(cols);
+    std::iota(lanes.begin(), lanes.end(), 0);
     VTA_TRY(upload_async(ctx, d_len, lens.data(), cols * sizeof(int), st));
+    VTA_TRY(upload_async(ctx, d_lanes, lanes.data(), cols * sizeof(int), st));
     VTA_TRY(upload_async(ctx, d_job, &J, sizeof(PlanJob), st));
     VTA_TRY(upload_async(ctx, d_items, items.data(), n_items * sizeof(int4), st));
     VTA_CUDA_TRY(cudaMemsetAsync(d_ctr, 0, 2 * sizeof(int), st));
@@ -489,6 +516,7 @@ vta_status tm_job_enqueue(vta_ctx* ctx, int kind, int period, double param, cons
     a.jobs = d_job;
     a.n_jobs = 1;
     a.items = d_items;
+    a.lanes = d_lanes;
     a.n_items = (int)n_items;
     a.counter = d_ctr;
     a.stats = d_ctr + 1;

@@ -33,9 +33,10 @@ struct PlanArgs {
     const int* first_c;    // [cols] first valid close
     const PlanJob* jobs;
     int n_jobs;
-    const int4* items;     // {job, tile, chunk, 0}
+    const int4* items;     // {job, first entry of lanes, chunk, number of lanes}
+    const int* lanes;      // series lists of the chunks, in series order
     int n_items;
-    int* counter;          // work-list head (zeroed before each launch)
+    int* counter;          // items taken past each warp's first (zeroed before each launch)
     int* stats;            // [0] chunks recomputed by the fix-up pass
 };
 
