@@ -1114,19 +1114,20 @@ __device__ __forceinline__ float general_step(Op& op, bool active, bool seeded_e
 // AGG record of one (lane, chunk): state, and applied steps or a marker for
 // a chunk before the seed / holding the seed.
 template <class Op>
-__device__ __forceinline__ void write_agg(const RecurArgs& a, const Op& op, bool active, bool seeded_ever, int steps,
-                                          int chunk, int c0, int c1, int li) {
-    float4 g;
+__device__ __forceinline__ float4 agg_record(const Op& op, bool active, bool seeded_ever, int steps, int c0, int c1) {
     const bool abs_chunk = active && seeded_ever && c0 <= op.s && op.s < c1;
     const bool before = !active || !seeded_ever || c1 <= op.s;
+    float4 g;
     g.x = Op::NS > 0 ? op.get(0) : 0.f;
     g.y = Op::NS > 1 ? op.get(1) : 0.f;
     g.z = Op::NS > 2 ? op.get(2) : 0.f;
     g.w = before ? kBeforeSeed : (abs_chunk ? kAbsolute : (float)steps);
     if (before) g.x = g.y = g.z = 0.f;
-    reinterpret_cast<float4*>(a.agg)[(size_t)chunk * a.n_lanes + li] = g;
+    return g;
 }
-
+__device__ __forceinline__ float4* agg_slot(const RecurArgs& a, int chunk, int li) {
+    return reinterpret_cast<float4*>(a.agg) + (size_t)chunk * a.n_lanes + li;
+}
 
 // Batch EMIT stages 64 steps per lane (two 32-step tiles) and writes each
 // row's 256-byte segment with one float2 store per lane: on GB300 that write
@@ -1137,9 +1138,417 @@ __device__ __forceinline__ void write_agg(const RecurArgs& a, const Op& op, bool
 constexpr int kSeg = 64;
 constexpr int kStageW = kSeg + 2;
 
+// ------------------------------------------------------- warm-up tiles ----
+// Tiles in which some combos are still warming up.  All combos of a batch
+// sweep share the series and its first valid index f, so what their warm-up
+// needs is one prefix sum over [f, t] of the op's terms (x, the true ranges,
+// or the gains and losses): a lane whose seed index s lies in the tile takes
+// its seed from the prefix at s, and EMA's warm-up output, the running mean,
+// is the prefix over the count.  The prefix of a 32-step tile is one warp scan
+// of compensated pairs, and a step is then the running update under the
+// predicate t > s: no accumulators, divisions or branches per lane and step
+// (the general path's per-lane phases cost about 150 cycles a step, which made
+// the seeding chunk the longest of a sweep: with the shorter first chunks that
+// this allows, EMA 2..1000 on 20,000 bars 195 -> 46 us, RSI 225 -> 64).  Used when every input of [f, tile end) is finite;
+// otherwise the chunk's warm-up takes the general path.
+struct WarmTerm {
+    float2 a, b;  // compensated terms of one step (b: RSI's loss)
+};
+
+template <class Op> struct WarmOf { static constexpr bool ok = false; };
+template <> struct WarmOf<OpEma> { static constexpr bool ok = true, two = false; };
+template <> struct WarmOf<OpDema> { static constexpr bool ok = true, two = false; };
+template <> struct WarmOf<OpWilders> { static constexpr bool ok = true, two = false; };
+template <> struct WarmOf<OpAtr> { static constexpr bool ok = true, two = false; };
+template <> struct WarmOf<OpTema> { static constexpr bool ok = true, two = false; };
+template <> struct WarmOf<OpRsi<true>> { static constexpr bool ok = true, two = true; };
+
+__device__ __forceinline__ float2 exact_diff(float a, float b) {  // a - b as value and error
+    const float d = a - b;
+    const float bb = d - a;
+    return make_float2(d, (a - (d - bb)) - (b + bb));
+}
+
+// finite, and small enough that no sum of a warm-up overflows
+__device__ __forceinline__ bool warm_fin(float v) { return fabsf(v) <= 0x1p96f; }
+
+// Inputs of one lane's step t of a tile (x0 / c at t, x1 at t - 1), its term,
+// and the value the running step reads (x, the true range, or the difference)
+template <class Op>
+__device__ __forceinline__ WarmTerm warm_term(int t, int f, float x0, float x1, float h, float l, float& in, bool& fin) {
+    WarmTerm w{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    if constexpr (std::is_same<Op, OpAtr>::value) {
+        in = t == f ? h - l : true_range(h, l, x1);
+        fin = t < f || (warm_fin(x0) && warm_fin(in));
+        if (t >= f) w.a = t == f ? exact_diff(h, l) : make_float2(in, 0.f);
+    } else if constexpr (std::is_same<Op, OpRsi<true>>::value) {
+        in = t > f ? x0 - x1 : 0.f;
+        fin = t < f || (warm_fin(x0) && warm_fin(in));
+        if (t > f) {
+            if (x0 > x1) w.a = exact_diff(x0, x1);
+            else if (x0 < x1) w.b = exact_diff(x1, x0);
+        }
+    } else {
+        in = x0;
+        fin = t < f || warm_fin(x0);
+        if (t >= f) w.a = make_float2(x0, 0.f);
+    }
+    return w;
+}
+
+__device__ __forceinline__ float2 pair_scan(float2 v) {  // inclusive over the warp
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float2 u = make_float2(__shfl_up_sync(0xffffffffu, v.x, o), __shfl_up_sync(0xffffffffu, v.y, o));
+        if (lane >= o) v = pair_add(u, v);
+    }
+    return v;
+}
+__device__ __forceinline__ float2 pair_shfl(float2 v, int src) {
+    return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+// sum / p, from a compensated sum, correctly rounded up to the last bit
+__device__ __forceinline__ float pair_mean(float2 sum, int p) {
+    const D2 m = d2_mul(D2{sum.x, sum.y}, d2_ratio(1, p));
+    return m.hi + m.lo;
+}
+
+// The prefix of the terms over [f, c0) and whether every input of [f, tend) is
+// finite (whole warp)
+template <class Op>
+__device__ bool warm_prefix(const InBatch& in, int f, int c0, int tend, WarmTerm& pre) {
+    // (TEMA's stages start from values, not sums, and take any input)
+    if constexpr (std::is_same<Op, OpTema>::value) return true;
+    const int lane = threadIdx.x & 31;
+    WarmTerm acc{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    bool ok = true;
+#pragma unroll 4
+    for (int t = f + lane; t < tend; t += 32) {
+        float x0, x1 = 0.f, h = 0.f, l = 0.f, v;
+        bool fin;
+        if constexpr (Op::kHlc) {
+            x0 = in.C(t);
+            if (t > f) x1 = in.C(t - 1);
+            h = in.H(t);
+            l = in.L(t);
+        } else {
+            x0 = in.X(t);
+            if (t > f) x1 = in.X(t - 1);
+        }
+        const WarmTerm w = warm_term<Op>(t, f, x0, x1, h, l, v, fin);
+        ok = ok && fin;
+        if (t < c0) {
+            acc.a = pair_add(acc.a, w.a);
+            if (WarmOf<Op>::two) acc.b = pair_add(acc.b, w.b);
+        }
+    }
+    pre.a = pair_shfl(pair_scan(acc.a), 31);
+    pre.b = WarmOf<Op>::two ? pair_shfl(pair_scan(acc.b), 31) : acc.b;
+    return __all_sync(0xffffffffu, ok);
+}
+
+// Steps [tb, tb + nt) of a warm-up tile; xv .. lv: this lane's step of the tile,
+// x1: the step before it; pre: the prefix over [f, tb), updated.
+template <int PASS, class Op>
+__device__ __forceinline__ void warm_tile(Op& op, int f, int tb, int nt, float xv, float x1, float hv, float lv,
+                                          WarmTerm& pre, float* srow, int sw) {
+    const int lane = threadIdx.x & 31;
+    const int t = tb + lane, s = op.s;  // (f: the sweep's, also for lanes without a combo)
+    float in = 0.f;
+    bool fin;
+    WarmTerm w = warm_term<Op>(lane < nt ? t : f - 1, f, xv, x1, hv, lv, in, fin);
+    if (!std::is_same<Op, OpTema>::value && !std::is_same<Op, OpDema>::value) {
+        w.a = pair_add(pre.a, pair_scan(w.a));  // the prefix over [f, t]
+        pre.a = pair_shfl(w.a, 31);
+    }
+    if (WarmOf<Op>::two) {
+        w.b = pair_add(pre.b, pair_scan(w.b));
+        pre.b = pair_shfl(w.b, 31);
+    }
+    const bool here = s >= tb && s < tb + nt;
+    const int sl = here ? s - tb : 0;  // the lane holding this lane's seed step
+    if constexpr (std::is_same<Op, OpEma>::value) {
+        const float mean = (w.a.x + w.a.y) / (float)(t - f + 1);
+        float y = op.y;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) {
+            if (j >= nt) break;
+            const float x = __shfl_sync(0xffffffffu, in, j), m = __shfl_sync(0xffffffffu, mean, j);
+            y = tb + j > s ? fmaf(op.alpha, x - y, y) : m;
+            if (PASS == PASS_EMIT) srow[j ^ sw] = tb + j < f ? qnan() : y;
+        }
+        op.y = y;
+    } else if constexpr (std::is_same<Op, OpDema>::value) {
+        float e1 = op.e1, e2 = op.e2;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) {
+            if (j >= nt) break;
+            const float x = __shfl_sync(0xffffffffu, in, j);
+            const bool run = tb + j > f;
+            e1 = run ? fmaf(op.alpha, x - e1, e1) : x;
+            e2 = run ? fmaf(op.alpha, e1 - e2, e2) : x;
+            if (PASS == PASS_EMIT) srow[j ^ sw] = tb + j < op.warm ? qnan() : fmaf(e1, 2.f, -e2);
+        }
+        op.e1 = e1;
+        op.e2 = e2;
+    } else if constexpr (std::is_same<Op, OpTema>::value) {
+        // the three stages join at f, start2 and s as copies of the one before
+        // (a stage not yet started holds nothing that is read)
+        const float a = op.per;
+        const bool copy = op.p1 == 0;
+        float e1 = op.e1, e2 = op.e2, e3 = op.e3;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) {
+            if (j >= nt) break;
+            const float x = __shfl_sync(0xffffffffu, in, j);
+            const float b1 = tb + j == f ? x : e1;
+            e1 = copy ? x : fmaf(a, x - b1, b1);
+            const float b2 = tb + j == op.start2 ? e1 : e2;
+            e2 = fmaf(a, e1 - b2, b2);
+            const float b3 = tb + j == s ? e2 : e3;
+            e3 = fmaf(a, e2 - b3, b3);
+            if (PASS == PASS_EMIT) srow[j ^ sw] = tb + j < op.warm ? qnan() : (copy ? x : fmaf(3.f, e1 - e2, e3));
+        }
+        op.e1 = e1;
+        op.e2 = e2;
+        op.e3 = e3;
+    } else if constexpr (std::is_same<Op, OpRsi<true>>::value) {
+        const float2 ga = pair_shfl(w.a, sl), la = pair_shfl(w.b, sl);
+        const int p = (int)op.pf;
+        const float sg = here ? pair_mean(ga, p) : 0.f, sl_ = here ? pair_mean(la, p) : 0.f;
+        float ag = op.ag, al = op.al;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) {
+            if (j >= nt) break;
+            const float d = __shfl_sync(0xffffffffu, in, j);
+            const bool run = tb + j > s;
+            ag = run ? fmaf(ag, op.beta, op.inv_p * fmaxf(d, 0.f)) : sg;
+            al = run ? fmaf(al, op.beta, op.inv_p * fmaxf(-d, 0.f)) : sl_;
+            if (PASS == PASS_EMIT) {
+                const float den = ag + al;
+                const float v = den == 0.f ? 50.f : __fdividef(100.f * ag, den);
+                srow[j ^ sw] = tb + j < s ? qnan() : v;
+            }
+        }
+        op.ag = ag;
+        op.al = al;
+    } else {  // Wilders, ATR
+        const float2 sum = pair_shfl(w.a, sl);
+        const float seed = here ? pair_mean(sum, op.p) : 0.f;
+        const bool copy = std::is_same<Op, OpWilders>::value && op.p == 1;
+        float y = op.y;
+#pragma unroll 8
+        for (int j = 0; j < 32; ++j) {
+            if (j >= nt) break;
+            const float x = __shfl_sync(0xffffffffu, in, j);
+            float n;
+            if constexpr (std::is_same<Op, OpWilders>::value) n = copy ? x : fmaf(x - y, op.alpha, y);
+            else n = fmaf(-op.alpha, y, y) + op.alpha * x;
+            y = tb + j > s ? n : seed;
+            if (PASS == PASS_EMIT) srow[j ^ sw] = tb + j < s ? qnan() : y;
+        }
+        op.y = y;
+    }
+}
+
+// One warp's 32 lanes (combos 32 group .. 32 group + 31) over [c0, c1): AGG
+// returns the lane's record, EMIT starts from the state `cv` where the lane is
+// running and writes the outputs.  stage: 32 x kStageW floats, xin: 16 float4
+// of the warp's own (EMIT only).
+template <class Op, int PASS>
+__device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int c0, int c1, const float4 cv,
+                                             float* stage, float4* xin) {
+    const int lane = threadIdx.x & 31;
+    const int li = group * 32 + lane;
+    const bool valid = li < a.n_lanes;
+    Op op;
+    int p = 0, first = a.n;
+    if (valid) {
+        p = a.periods[li];
+        first = a.first;
+    }
+    op.init(p > 0 ? p : 1, first);
+    const bool active = valid && first < a.n && p > 0;
+    const bool seeded_ever = active && op.s < a.n;
+    const InBatch in{a.x, a.h, a.l, a.c};
+
+    // first time index from which this lane needs no phase checks; lanes that
+    // never write (invalid / all-NaN) do not hold the warp back
+    const int run_from = (active && seeded_ever) ? max(op.s + 1, op.warm) : (valid ? INT_MAX : INT_MIN);
+    const int warp_run_from = warp_max(run_from);
+    // warm-up tiles: the prefix at c0, if every input they read is finite
+    bool warm_ok = false;
+    WarmTerm pre{};
+    if constexpr (WarmOf<Op>::ok) {
+        if (c0 < warp_run_from && a.first < a.n) {  // up to the end of the last such tile
+            const int tend = warp_run_from >= c1 ? c1 : min(c1, c0 + (warp_run_from - c0 + 31) / 32 * 32);
+            warm_ok = warm_prefix<Op>(in, a.first, c0, tend, pre);
+        }
+    }
+
+    // chunk entry state
+    bool running = false;
+    if (active) {
+        if (c0 > op.s && seeded_ever) {
+            if (PASS == PASS_AGG) {
+                op.zero();
+            } else {
+                if (Op::NS > 0) op.set(0, cv.x);
+                if (Op::NS > 1) op.set(1, cv.y);
+                if (Op::NS > 2) op.set(2, cv.z);
+            }
+            running = true;
+        } else if (c0 > op.f && (!warm_ok || std::is_same<Op, OpTema>::value)) {
+            // the chunk starts inside the warm-up: accumulate [f, c0) first
+            // (TEMA's stages have no closed form in the terms)
+            const int end = min(c0, op.s + 1);
+#pragma unroll 8
+            for (int t = op.f; t < end; ++t) op.accum(in, t);
+        }
+    }
+
+    int steps = 0;
+    // this lane's staging row (batch EMIT): the current 64-step segment starts
+    // at seg0, the tile at column off = tb - seg0 (0 or 32), swizzle sw
+    const int sw = (lane >> 4) & 1;
+    const bool vec2 = PASS == PASS_EMIT && (a.n & 1) == 0 && (c0 & 1) == 0 &&
+                      (reinterpret_cast<uintptr_t>(a.out) & 7) == 0;
+    // writes a completed segment of the warp's 32 rows (tile [tb, te))
+    auto flush = [&](int seg0, int off, int te) {
+        if (PASS != PASS_EMIT || (off != kSeg - 32 && te != c1)) return;
+        __syncwarp();
+        const int row0 = group * 32;
+        const int rows = min(32, a.n_lanes - row0);
+        const int len = te - seg0;
+        float* ob = a.out + (size_t)row0 * a.n + seg0;
+        if (vec2 && len == kSeg) {
+            // rows 0..15 as staged, rows 16..31 with each pair swapped back
+            const int r16 = min(rows, 16);
+            float* op = ob + 2 * lane;
+#pragma unroll 4
+            for (int r = 0; r < r16; ++r, op += a.n)
+                *reinterpret_cast<float2*>(op) = *reinterpret_cast<const float2*>(stage + r * kStageW + 2 * lane);
+#pragma unroll 4
+            for (int r = 16; r < rows; ++r, op += a.n) {
+                const float2 v = *reinterpret_cast<const float2*>(stage + r * kStageW + 2 * lane);
+                *reinterpret_cast<float2*>(op) = make_float2(v.y, v.x);
+            }
+        } else {
+            for (int h = lane; h < len; h += 32) {
+#pragma unroll 4
+                for (int r = 0; r < rows; ++r) ob[(size_t)r * a.n + h] = stage[r * kStageW + (h ^ ((r >> 4) & 1))];
+            }
+        }
+        __syncwarp();
+    };
+    // two loops, so that nothing of the warm-up's state is live in the second
+    int tb = c0;
+    for (; tb < c1 && tb < warp_run_from; tb += 32) {
+        const int te = min(tb + 32, c1);
+        const int seg0 = c0 + ((tb - c0) & ~(kSeg - 1));
+        const int off = tb - seg0;
+        float* srow = stage + lane * kStageW + off;
+        // ---- general path: per-step phase logic
+        rsi_fast_exit(op);  // (a no-op: general tiles come before the fast ones)
+        // the tile's inputs in registers (one coalesced load per lane);
+        // each step's values are broadcast by shuffles at the top of
+        // the warp-uniform step loop, before any per-lane branch
+        const int nt = te - tb;
+        float xv = 0.f, hv = 0.f, lv = 0.f, pb = 0.f;
+        if constexpr (Op::kHlc) {
+            if (lane < nt) {
+                hv = __ldg(a.h + tb + lane);
+                lv = __ldg(a.l + tb + lane);
+                xv = __ldg(a.c + tb + lane);
+            }
+            if (tb > 0) pb = __ldg(a.c + tb - 1);
+        } else {
+            if (lane < nt) xv = __ldg(a.x + tb + lane);
+            if (tb > 0) pb = __ldg(a.x + tb - 1);
+        }
+        bool done = false;
+        if constexpr (WarmOf<Op>::ok) {
+            if (warm_ok) {
+                float xm = __shfl_up_sync(0xffffffffu, xv, 1);
+                if (lane == 0) xm = pb;
+                warm_tile<PASS>(op, a.first, tb, nt, xv, xm, hv, lv, pre, srow, sw);
+                if (active && seeded_ever) {
+                    steps += max(0, te - max(tb, op.s + 1));
+                    running = op.s < te;
+                }
+                done = true;
+            }
+        }
+        for (int j = 0; j < (done ? 0 : nt); ++j) {
+            InStep st;
+            st.t = tb + j;
+            st.x0 = __shfl_sync(0xffffffffu, xv, j);
+            const float xm = __shfl_sync(0xffffffffu, xv, (j - 1) & 31);
+            st.x1 = j > 0 ? xm : pb;
+            if constexpr (Op::kHlc) {
+                st.h0 = __shfl_sync(0xffffffffu, hv, j);
+                st.l0 = __shfl_sync(0xffffffffu, lv, j);
+            }
+            const float v = general_step(op, active, seeded_ever, running, steps, st, tb + j);
+            if (PASS == PASS_EMIT) srow[j ^ sw] = v;
+        }
+        flush(seg0, off, te);
+    }
+    for (; tb < c1; tb += 32) {
+        const int te = min(tb + 32, c1);
+        const int seg0 = c0 + ((tb - c0) & ~(kSeg - 1));
+        const int off = tb - seg0;
+        float* srow = stage + lane * kStageW + off;
+        // ---- fast path: every lane running and past warm-up
+        if (te - tb == 32) {
+            // the tile's inputs in registers, one coalesced load per lane
+            InTile ti;
+            ti.tb = tb;
+            ti.xs = xin;
+            if constexpr (Op::kHlc) {
+                ti.hv = __ldg(a.h + tb + lane);
+                ti.lv = __ldg(a.l + tb + lane);
+                ti.cv = __ldg(a.c + tb + lane);
+                ti.cb = __ldg(a.c + tb - 1);
+                ti.xv = ti.cv;
+                ti.xb = ti.cb;
+            } else {
+                ti.xv = __ldg(a.x + tb + lane);
+                ti.xb = __ldg(a.x + tb - 1);
+            }
+            // a tile whose inputs (and the value before it) are all finite
+            // runs without per-step skip / NaN logic
+            bool fin;
+            if constexpr (Op::kHlc) {
+                fin = __all_sync(0xffffffffu, isfinite(ti.hv) && isfinite(ti.lv) && isfinite(ti.cv) &&
+                                                  isfinite(ti.cb));
+            } else {
+                fin = __all_sync(0xffffffffu, isfinite(ti.xv) && isfinite(ti.xb));
+            }
+            if (fin) {
+                run_tile<true, PASS>(op, ti, srow, sw, steps);
+            } else {
+                rsi_fast_exit(op);
+                run_tile<false, PASS>(op, ti, srow, sw, steps);
+            }
+        } else if (PASS == PASS_EMIT) {
+            rsi_fast_exit(op);
+#pragma unroll 8
+            for (int t = tb; t < te; ++t) srow[(t - tb) ^ sw] = op.fast(in, t, steps);
+        } else {
+#pragma unroll 8
+            for (int t = tb; t < te; ++t) op.fast(in, t, steps);
+        }
+        flush(seg0, off, te);
+    }
+    return agg_record(op, active, seeded_ever, steps, c0, c1);
+}
+
 template <class Op, int PASS>
 __global__ void __launch_bounds__(kWarps * 32)
 k_recur(RecurArgs a) {
+    // (AGG stages the chunk's inputs in it)
     __shared__ __align__(16) float stage[kWarps][32][PASS == PASS_EMIT ? kStageW : 33];
     // per warp: a fast tile's broadcast inputs (EMIT), 2 x 32 floats
     __shared__ float4 xin[kWarps][PASS == PASS_EMIT ? 16 : 1];
@@ -1163,206 +1572,27 @@ k_recur(RecurArgs a) {
             agg_fast_block<FastKindOf<Op>::k>(a, chunk, c0, c1, &stage[0][0][0]))
             return;
         __syncthreads();  // the general pass below reuses `stage`
-        // the seed chunk: each thread replays its combo's warm-up and seed
-        // from the chunk's inputs staged in shared memory (no per-step
-        // shuffles or warp-wide tiles: the lanes run independently)
-        if (a.fast_agg && chunk == 0 && c1 <= (int)(sizeof(stage) / sizeof(float))) {
-            float* xs = &stage[0][0][0];
-            for (int i = threadIdx.x; i < c1; i += blockDim.x) xs[i] = __ldg(a.x + i);
-            __syncthreads();
-            constexpr int FK = FastKindOf<Op>::k;
-            if constexpr (FK == FK_EMA || FK == FK_RSI || FK == FK_TEMA) {
-                if (a.first < a.n && agg_seed_fast<FK>(a, xs, c1, (int)(sizeof(stage) / sizeof(float)))) return;
+        // a first chunk that holds every combo's seed: each thread runs its
+        // combo from the chunk's inputs staged in shared memory
+        constexpr int FK = FastKindOf<Op>::k;
+        if constexpr (FK == FK_EMA || FK == FK_RSI || FK == FK_TEMA) {
+            if (a.fast_agg && chunk == 0 && a.fast_from == 1 && c1 <= (int)(sizeof(stage) / sizeof(float)) &&
+                a.first < a.n) {
+                float* xs = &stage[0][0][0];
+                for (int i = threadIdx.x; i < c1; i += blockDim.x) xs[i] = __ldg(a.x + i);
+                __syncthreads();
+                if (agg_seed_fast<FK>(a, xs, c1, (int)(sizeof(stage) / sizeof(float)))) return;
+                __syncthreads();
             }
-            const int l0 = blockIdx.x * blockDim.x + threadIdx.x;
-            if (l0 < a.n_lanes) {
-                const int p0 = a.periods[l0];
-                Op op0;
-                op0.init(p0 > 0 ? p0 : 1, a.first);
-                const bool act0 = a.first < a.n && p0 > 0;
-                const bool seeded0 = act0 && op0.s < a.n;
-                bool run0 = false;
-                int st0 = 0;
-                int t = min(a.first, c1);
-                // warm-up and seed through the per-step phase logic ...
-                for (; t < c1 && !run0; ++t) {
-                    InStep st;  // x[t] and x[t - 1] from shared memory
-                    st.t = t;
-                    st.x0 = xs[t];
-                    st.x1 = t > 0 ? xs[t - 1] : 0.f;
-                    st.h0 = st.l0 = 0.f;
-                    general_step(op0, act0, seeded0, run0, st0, st, t);
-                }
-                // ... then the running steps without it (the same state update
-                // as the op's step(); t > s >= 0 here)
-                if constexpr (!HasUni<Op>::value) {
-                    float xprev = t > 0 && t <= c1 ? xs[t - 1] : 0.f;
-#pragma unroll 4
-                    for (; t < c1; ++t) {
-                        const float xv = xs[t];
-                        const InStep st{t, xv, xprev, 0.f, 0.f};
-                        op0.template fast<false>(st, t, st0);
-                        xprev = xv;
-                    }
-                }
-                write_agg(a, op0, act0, seeded0, st0, 0, 0, c1, l0);
-            }
-            return;
         }
     }
-    // a warp with no valid lane has nothing to compute (whole warp leaves; the
-    // kernel has no block-wide barrier)
+    // a warp with no valid lane has nothing to compute (whole warp leaves; no
+    // block-wide barrier follows)
     if (group * 32 >= a.n_lanes) return;
-
-    Op op;
-    int p = 0, first = a.n;
-    if (valid) {
-        p = a.periods[li];
-        first = a.first;
-    }
-    op.init(p > 0 ? p : 1, first);
-    const bool active = valid && first < a.n && p > 0;
-    const bool seeded_ever = active && op.s < a.n;
-    const InBatch in{a.x, a.h, a.l, a.c};
-
-    // chunk entry state
-    bool running = false;
-    if (active) {
-        if (c0 > op.s && seeded_ever) {
-            if (PASS == PASS_AGG) {
-                op.zero();
-            } else {
-                float4 cv = reinterpret_cast<const float4*>(a.carry)[(size_t)chunk * a.n_lanes + li];
-                if (Op::NS > 0) op.set(0, cv.x);
-                if (Op::NS > 1) op.set(1, cv.y);
-                if (Op::NS > 2) op.set(2, cv.z);
-            }
-            running = true;
-        } else if (c0 > op.f) {
-            // the chunk starts inside the warm-up: accumulate [f, c0) first
-            const int end = min(c0, op.s + 1);
-            for (int t = op.f; t < end; ++t) op.accum(in, t);
-        }
-    }
-    // first time index from which this lane needs no phase checks; lanes that
-    // never write (invalid / all-NaN) do not hold the warp back
-    const int run_from = (active && seeded_ever) ? max(op.s + 1, op.warm) : (valid ? INT_MAX : INT_MIN);
-    const int warp_run_from = warp_max(run_from);
-
-    int steps = 0;
-    // this lane's staging row (batch EMIT): the current 64-step segment starts
-    // at seg0, the tile at column off = tb - seg0 (0 or 32), swizzle sw
-    const int sw = (lane >> 4) & 1;
-    const bool vec2 = PASS == PASS_EMIT && (a.n & 1) == 0 && (c0 & 1) == 0 &&
-                      (reinterpret_cast<uintptr_t>(a.out) & 7) == 0;
-    for (int tb = c0; tb < c1; tb += 32) {
-        const int te = min(tb + 32, c1);
-        const int seg0 = c0 + ((tb - c0) & ~(kSeg - 1));
-        const int off = tb - seg0;
-        float* srow = &stage[warp][lane][off];
-        if (tb >= warp_run_from) {
-            // ---- fast path: every lane running and past warm-up
-            if (te - tb == 32) {
-                // the tile's inputs in registers, one coalesced load per lane
-                InTile ti;
-                ti.tb = tb;
-                ti.xs = &xin[warp][0];
-                if constexpr (Op::kHlc) {
-                    ti.hv = __ldg(a.h + tb + lane);
-                    ti.lv = __ldg(a.l + tb + lane);
-                    ti.cv = __ldg(a.c + tb + lane);
-                    ti.cb = __ldg(a.c + tb - 1);
-                    ti.xv = ti.cv;
-                    ti.xb = ti.cb;
-                } else {
-                    ti.xv = __ldg(a.x + tb + lane);
-                    ti.xb = __ldg(a.x + tb - 1);
-                }
-                // a tile whose inputs (and the value before it) are all finite
-                // runs without per-step skip / NaN logic
-                bool fin;
-                if constexpr (Op::kHlc) {
-                    fin = __all_sync(0xffffffffu, isfinite(ti.hv) && isfinite(ti.lv) && isfinite(ti.cv) &&
-                                                      isfinite(ti.cb));
-                } else {
-                    fin = __all_sync(0xffffffffu, isfinite(ti.xv) && isfinite(ti.xb));
-                }
-                if (fin) {
-                    run_tile<true, PASS>(op, ti, srow, sw, steps);
-                } else {
-                    rsi_fast_exit(op);
-                    run_tile<false, PASS>(op, ti, srow, sw, steps);
-                }
-            } else if (PASS == PASS_EMIT) {
-                rsi_fast_exit(op);
-#pragma unroll 8
-                for (int t = tb; t < te; ++t) srow[(t - tb) ^ sw] = op.fast(in, t, steps);
-            } else {
-#pragma unroll 8
-                for (int t = tb; t < te; ++t) op.fast(in, t, steps);
-            }
-        } else {
-            // ---- general path: per-step phase logic
-            rsi_fast_exit(op);  // (a no-op: general tiles come before the fast ones)
-            // the tile's inputs in registers (one coalesced load per lane);
-            // each step's values are broadcast by shuffles at the top of
-            // the warp-uniform step loop, before any per-lane branch
-            const int nt = te - tb;
-            float xv = 0.f, hv = 0.f, lv = 0.f, pb = 0.f;
-            if constexpr (Op::kHlc) {
-                if (lane < nt) {
-                    hv = __ldg(a.h + tb + lane);
-                    lv = __ldg(a.l + tb + lane);
-                    xv = __ldg(a.c + tb + lane);
-                }
-                if (tb > 0) pb = __ldg(a.c + tb - 1);
-            } else {
-                if (lane < nt) xv = __ldg(a.x + tb + lane);
-                if (tb > 0) pb = __ldg(a.x + tb - 1);
-            }
-            for (int j = 0; j < nt; ++j) {
-                InStep st;
-                st.t = tb + j;
-                st.x0 = __shfl_sync(0xffffffffu, xv, j);
-                const float xm = __shfl_sync(0xffffffffu, xv, (j - 1) & 31);
-                st.x1 = j > 0 ? xm : pb;
-                if constexpr (Op::kHlc) {
-                    st.h0 = __shfl_sync(0xffffffffu, hv, j);
-                    st.l0 = __shfl_sync(0xffffffffu, lv, j);
-                }
-                const float v = general_step(op, active, seeded_ever, running, steps, st, tb + j);
-                if (PASS == PASS_EMIT) srow[j ^ sw] = v;
-            }
-        }
-        if (PASS == PASS_EMIT && (off == kSeg - 32 || te == c1)) {
-            // flush the segment [seg0, te) of the warp's 32 rows
-            __syncwarp();
-            const int row0 = group * 32;
-            const int rows = min(32, a.n_lanes - row0);
-            const int len = te - seg0;
-            float* ob = a.out + (size_t)row0 * a.n + seg0;
-            if (vec2 && len == kSeg) {
-                // rows 0..15 as staged, rows 16..31 with each pair swapped back
-                const int r16 = min(rows, 16);
-                float* op = ob + 2 * lane;
-#pragma unroll 4
-                for (int r = 0; r < r16; ++r, op += a.n)
-                    *reinterpret_cast<float2*>(op) = *reinterpret_cast<const float2*>(&stage[warp][r][2 * lane]);
-#pragma unroll 4
-                for (int r = 16; r < rows; ++r, op += a.n) {
-                    const float2 v = *reinterpret_cast<const float2*>(&stage[warp][r][2 * lane]);
-                    *reinterpret_cast<float2*>(op) = make_float2(v.y, v.x);
-                }
-            } else {
-                for (int h = lane; h < len; h += 32) {
-#pragma unroll 4
-                    for (int r = 0; r < rows; ++r) ob[(size_t)r * a.n + h] = stage[warp][r][h ^ ((r >> 4) & 1)];
-                }
-            }
-            __syncwarp();
-        }
-    }
-    if (PASS == PASS_AGG && valid) write_agg(a, op, active, seeded_ever, steps, chunk, c0, c1, li);
+    float4 cv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (PASS == PASS_EMIT && valid) cv = __ldg(reinterpret_cast<const float4*>(a.carry) + (size_t)chunk * a.n_lanes + li);
+    const float4 g = recur_span<Op, PASS>(a, group, c0, c1, cv, &stage[warp][0][0], &xin[warp][0]);
+    if (PASS == PASS_AGG && valid) *agg_slot(a, chunk, li) = g;
 }
 
 // Time-major passes: lane = series (each row of a warp is one 128-byte load or
@@ -1469,7 +1699,7 @@ __global__ void __launch_bounds__(kWarps * 32) k_recur_tm(RecurArgs a) {
         before = cur.x[kTmRows - 1];
         cur = nxt;
     }
-    if (PASS == PASS_AGG && valid) write_agg(a, op, active, seeded_ever, steps, chunk, c0, c1, li);
+    if (PASS == PASS_AGG && valid) *agg_slot(a, chunk, li) = agg_record(op, active, seeded_ever, steps, c0, c1);
 }
 
 // Carry-in of every chunk: an exclusive scan, over the chunks of one lane, of
@@ -1731,8 +1961,15 @@ vta_status run(const RecurArgs& a, cudaStream_t st) {
     const int groups = (int)ceil_div(a.n_lanes, 32);
     dim3 grid(ceil_div(groups, kWarps), n_chunks);
     if (n_chunks > 65535) return fail(VTA_ERR_LAUNCH_CONFIG_TOO_LARGE, "recurrence: too many time chunks");
-    auto agg = TM ? k_recur_tm<Op, PASS_AGG> : k_recur<Op, PASS_AGG>;
-    auto emit = TM ? k_recur_tm<Op, PASS_EMIT> : k_recur<Op, PASS_EMIT>;
+    void (*agg)(RecurArgs);
+    void (*emit)(RecurArgs);
+    if constexpr (TM) {
+        agg = k_recur_tm<Op, PASS_AGG>;
+        emit = k_recur_tm<Op, PASS_EMIT>;
+    } else {
+        agg = k_recur<Op, PASS_AGG>;
+        emit = k_recur<Op, PASS_EMIT>;
+    }
     if (n_chunks > 1) {
         agg<<<grid, kWarps * 32, 0, st>>>(a);
         VTA_TRY(check_launch("k_recur_agg"));

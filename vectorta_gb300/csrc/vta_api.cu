@@ -736,8 +736,10 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
         case I_EMA: case I_DEMA: case I_TEMA: case I_RSI: case I_WILDERS: case I_ATR: {
             // EMA/DEMA/TEMA/RSI: the last seed index of the sweep; chunks that
             // start past it run the fast aggregate pass.  With the automatic
-            // policy chunk 0 ends just past it, so that only one short chunk
-            // takes the general seeding path.
+            // policy chunk 0 ends just past it where that is shorter than a
+            // chunk, and always for TEMA, whose staged start has to run from the
+            // first bar (the others' warm-up is cut into chunks like the rest:
+            // its sums come from a prefix).
             const bool fast_kind = ind == I_EMA || ind == I_DEMA || ind == I_TEMA || ind == I_RSI;
             long long s_max = 0;
             for (int i = 0; i < nc; ++i) {
@@ -757,8 +759,10 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
                 Chunking c{};
                 c.chunk = pick_chunk(ctx, n, nc, wps);
                 c.chunk0 = c.chunk;
-                if (fast_kind && ctx->policy.recur_chunk == 0 && s_max + 1 < n)
-                    c.chunk0 = (int)std::max<long long>(64, ((s_max + 1 + 63) / 64) * 64);
+                if (fast_kind && ctx->policy.recur_chunk == 0 && s_max + 1 < n) {
+                    const long long seeds = std::max<long long>(64, ((s_max + 1 + 63) / 64) * 64);
+                    c.chunk0 = (int)(ind == I_TEMA ? seeds : std::min<long long>(seeds, c.chunk));
+                }
                 c.nch = recur_n_chunks(n, c.chunk, c.chunk0);
                 c.fast_from = c.nch;
                 for (int k = 1; k < c.nch; ++k) {
@@ -791,8 +795,12 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
             const int tc_kind = ind == I_EMA ? RK_EMA : ind == I_DEMA ? RK_DEMA : ind == I_TEMA ? RK_TEMA : RK_RSI;
             constexpr size_t kTcWsCap = size_t(1) << 30;
             auto tc_geo = [&](const Chunking& c) { return recur_agg_tc_geo(tc_kind, nc, c.chunk, c.tc_nc, ctx->num_sms); };
+            // (auto: from 2e8 outputs on, where the contraction saves more than its
+            // two launches cost; us with / without it: EMA 2..1000 on 100k bars
+            // 202 / 190, on 400k 295 / 300; TEMA 241 / 230 and 330 / 361)
+            const bool tc_worth = ctx->policy.recur_agg == 2 || n >= 1000000 || (long long)n * nc >= 200000000LL;
             auto tc_ok = [&](const Chunking& c) {
-                if (!(fast_kind && ctx->policy.recur_agg != 1 && c.nch > 1 && c.tc_nc >= 2 && c.chunk % 32 == 0 &&
+                if (!(fast_kind && tc_worth && ctx->policy.recur_agg != 1 && c.nch > 1 && c.tc_nc >= 2 && c.chunk % 32 == 0 &&
                       ctx->smem_optin >= recur_agg_tc_smem()))
                     return false;
                 const RecurTcGeo g = tc_geo(c);
