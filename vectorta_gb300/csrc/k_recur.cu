@@ -1149,7 +1149,7 @@ constexpr int kStageW = kSeg + 2;
 // predicate t > s: no accumulators, divisions or branches per lane and step
 // (the general path's per-lane phases cost about 150 cycles a step, which made
 // the seeding chunk the longest of a sweep: with the shorter first chunks that
-// this allows, EMA 2..1000 on 20,000 bars 195 -> 46 us, RSI 225 -> 64).  Used when every input of [f, tile end) is finite;
+// this allows, EMA 2..1000 on 20,000 bars 195 -> 45 us, RSI 225 -> 65).  Used when every input of [f, tile end) is finite;
 // otherwise the chunk's warm-up takes the general path.
 struct WarmTerm {
     float2 a, b;  // compensated terms of one step (b: RSI's loss)
@@ -1954,9 +1954,87 @@ __global__ void k_recur_carry(RecurArgs a, int n_chunks) {
     }
 }
 
+// Short sweeps in one launch: a block owns 32 combos and cuts the series into
+// one chunk per warp.  Every warp aggregates its chunk into shared memory,
+// composes the records of the chunks before it (its own carry-in) and emits,
+// so nothing waits for a second and third launch.  Up to kOneMax bars, where a
+// warp's chunk is still 128 steps; TEMA up to period kOneMaxTemaP (a chunk
+// inside its staged start runs from the first bar).  us of a call, three
+// launches / one: EMA of 10 periods on 1,001 bars 22.6 / 12.3, RSI 30.8 / 18.5; 200
+// periods on 2,001 bars: DEMA 24.7 / 18.5, RSI 41 / 33, on 4,001: 24.7 / 28.8
+// and 41 / 51; TEMA of 200 periods on 1,001 bars 39 / 62.
+constexpr int kOneWarps = 16;
+constexpr int kOneMax = 2048, kOneMaxTemaP = 64;
+constexpr size_t kOneSmem = (size_t)kOneWarps * (32 * kStageW * sizeof(float) + 16 * sizeof(float4) + 32 * sizeof(float4));
+
+template <class Op>
+__global__ void __launch_bounds__(32 * kOneWarps) k_recur_one(RecurArgs a) {
+    extern __shared__ __align__(16) float one_smem[];
+    float* stage = one_smem;                                                     // [kOneWarps][32][kStageW]
+    float4* xin = reinterpret_cast<float4*>(stage + kOneWarps * 32 * kStageW);  // [kOneWarps][16]
+    float4* rec = xin + kOneWarps * 16;                                         // [kOneWarps][32]
+    const int group = blockIdx.x, lane = threadIdx.x & 31, q = threadIdx.x >> 5;  // q: this warp's chunk
+    const int li = group * 32 + lane;
+    const bool valid = li < a.n_lanes;
+    const int c0 = min(q * a.chunk, a.n), c1 = min(c0 + a.chunk, a.n);
+    float* st = stage + q * 32 * kStageW;
+    float4* xi = xin + q * 16;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 g = make_float4(0.f, 0.f, 0.f, kBeforeSeed);
+    if (c1 < a.n) g = recur_span<Op, PASS_AGG>(a, group, c0, c1, zero, st, xi);  // (nobody reads the last record)
+    rec[threadIdx.x] = g;
+    // the transition of a full chunk, while other warps still aggregate
+    constexpr int N = Op::NS;
+    constexpr int SH = ShapeOf<Op>::v;
+    const int p = valid ? a.periods[li] : 1;
+    D2 ml[N][N];
+    trans_pow<Op>((long long)a.chunk, p, ml);
+    __syncthreads();
+    if (c0 >= a.n) return;
+    D2 S[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) S[r] = {0.f, 0.f};
+#pragma unroll 1
+    for (int k = 0; k < q; ++k) {
+        const float4 e = rec[k * 32 + lane];
+        if (e.w == kBeforeSeed) continue;
+        AffD<N> m;
+        chunk_map<Op>(e, p, a.chunk, ml, m);
+        D2 t[N];
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            D2 v = m.b[r];
+#pragma unroll
+            for (int c = 0; c < N; ++c)
+                if (shape_nz(SH, r, c)) v = d2_fma(m.m[r][c], S[c], v);
+            t[r] = v;
+        }
+#pragma unroll
+        for (int r = 0; r < N; ++r) S[r] = t[r];
+    }
+    float4 cv = zero;
+    cv.x = S[0].hi + S[0].lo;
+    if (N > 1) cv.y = S[N > 1 ? 1 : 0].hi + S[N > 1 ? 1 : 0].lo;
+    if (N > 2) cv.z = S[N > 2 ? 2 : 0].hi + S[N > 2 ? 2 : 0].lo;
+    recur_span<Op, PASS_EMIT>(a, group, c0, c1, cv, st, xi);
+}
+
+template <class Op>
+vta_status run_one(RecurArgs a, cudaStream_t st) {
+    a.chunk = a.chunk0 = (a.n + 64 * kOneWarps - 1) / (64 * kOneWarps) * 64;
+    VTA_CUDA_TRY(cudaFuncSetAttribute(k_recur_one<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOneSmem));
+    ktimer_begin(st);
+    k_recur_one<Op><<<ceil_div(a.n_lanes, 32), 32 * kOneWarps, kOneSmem, st>>>(a);
+    ktimer_end(st);
+    return check_launch("k_recur_one");
+}
+
 // AGG and CARRY (more than one chunk), then EMIT
 template <class Op, bool TM>
 vta_status run(const RecurArgs& a, cudaStream_t st) {
+    if constexpr (!TM) {
+        if (a.one_launch) return run_one<Op>(a, st);
+    }
     const int n_chunks = recur_n_chunks(a.n, a.chunk, a.chunk0);
     const int groups = (int)ceil_div(a.n_lanes, 32);
     dim3 grid(ceil_div(groups, kWarps), n_chunks);
@@ -1983,6 +2061,10 @@ vta_status run(const RecurArgs& a, cudaStream_t st) {
 }
 
 }  // namespace
+
+bool recur_one_ok(int kind, int n, int pmax, size_t smem_optin) {
+    return n <= kOneMax && smem_optin >= kOneSmem && (kind != RK_TEMA || pmax <= kOneMaxTemaP);
+}
 
 int recur_state_dim(int kind) {
     switch (kind) {

@@ -750,6 +750,24 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
                                     : (long long)first + p;
                 s_max = std::max(s_max, s);
             }
+            RecurArgs a{};
+            a.kind = ind == I_EMA ? RK_EMA : ind == I_DEMA ? RK_DEMA : ind == I_TEMA ? RK_TEMA
+                   : ind == I_RSI ? RK_RSI : ind == I_WILDERS ? RK_WILDERS : RK_ATR;
+            a.layout = 0;
+            a.x = in.p[0];
+            if (ind == I_ATR) { a.h = in.p[0]; a.l = in.p[1]; a.c = in.p[2]; a.x = in.p[2]; }
+            a.n = n;
+            a.first = (int)first;
+            a.n_lanes = nc;
+            a.out = out[0];
+            if (ctx->policy.recur_chunk == 0 && ctx->policy.recur_agg != 2 &&
+                recur_one_ok(a.kind, n, pmax, ctx->smem_optin)) {
+                VTA_TRY(ar.commit());
+                VTA_TRY(const_upload(ctx, periods.data(), nc, ar.take<int>(nc), &a.periods));
+                a.one_launch = 1;
+                ctx->last_kernel = "recurrence_chunked(one launch)";
+                return launch_recurrence(a, st);
+            }
             // chunking for a target of `wps` lane-warps x chunks per SM
             struct Chunking {
                 int chunk, chunk0, nch, fast_from;
@@ -846,17 +864,7 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
             void* d_tc_w = tc_any && !tc_cache ? ar.take<char>(tc_w) : nullptr;
             int* d_tc_done = tc_any ? ar.take<int>(max_nch) : nullptr;
             int* d_tc_err = tc_any ? ar.take<int>(1) : nullptr;
-            RecurArgs a{};
-            a.kind = ind == I_EMA ? RK_EMA : ind == I_DEMA ? RK_DEMA : ind == I_TEMA ? RK_TEMA
-                   : ind == I_RSI ? RK_RSI : ind == I_WILDERS ? RK_WILDERS : RK_ATR;
-            a.layout = 0;
-            a.x = in.p[0];
-            if (ind == I_ATR) { a.h = in.p[0]; a.l = in.p[1]; a.c = in.p[2]; a.x = in.p[2]; }
-            a.n = n;
-            a.first = (int)first;
             a.periods = d_per;
-            a.n_lanes = nc;
-            a.out = out[0];
             a.agg = d_agg;
             a.carry = d_carry;
             int nch_used = 1;

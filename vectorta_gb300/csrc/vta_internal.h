@@ -318,7 +318,9 @@ struct RecurArgs {
     // tensor-core partial sums of the full chunks (k_recur_tc.cu); done ==
     // null: none
     RecurTcView tc;
+    int one_launch;        // batch: AGG, carry and EMIT in one launch (recur_one_ok; no agg / carry scratch)
 };
+bool recur_one_ok(int kind, int n, int pmax, size_t smem_optin);
 vta_status launch_recurrence(const RecurArgs& a, cudaStream_t st);
 
 // Chunk aggregates of a batch EMA / DEMA / TEMA / RSI sweep as one
