@@ -24,10 +24,11 @@
 // within ~1e-7 relative of the FP64 sum.  A BF16 hi/lo variant (8-bit
 // significands, ~16 bits per operand) is selectable for comparison.
 //
-// Two kernels.  k_hankel_strips builds, once per 256-wide time tile, the hi/lo
-// strips for the largest period in the sweep (plus the tile's centring value
-// and x scale) in global memory; a combo tile of smaller period K reads the
-// same strip starting 16 * (Kmax - K) bytes in, so every combo tile shares it.
+// Two kernels.  k_wwma_prep forms the packed weight rows and, once per 256-wide
+// time tile, the hi/lo strips for the largest period in the sweep (plus the
+// tile's centring value, x scale and NaN bars) in global memory; a combo tile
+// of smaller period K reads the same strip starting 16 * (Kmax - K) bytes in, so
+// every combo tile shares it.
 // k_wwma_tc (288 threads): thread 0 bulk-copies the weights of the current
 // combo tile, then per item waits for its strip (double-buffered, cp.async.bulk + mbarrier
 // complete_tx), issues the MMAs into one of two 256-column TMEM accumulators,
@@ -48,8 +49,10 @@
 #include <cstdlib>
 #include <cstring>
 
+#include <climits>
+
 #include "tc_ops.cuh"
-#include "vta_internal.h"
+#include "wwma_weights.cuh"
 
 namespace vta {
 namespace {
@@ -74,111 +77,26 @@ __device__ __forceinline__ float qnan() { return __int_as_float(0x7fc00000); }
 // A K-major, B MN-major, N >> 3 at bit 17, M >> 4 at bit 24.
 __host__ __device__ constexpr uint32_t instr_desc(uint32_t ab_type) { return tc::instr_desc_f16(ab_type, kM, kN, 1u); }
 
-// ------------------------------------------------------------ A packing ---
-// Per combo tile m (rows c = 128 m + r): K_m = roundup16(max period), the last
-// K_m columns of the right-aligned weight matrix, scaled by 2^e_r so the row
-// maximum lies in [2^13, 2^14), split hi/lo and laid out as core matrices
-// [K_m/8][16 row groups][8 rows][8 elements].
-struct PackArgs {
-    const float* w;
-    int kmax, n_combos;
-    const int* tile_k;          // [tiles] K_m
-    const long long* tile_off;  // [tiles] offset (elements) of the hi block; lo follows
-    uint16_t* packed;
-    float* row_scale;           // [tiles*128] 2^-e_r
-    float* row_sum;             // [tiles*128] sum of the f32 weights
-};
-
-constexpr int kPackThreads = 512;
-
-template <int VARIANT>
-__global__ void __launch_bounds__(kPackThreads) k_pack_a(PackArgs a) {
-    __shared__ float sc_sh[kM];
-    const int m = blockIdx.x;
-    const int K = a.tile_k[m];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int col0 = a.kmax - K;  // weight column of k = 0 (negative: zero padding)
-    // row statistics, one warp per row (coalesced along the row): maximum
-    // magnitude and the row sum as a compensated float pair (Neumaier; an f64
-    // running sum is a chain of slow FP64 adds on GB300)
-    constexpr int kSlots = (kMaxK + 31) / 32;  // row elements per lane per pass
-    for (int r = warp; r < kM; r += kPackThreads / 32) {
-        const int c = m * kM + r;
-        float mx = 0.f, sum = 0.f, comp = 0.f;
-        if (c < a.n_combos) {
-            const float* row = a.w + (size_t)c * a.kmax;
-            for (int k0 = 0; k0 < K; k0 += 32 * kSlots) {
-                // all of the lane's loads first (independent), then the sums
-                float v[kSlots];
-#pragma unroll
-                for (int j = 0; j < kSlots; ++j) {
-                    const int k = k0 + lane + 32 * j;
-                    v[j] = (k < K && col0 + k >= 0) ? row[col0 + k] : 0.f;
-                }
-#pragma unroll
-                for (int j = 0; j < kSlots; ++j) {
-                    mx = fmaxf(mx, fabsf(v[j]));
-                    const float t = sum + v[j];
-                    comp += fabsf(sum) >= fabsf(v[j]) ? (sum - t) + v[j] : (v[j] - t) + sum;
-                    sum = t;
-                }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            const float so = __shfl_xor_sync(0xffffffffu, sum, o);
-            const float co = __shfl_xor_sync(0xffffffffu, comp, o);
-            const float t = sum + so;
-            comp += co + (fabsf(sum) >= fabsf(so) ? (sum - t) + so : (so - t) + sum);
-            sum = t;
-        }
-        if (lane == 0) {
-            int e = 0;
-            if (mx > 0.f) {
-                int ex;
-                frexpf(mx, &ex);  // mx = f * 2^ex, f in [0.5, 1)
-                e = 14 - ex;
-            }
-            sc_sh[r] = ldexpf(1.f, e);
-            a.row_scale[(size_t)m * kM + r] = mx > 0.f ? ldexpf(1.f, -e) : 0.f;
-            a.row_sum[(size_t)m * kM + r] = sum + comp;
-        }
-    }
-    __syncthreads();
-    // packed element o = ((k / 8) * 16 + g) * 64 + rr * 8 + (k % 8) of row
-    // r = 8 g + rr: consecutive threads write consecutive elements and read 8
-    // consecutive weights of one row
-    uint16_t* hi = a.packed + a.tile_off[m];
-    uint16_t* lo = hi + (size_t)kM * K;
-    const int total = kM * K;
-#pragma unroll 4
-    for (int o = threadIdx.x; o < total; o += kPackThreads) {
-        const int kb = o >> 10, rem = o & 1023;
-        const int r = ((rem >> 6) << 3) | ((rem >> 3) & 7);
-        const int k = (kb << 3) | (rem & 7);
-        const int c = m * kM + r;
-        float v = 0.f;
-        if (c < a.n_combos && col0 + k >= 0) v = a.w[(size_t)c * a.kmax + col0 + k] * sc_sh[r];
-        uint16_t h, l;
-        Split<VARIANT>::run(v, h, l);
-        hi[o] = h;
-        lo[o] = l;
-    }
-}
-
 // Warm-up / NaN masks of one staged row of 32 consecutive outputs (tiles that
 // need them are few; kept out of line so the hot epilogue loop stays small).
-// `swz` selects the 128-byte-swizzled staging layout of the TMA store path.
+// A NaN at or after the first valid bar poisons the windows that hold it
+// (nan_mode 0: the bit words of the NaN bars, 32 bars a word, are searched over
+// the window) or every later output (nan_mode 1).  `swz` selects the
+// 128-byte-swizzled staging layout of the TMA store path.
 __device__ __noinline__ void mask_staged(float* row, bool swz, int lane, int tb, int warm, int p, bool has_nan,
-                                         int n, int nan_mode, const double* nanp) {
+                                         int n, int nan_mode, int first_nan, const uint32_t* nan_bits) {
     for (int j = 0; j < 32; ++j) {
         const int t = tb + j;
         bool bad = t < warm;
-        if (!bad && has_nan && t < n) {
-            const double hi = nanp[t];
-            const double lo = (nan_mode == 0 && t - p >= 0) ? nanp[t - p] : 0.0;
-            bad = hi - lo > 0.5;
+        if (!bad && has_nan && t < n && t >= first_nan) {
+            bad = nan_mode != 0;
+            const int lo = t - p + 1;  // the window's first bar (>= first valid)
+            for (int w = t >> 5; !bad && w >= max(lo, first_nan) >> 5; --w) {
+                uint32_t m = nan_bits[w];
+                if (w == t >> 5) m &= 0xffffffffu >> (31 - (t & 31));
+                if (w == lo >> 5) m &= 0xffffffffu << (lo & 31);
+                bad = m != 0;
+            }
         }
         if (bad) {
             const int pos = swz ? ((((j >> 2) ^ (lane & 7)) << 2) | (j & 3)) : j;
@@ -187,7 +105,110 @@ __device__ __noinline__ void mask_staged(float* row, bool swz, int lane, int tb,
     }
 }
 
-// ------------------------------------------------------------ B strips ----
+// ------------------------------------------------------------ preparation -
+// One launch forms both operands: its first blocks the weight rows (A), the
+// others the Hankel strips of the time tiles (B).  (Weights, a three-pass f64
+// prefix of the NaN count, packing and strips were six launches: 38 us for 232
+// combos on 20,001 bars, now 7.3; 64 us for the 17,920-combo grid, now 25.)
+constexpr int kPrepThreads = 128;
+constexpr int kPrepRows = kPrepThreads / 32;  // weight rows per block, one warp each
+
+// Per combo tile m (rows c = 128 m + r): K_m = roundup16(max period), the
+// weights right-aligned in K_m columns, scaled by 2^e_r so the row maximum lies
+// in [2^13, 2^14), split hi/lo and laid out as core matrices
+// [K_m/8][16 row groups][8 rows][8 elements].
+struct RowArgs {
+    int kind;
+    const int* periods;
+    const double* pa;
+    const double* pb;
+    int n_combos;
+    const int* tile_k;          // [tiles] K_m
+    const long long* tile_off;  // [tiles] offset (elements) of the hi block; lo follows
+    uint16_t* packed;
+    float* row_scale;           // [tiles*128] 2^-e_r
+    float* row_sum;             // [tiles*128] sum of the f32 weights
+    int blocks, kcap;           // blocks of the launch that form rows; weights the staging holds per row
+};
+
+// A lane owns whole octets of the row (8 columns = one 16-byte piece of a core
+// matrix row), so the packed stores are 16 bytes wide.  The raw weights are
+// evaluated once, summed, and kept in shared memory for the two passes over
+// the normalised f32 weights (maximum and sum, then scale and split).
+template <int VARIANT>
+__device__ void prep_row(const RowArgs& a, int row, wts::DS* raw) {
+    const int lane = threadIdx.x & 31;
+    const int m = row / kM, r = row - m * kM;
+    const int K = a.tile_k[m];
+    uint16_t* hi = a.packed + a.tile_off[m];
+    uint16_t* lo = hi + (size_t)kM * K;
+    const bool live = row < a.n_combos;
+    const int p = live ? a.periods[row] : 0;
+    const int lead = K - p;  // zero columns before the window
+    wts::DS inv{0.f, 0.f};
+    if (live) {
+        const wts::RowConst rc = wts::row_const(a.kind, a.pa, a.pb, row);
+        wts::DS s{0.f, 0.f};
+        for (int i = lane; i < p; i += 32) {
+            const wts::DS w = wts::raw_weight(a.kind, i, p, rc);
+            raw[i] = w;
+            s = wts::ds_add(s, w);
+        }
+        inv = wts::row_inv(s);
+        __syncwarp();
+    }
+    auto weight = [&](int k) {  // the f32 weight of column k
+        const int i = k - lead;
+        if (i < 0 || i >= p) return 0.f;
+        const wts::DS v = wts::ds_mul(raw[i], inv);
+        return v.hi + v.lo;
+    };
+    // maximum magnitude and the row sum as a compensated float pair (Neumaier)
+    float mx = 0.f, sum = 0.f, comp = 0.f;
+    for (int k = lane; k < K; k += 32) {
+        const float v = weight(k);
+        mx = fmaxf(mx, fabsf(v));
+        const float t = sum + v;
+        comp += fabsf(sum) >= fabsf(v) ? (sum - t) + v : (v - t) + sum;
+        sum = t;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float so = __shfl_xor_sync(0xffffffffu, sum, o);
+        const float co = __shfl_xor_sync(0xffffffffu, comp, o);
+        const float t = sum + so;
+        comp += co + (fabsf(sum) >= fabsf(so) ? (sum - t) + so : (so - t) + sum);
+        sum = t;
+    }
+    int e = 0;
+    if (mx > 0.f) {
+        int ex;
+        frexpf(mx, &ex);  // mx = f * 2^ex, f in [0.5, 1)
+        e = 14 - ex;
+    }
+    const float sc = ldexpf(1.f, e);
+    if (lane == 0) {
+        a.row_scale[row] = mx > 0.f ? ldexpf(1.f, -e) : 0.f;
+        a.row_sum[row] = sum + comp;
+    }
+    for (int kb = lane; kb < (K >> 3); kb += 32) {
+        uint32_t h4[4], l4[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uint16_t h0, l0, h1, l1;
+            Split<VARIANT>::run(weight(8 * kb + 2 * q) * sc, h0, l0);
+            Split<VARIANT>::run(weight(8 * kb + 2 * q + 1) * sc, h1, l1);
+            h4[q] = (uint32_t)h0 | ((uint32_t)h1 << 16);
+            l4[q] = (uint32_t)l0 | ((uint32_t)l1 << 16);
+        }
+        // element ((kb * 16 + r / 8) * 8 + r % 8) * 8 of the tile
+        const size_t o = ((size_t)kb * 16 + (r >> 3)) * 64 + (r & 7) * 8;
+        *reinterpret_cast<uint4*>(hi + o) = make_uint4(h4[0], h4[1], h4[2], h4[3]);
+        *reinterpret_cast<uint4*>(lo + o) = make_uint4(l4[0], l4[1], l4[2], l4[3]);
+    }
+}
+
 // One expanded Hankel strip per 256-wide time tile, built once for the largest
 // tile K (Kmax) and shared by every combo tile: E[q] = lin[q .. q+7] (16 bytes)
 // with lin[i] = split((x[base + i] - r) * 2^e_x), base = t0 - Kmax + 1.  A
@@ -201,12 +222,12 @@ struct StripArgs {
     uint8_t* strips_lo;
     float* ref;               // [n_time_tiles] centring value r
     float* xscale;            // [n_time_tiles] 2^-e_x
+    int* tile_nan;            // [n_time_tiles] first NaN bar at or after `first` (INT_MAX: none)
+    uint32_t* nan_bits;       // [n_time_tiles * 8] the NaN bars
 };
 
 template <int VARIANT>
-__global__ void __launch_bounds__(128) k_hankel_strips(StripArgs a) {
-    extern __shared__ uint8_t sm[];
-    const int g = blockIdx.x;
+__device__ void prep_strip(const StripArgs& a, int g, uint8_t* sm) {
     const int t0 = g * kN;
     const int base = t0 - a.kmax + 1;
     const int L = a.jmax * 8 + 8;  // linear values needed
@@ -214,11 +235,23 @@ __global__ void __launch_bounds__(128) k_hankel_strips(StripArgs a) {
     uint16_t* lh = reinterpret_cast<uint16_t*>(xf + L);
     uint16_t* ll = lh + ((L + 7) & ~7);
     __shared__ float red[4];
+    __shared__ int bad[4];
+    // the tile's NaN bars
+    int nan_at = INT_MAX;
+    for (int i = threadIdx.x; i < kN; i += kPrepThreads) {
+        const int t = t0 + i;
+        const bool nan = t >= a.first && t < a.n && isnan(a.x[t]);
+        const uint32_t bits = __ballot_sync(0xffffffffu, nan);
+        if ((threadIdx.x & 31) == 0) a.nan_bits[t >> 5] = bits;
+        if (nan) nan_at = min(nan_at, t);
+    }
+    nan_at = __reduce_min_sync(0xffffffffu, nan_at);
+    if ((threadIdx.x & 31) == 0) bad[threadIdx.x >> 5] = nan_at;
     const int gref = min(t0 + kN - 1, a.n - 1);
     const float vref = (gref >= a.first && gref >= 0) ? a.x[gref] : 0.f;
     const float ref = isfinite(vref) ? vref : 0.f;
     float mx = 0.f;
-    for (int q = threadIdx.x; q < L; q += 128) {
+    for (int q = threadIdx.x; q < L; q += kPrepThreads) {
         const int gi = base + q;
         float v = __int_as_float(0x7fc00000);  // outside the series / not finite: zero after centring
         if (gi >= a.first && gi < a.n) {
@@ -240,7 +273,7 @@ __global__ void __launch_bounds__(128) k_hankel_strips(StripArgs a) {
         ex = 13 - e2;
     }
     const float sc = ldexpf(1.f, ex);
-    for (int q = threadIdx.x; q < L; q += 128) {
+    for (int q = threadIdx.x; q < L; q += kPrepThreads) {
         const float v = isnan(xf[q]) ? 0.f : (xf[q] - ref) * sc;
         uint16_t h, l;
         Split<VARIANT>::run(v, h, l);
@@ -250,13 +283,14 @@ __global__ void __launch_bounds__(128) k_hankel_strips(StripArgs a) {
     if (threadIdx.x == 0) {
         a.ref[g] = ref;
         a.xscale[g] = ldexpf(1.f, -ex);
+        a.tile_nan[g] = min(min(bad[0], bad[1]), min(bad[2], bad[3]));
     }
     __syncthreads();
     const uint32_t* wh = reinterpret_cast<const uint32_t*>(lh);
     const uint32_t* wl = reinterpret_cast<const uint32_t*>(ll);
     uint4* oh = reinterpret_cast<uint4*>(a.strips_hi + (size_t)g * a.jmax * 128);
     uint4* ol = reinterpret_cast<uint4*>(a.strips_lo + (size_t)g * a.jmax * 128);
-    for (int q = threadIdx.x; q < a.jmax * 8; q += 128) {
+    for (int q = threadIdx.x; q < a.jmax * 8; q += kPrepThreads) {
         const int w0 = q >> 1;
         uint4 h4, l4;
         if (q & 1) {
@@ -271,6 +305,17 @@ __global__ void __launch_bounds__(128) k_hankel_strips(StripArgs a) {
         oh[q] = h4;
         ol[q] = l4;
     }
+}
+
+template <int VARIANT>
+__global__ void __launch_bounds__(kPrepThreads) k_wwma_prep(RowArgs ra, StripArgs sa, int rows) {
+    extern __shared__ __align__(16) uint8_t sm[];
+    if ((int)blockIdx.x >= ra.blocks) {
+        prep_strip<VARIANT>(sa, blockIdx.x - ra.blocks, sm);
+        return;
+    }
+    const int warp = threadIdx.x >> 5, row = blockIdx.x * kPrepRows + warp;
+    if (row < rows) prep_row<VARIANT>(ra, row, reinterpret_cast<wts::DS*>(sm) + (size_t)warp * ra.kcap);
 }
 
 // ------------------------------------------------------------ main kernel -
@@ -290,13 +335,14 @@ struct TcArgs {
     const float* ref;
     const float* xscale;
     int nan_mode;
-    const double* nanp;
+    const int* tile_nan;        // [n_time_tiles] first NaN bar of the tile (INT_MAX: none)
+    const uint32_t* nan_bits;
     const int* warm_extra;  // [n_combos] extra warm-up steps (null: 0)
     float* out;
     int n_time_tiles;     // time tiles per combo tile
     int items;            // combo tiles x time tiles, combo-tile major
     int nchunks;          // items are cut into nchunks near-equal runs; CTA b takes b, b+G, ...
-    int* err;             // error word (0 = ok)
+    int* err;             // error word in mapped host memory (0 = ok)
     unsigned long long* trace;  // optional pipeline trace of CTA (0, 0): [tile][event]
 };
 // trace events per tile (globaltimer ns)
@@ -311,6 +357,7 @@ struct __align__(16) SmemCtl {
     uint64_t acc_empty[2];
     uint32_t tmem_base;
     int abort_flag;
+    int first_nan;  // first NaN bar of the series (INT_MAX: none)
     int issued;  // tiles whose MMAs were committed
 };
 
@@ -384,6 +431,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
         }
         ctl->abort_flag = 0;
         ctl->issued = 0;
+        ctl->first_nan = INT_MAX;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -550,7 +598,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
         int cur_mt = -1, p = 1, warm = 0, rbase = 0;
         float rscale = 0.f, rsum = 0.f;
         const bool vec_ok = (a.n & 3) == 0;
-        const bool has_nan = a.nanp != nullptr && a.nanp[a.n - 1] > 0.5;
+        // the first NaN bar, from the time tiles' (while the first operands load)
+        int nan_at = INT_MAX;
+        for (int g = tid - 32; g < a.n_time_tiles; g += kEpiThreads) nan_at = min(nan_at, __ldg(a.tile_nan + g));
+        nan_at = __reduce_min_sync(0xffffffffu, nan_at);
+        if (lane == 0 && nan_at != INT_MAX) atomicMin(&ctl->first_nan, nan_at);
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+        const int first_nan = ctl->first_nan;
+        const bool has_nan = first_nan != INT_MAX;
         float* st = TMA_STORE ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(stage) + (size_t)(warp - 1) * kStageTma)
                               : stage + (size_t)(warp - 1) * 32 * kStageLd;
         ItemIter it;
@@ -612,7 +667,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
                             make_float4(y[4 * j4], y[4 * j4 + 1], y[4 * j4 + 2], y[4 * j4 + 3]);
                     if (!plain)
                         mask_staged(reinterpret_cast<float*>(row8), true, lane, t0 + cb, warm, p, has_nan, a.n,
-                                    a.nan_mode, a.nanp);
+                                    a.nan_mode, first_nan, a.nan_bits);
                     // the TMA engine writes the 32 x 32 block (clipping rows / times past the ends)
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
@@ -632,7 +687,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
                             make_float4(y[4 * j4], y[4 * j4 + 1], y[4 * j4 + 2], y[4 * j4 + 3]);
                     if (!plain)
                         mask_staged(st + lane * kStageLd, false, lane, t0 + cb, warm, p, has_nan, a.n, a.nan_mode,
-                                    a.nanp);
+                                    first_nan, a.nan_bits);
                     __syncwarp();
                     // 8 lanes per row: each store instruction writes 4 rows x 128 B
                     const int c4 = lane & 7;
@@ -673,7 +728,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
             while (!mbar_try(&ctl->mma_done[last & 1], (last >> 1) & 1) && now_ns() - t0 < kWaitNs) {
             }
         }
-        if (ctl->abort_flag) atomicExch(a.err, 1);
+        if (ctl->abort_flag) {
+            *reinterpret_cast<volatile int*>(a.err) = 1;
+            __threadfence_system();
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -717,13 +775,25 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     const int n_time_tiles = (a.n + kN - 1) / kN;
     const int jmax = kbig / 8 + kN / 8 - 1;
     const size_t strip_tile = (size_t)jmax * 128;
+    // preparation: shared memory of a strip (its linear values, split) or of a
+    // block's weight rows
+    const int L = jmax * 8 + 8;
+    const size_t psmem = std::max((size_t)L * 4 + 2 * (size_t)((L + 7) & ~7) * 2 + 64,
+                                  (size_t)kPrepRows * kbig * sizeof(wts::DS));
+    if (psmem > ctx->smem_optin) return fail(VTA_ERR_NOT_IMPLEMENTED, "tcgen05 path: period above the strip limit");
+    if (!ctx->err_host) {
+        VTA_CUDA_TRY(cudaHostAlloc((void**)&ctx->err_host, sizeof(int), cudaHostAllocMapped));
+        *ctx->err_host = 0;
+    }
+    int* d_err = nullptr;
+    VTA_CUDA_TRY(cudaHostGetDevicePointer((void**)&d_err, ctx->err_host, 0));
     // operands in the context's second workspace (the first holds the
-    // caller's weights and periods during this call)
+    // caller's periods and parameters during this call)
     auto al256 = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t total = al256(n_tiles_m * sizeof(int)) + al256(n_tiles_m * sizeof(long long)) +
                          al256((size_t)off * sizeof(uint16_t)) + 2 * al256((size_t)n_tiles_m * kM * sizeof(float)) +
                          2 * al256(strip_tile * n_time_tiles) + 2 * al256(n_time_tiles * sizeof(float)) +
-                         al256(sizeof(int));
+                         al256(n_time_tiles * sizeof(int)) + al256((size_t)n_time_tiles * (kN / 32) * sizeof(uint32_t));
     void* buf = nullptr;
     VTA_TRY(ctx_aux(ctx, total, &buf));
     char* bp = static_cast<char*>(buf);
@@ -732,8 +802,8 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
         bp += al256(bytes);
         return r;
     };
-    int* d_tk = reinterpret_cast<int*>(take(n_tiles_m * sizeof(int)));
-    long long* d_toff = reinterpret_cast<long long*>(take(n_tiles_m * sizeof(long long)));
+    const int* d_tk = reinterpret_cast<int*>(take(n_tiles_m * sizeof(int)));
+    const long long* d_toff = reinterpret_cast<long long*>(take(n_tiles_m * sizeof(long long)));
     uint16_t* d_packed = reinterpret_cast<uint16_t*>(take((size_t)off * sizeof(uint16_t)));
     float* d_rs = reinterpret_cast<float*>(take((size_t)n_tiles_m * kM * sizeof(float)));
     float* d_rsum = reinterpret_cast<float*>(take((size_t)n_tiles_m * kM * sizeof(float)));
@@ -741,26 +811,19 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     uint8_t* d_sl = reinterpret_cast<uint8_t*>(take(strip_tile * n_time_tiles));
     float* d_ref = reinterpret_cast<float*>(take(n_time_tiles * sizeof(float)));
     float* d_xs = reinterpret_cast<float*>(take(n_time_tiles * sizeof(float)));
-    int* d_err = reinterpret_cast<int*>(take(sizeof(int)));
-    VTA_TRY(upload_async(ctx, d_tk, tk.data(), n_tiles_m * sizeof(int), st));
-    VTA_TRY(upload_async(ctx, d_toff, toff.data(), n_tiles_m * sizeof(long long), st));
-    VTA_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), st));
-    PackArgs pa{a.w, a.kmax, a.n_combos, d_tk, d_toff, d_packed, d_rs, d_rsum};
-    if (variant == 1) k_pack_a<1><<<n_tiles_m, kPackThreads, 0, st>>>(pa);
-    else k_pack_a<0><<<n_tiles_m, kPackThreads, 0, st>>>(pa);
-    VTA_TRY(check_launch("k_pack_a"));
-    StripArgs sa{a.x, a.n, a.first, kbig, jmax, d_sh, d_sl, d_ref, d_xs};
-    const int L = jmax * 8 + 8;
-    const size_t ssmem = (size_t)L * 4 + 2 * (size_t)((L + 7) & ~7) * 2 + 64;
-    if (ssmem > ctx->smem_optin) return fail(VTA_ERR_NOT_IMPLEMENTED, "tcgen05 path: period above the strip limit");
-    if (variant == 1) {
-        VTA_CUDA_TRY(cudaFuncSetAttribute(k_hankel_strips<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem));
-        k_hankel_strips<1><<<n_time_tiles, 128, ssmem, st>>>(sa);
-    } else {
-        VTA_CUDA_TRY(cudaFuncSetAttribute(k_hankel_strips<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssmem));
-        k_hankel_strips<0><<<n_time_tiles, 128, ssmem, st>>>(sa);
-    }
-    VTA_TRY(check_launch("k_hankel_strips"));
+    int* d_tnan = reinterpret_cast<int*>(take(n_time_tiles * sizeof(int)));
+    uint32_t* d_nbits = reinterpret_cast<uint32_t*>(take((size_t)n_time_tiles * (kN / 32) * sizeof(uint32_t)));
+    VTA_TRY(const_upload(ctx, tk.data(), tk.size(), const_cast<int*>(d_tk), &d_tk));
+    VTA_TRY(const_upload(ctx, toff.data(), toff.size(), const_cast<long long*>(d_toff), &d_toff));
+    const int rows = n_tiles_m * kM;
+    RowArgs ra{a.kind, a.periods, a.pa, a.pb, a.n_combos, d_tk, d_toff, d_packed, d_rs, d_rsum,
+               (int)ceil_div(rows, kPrepRows), kbig};
+    StripArgs sa{a.x, a.n, a.first, kbig, jmax, d_sh, d_sl, d_ref, d_xs, d_tnan, d_nbits};
+    auto prep = variant == 1 ? k_wwma_prep<1> : k_wwma_prep<0>;
+    if (psmem > 48 * 1024)
+        VTA_CUDA_TRY(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem));
+    prep<<<ra.blocks + n_time_tiles, kPrepThreads, psmem, st>>>(ra, sa, rows);
+    VTA_TRY(check_launch("k_wwma_prep"));
 
     TcArgs t{};
     t.n = a.n;
@@ -781,7 +844,8 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     t.ref = d_ref;
     t.xscale = d_xs;
     t.nan_mode = a.nan_mode;
-    t.nanp = a.nanp;
+    t.tile_nan = d_tnan;
+    t.nan_bits = d_nbits;
     t.warm_extra = a.warm_extra;
     t.out = a.out;
     t.err = d_err;
@@ -840,15 +904,11 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     kern<<<grid, kThreads, smem, st>>>(t, tmap);
     ktimer_end(st);
     VTA_TRY(check_launch("k_wwma_tc"));
-    if (ctx->async_alloc && !d_trace) {
-        // server slot: the error word is read when the request completes
-        VTA_CUDA_TRY(cudaMemcpyAsync(ctx->err_host, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        return VTA_OK;
-    }
-    int err = 0;
-    VTA_CUDA_TRY(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    // the error word is read where the host next waits for this work (tc_error,
+    // or the server when the request completes)
+    if (!d_trace) return VTA_OK;
     VTA_CUDA_TRY(cudaStreamSynchronize(st));
-    if (d_trace) {
+    {
         std::vector<unsigned long long> h(kTraceTiles * TR_N);
         cudaMemcpy(h.data(), d_trace, h.size() * 8, cudaMemcpyDeviceToHost);
         cudaFree(d_trace);
@@ -861,7 +921,6 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
             std::fprintf(stderr, "\n");
         }
     }
-    if (err) return fail(VTA_ERR_CUDA, "tcgen05 contraction: pipeline wait timed out");
     return VTA_OK;
 }
 

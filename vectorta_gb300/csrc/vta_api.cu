@@ -672,55 +672,43 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
             any_extra = any_extra || wextra[i] != 0;
             kmax = std::max(kmax, periods[i]);
         }
+        const int pol = ctx->policy.wma_batch;
+        const bool try_tc = pol == 0 || pol >= 2;
         const int ntile = (nc + 15) / 16;
-        ar.need((size_t)nc * kmax * sizeof(float));
-        ar.need(ntile * sizeof(int));
-        ar.need(len * sizeof(double));
-        ar.need(prefix_tmp_doubles(n) * sizeof(double));
         ar.need(nc * sizeof(int));
         VTA_TRY(ar.commit());
-        int* d_per = ar.take<int>(nc);
-        double* d_pa = ar.take<double>(nc);
-        double* d_pb = ar.take<double>(nc);
+        WwmaBatchArgs a{};
+        a.kind = wwma_weight_kind(ind);
+        int* per_slot = ar.take<int>(nc);
+        double* pa_slot = ar.take<double>(nc);
+        double* pb_slot = ar.take<double>(nc);
         ar.take<float>(nc);
         ar.take<float>(nc);
-        float* d_w = ar.take<float>((size_t)nc * kmax);
-        int* d_tk = ar.take<int>(ntile);
-        double* d_nanp = ar.take<double>(len);
-        double* d_tmp = ar.take<double>(prefix_tmp_doubles(n));
-        int* d_wx = ar.take<int>(nc);
+        int* wx_slot = ar.take<int>(nc);
         if (ind == I_ALMA)  // the weight kernel takes m = offset (p - 1) and 1 / (2 s^2) = sigma^2 / (2 p^2)
             for (int i = 0; i < nc; ++i) {
                 const double pd = (double)periods[i];
                 pa[i] = pa[i] * (pd - 1.0);
                 pb[i] = pb[i] * pb[i] / (2.0 * pd * pd);
             }
-        std::vector<int> tk(ntile, 0);
-        for (int i = 0; i < nc; ++i) tk[i / 16] = std::max(tk[i / 16], periods[i]);
-        VTA_TRY(upload(ctx, d_per, periods.data(), nc * sizeof(int)));
-        VTA_TRY(upload(ctx, d_pa, pa.data(), nc * sizeof(double)));
-        VTA_TRY(upload(ctx, d_pb, pb.data(), nc * sizeof(double)));
-        VTA_TRY(upload(ctx, d_tk, tk.data(), ntile * sizeof(int)));
-        if (any_extra) VTA_TRY(upload(ctx, d_wx, wextra.data(), nc * sizeof(int)));
-        VTA_TRY(launch_weights(wwma_weight_kind(ind), d_per, d_pa, d_pb, nc, kmax, d_w, st));
-        VTA_TRY(launch_prefix_f64(in.p[0], n, (int)first, PK_NAN, d_nanp, nullptr, d_tmp, st));
-        WwmaBatchArgs a{};
+        auto put = [&]() -> vta_status {
+            VTA_TRY(const_upload(ctx, periods.data(), nc, per_slot, &a.periods));
+            VTA_TRY(const_upload(ctx, pa.data(), nc, pa_slot, &a.pa));
+            VTA_TRY(const_upload(ctx, pb.data(), nc, pb_slot, &a.pb));
+            if (any_extra) VTA_TRY(const_upload(ctx, wextra.data(), nc, wx_slot, &a.warm_extra));
+            return VTA_OK;
+        };
+        VTA_TRY(put());
         a.x = in.p[0];
         a.n = n;
         a.first = (int)first;
-        a.w = d_w;
-        a.periods = d_per;
         a.periods_host = periods.data();
-        a.tile_kmax = d_tk;
         a.kmax = kmax;
         a.n_combos = nc;
         // running-sum indicators (WMA, SWMA, TRIMA) keep a NaN forever
         a.nan_mode = (ind == I_WMA || ind == I_SWMA || ind == I_TRIMA) ? 1 : 0;
-        a.nanp = d_nanp;
-        a.warm_extra = any_extra ? d_wx : nullptr;
         a.out = out[0];
-        const int pol = ctx->policy.wma_batch;
-        if (pol == 0 || pol >= 2) {
+        if (try_tc) {
             const vta_status s = launch_wwma_batch_tc(a, pol == 3 ? 1 : 0, ctx, st);
             if (s == VTA_OK) {
                 ctx->last_kernel = pol == 3 ? "wwma_tc_bf16x3" : "wwma_tc_fp16x3";
@@ -728,6 +716,34 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
             }
             if (s != VTA_ERR_NOT_IMPLEMENTED || pol >= 2) return s;
         }
+        // the plain kernel: f32 weight rows and the NaN-count prefix
+        Arena pl(ctx);
+        pl.need(nc * sizeof(int));
+        pl.need(nc * sizeof(double));
+        pl.need(nc * sizeof(double));
+        pl.need(nc * sizeof(int));
+        pl.need((size_t)nc * kmax * sizeof(float));
+        pl.need(ntile * sizeof(int));
+        pl.need(len * sizeof(double));
+        pl.need(prefix_tmp_doubles(n) * sizeof(double));
+        VTA_TRY(pl.commit());
+        per_slot = pl.take<int>(nc);
+        pa_slot = pl.take<double>(nc);
+        pb_slot = pl.take<double>(nc);
+        wx_slot = pl.take<int>(nc);
+        VTA_TRY(put());  // (the arena may have moved)
+        float* d_w = pl.take<float>((size_t)nc * kmax);
+        int* d_tk = pl.take<int>(ntile);
+        double* d_nanp = pl.take<double>(len);
+        double* d_tmp = pl.take<double>(prefix_tmp_doubles(n));
+        std::vector<int> tk(ntile, 0);
+        for (int i = 0; i < nc; ++i) tk[i / 16] = std::max(tk[i / 16], periods[i]);
+        VTA_TRY(upload(ctx, d_tk, tk.data(), ntile * sizeof(int)));
+        VTA_TRY(launch_weights(a.kind, a.periods, a.pa, a.pb, nc, kmax, d_w, st));
+        VTA_TRY(launch_prefix_f64(in.p[0], n, (int)first, PK_NAN, d_nanp, nullptr, d_tmp, st));
+        a.w = d_w;
+        a.tile_kmax = d_tk;
+        a.nanp = d_nanp;
         ctx->last_kernel = "wwma_plain_f32";
         return launch_wwma_batch_plain(a, st);
     }
@@ -1426,9 +1442,11 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
 }
 
 // ------------------------------------------------------------ drivers ------
+static vta_status tc_error(vta_ctx* ctx);
 static vta_status check_ctx(vta_ctx* ctx) {
     if (!ctx) return fail(VTA_ERR_INVALID_INPUT, "null context");
     VTA_CUDA_TRY(cudaSetDevice(ctx->device));
+    VTA_TRY(tc_error(ctx));
     g_cur = ctx;
     ctx->timed = false;
     // the pinned staging buffer is reused once the copies of the calls that
@@ -1441,8 +1459,19 @@ static vta_status check_ctx(vta_ctx* ctx) {
     return VTA_OK;
 }
 
+// A pipeline wait of the tensor-core contraction that ran out (the kernel's
+// word in mapped host memory; server slots read theirs when a request
+// completes).  Reported once, by the call that next waits for the context's
+// work or enters it.
+static vta_status tc_error(vta_ctx* ctx) {
+    if (!ctx->err_host || ctx->async_alloc || *static_cast<volatile int*>(ctx->err_host) == 0) return VTA_OK;
+    *ctx->err_host = 0;
+    return fail(VTA_ERR_CUDA, "tcgen05 contraction: pipeline wait timed out");
+}
+
 static vta_status sync(vta_ctx* ctx) {
     VTA_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    VTA_TRY(tc_error(ctx));
     return check_async("stream");
 }
 

@@ -218,14 +218,17 @@ struct WwmaBatchArgs {
     const float* x;        // series (device)
     int n;                 // series length
     int first;             // first valid index
-    const float* w;        // [n_combos][kmax] normalised weights, right-aligned
+    int kind;              // weight kind and its per-combo parameters, as launch_weights takes them
+    const double* pa;
+    const double* pb;
+    const float* w;        // [n_combos][kmax] normalised weights, right-aligned (plain kernel only)
     const int* periods;    // [n_combos]
     const int* periods_host;  // [n_combos] host copy (tile sizing)
-    const int* tile_kmax;  // per 16-combo tile: max period (K of the tile)
+    const int* tile_kmax;  // per 16-combo tile: max period (K of the tile; plain kernel only)
     int kmax;
     int n_combos;
     int nan_mode;          // 0: window NaN -> NaN; 1: NaN poisons all later outputs
-    const double* nanp;    // [n] count of NaN in x[first..i] (null: series has none)
+    const double* nanp;    // [n] count of NaN in x[first..i] (plain kernel only)
     const int* warm_extra; // [n_combos] extra warm-up steps (device; null: 0)
     float* out;            // [n_combos][n]
 };
