@@ -93,12 +93,104 @@ vta_status Arena::commit() {
     return VTA_OK;
 }
 
+// ------------------------------------------------- result arrays ----------
+// Device arrays handed to callers (vta_device_array) come from cudaMalloc, and
+// their blocks are kept for the next result when the caller frees them: a
+// cudaMalloc / cudaFree pair costs 58 to 160 us, as much as the kernels of an
+// ordinary call.  At most kArrayIdle bytes are kept per process; freed blocks go
+// back when a call finds too little free memory, and all of them with the last
+// context.  Freeing waits for the device's work, as cudaFree does, so a block
+// is never reused under a kernel, whatever stream or thread used it.
+constexpr size_t kArrayIdle = size_t(256) << 20;
+struct ArrayBlock {
+    void* ptr;
+    size_t bytes;
+    int device;
+};
+static std::mutex g_arr_mu;
+static std::map<void*, ArrayBlock> g_arr_live;   // handed out
+static std::vector<ArrayBlock> g_arr_idle;       // oldest first
+static size_t g_arr_idle_bytes = 0;
+static std::atomic<int> g_contexts{0};
+
+// Gives idle blocks back until at most `keep` bytes remain (g_arr_mu held).
+static void arrays_trim(size_t keep) {
+    int cur = 0;
+    cudaGetDevice(&cur);
+    while (!g_arr_idle.empty() && g_arr_idle_bytes > keep) {
+        const ArrayBlock b = g_arr_idle.front();
+        g_arr_idle.erase(g_arr_idle.begin());
+        g_arr_idle_bytes -= b.bytes;
+        cudaSetDevice(b.device);
+        cudaFree(b.ptr);
+    }
+    cudaSetDevice(cur);
+}
+
+// A block of at least `bytes` on the current device `device`.
+static cudaError_t array_alloc(int device, size_t bytes, void** out) {
+    std::lock_guard<std::mutex> lock(g_arr_mu);
+    const size_t most = bytes + bytes / 4 + (size_t(64) << 10);
+    for (size_t i = g_arr_idle.size(); i-- > 0;) {
+        const ArrayBlock b = g_arr_idle[i];
+        if (b.device != device || b.bytes < bytes || b.bytes > most) continue;
+        g_arr_idle.erase(g_arr_idle.begin() + (long)i);
+        g_arr_idle_bytes -= b.bytes;
+        g_arr_live[b.ptr] = b;
+        *out = b.ptr;
+        return cudaSuccess;
+    }
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e != cudaSuccess && !g_arr_idle.empty()) {
+        cudaGetLastError();
+        arrays_trim(0);
+        e = cudaMalloc(out, bytes);
+    }
+    if (e == cudaSuccess) g_arr_live[*out] = ArrayBlock{*out, bytes, device};
+    return e;
+}
+
+// Frees a result array (or any other cudaMalloc pointer) of `device`; keep:
+// its block may stay for the next result.
+cudaError_t array_free(int device, void* ptr, bool keep) {
+    int cur = 0;
+    cudaGetDevice(&cur);
+    cudaSetDevice(device);
+    cudaError_t e = cudaSuccess;
+    bool kept = false;
+    {
+        std::lock_guard<std::mutex> lock(g_arr_mu);
+        auto it = g_arr_live.find(ptr);
+        if (it != g_arr_live.end()) {
+            const ArrayBlock b = it->second;
+            g_arr_live.erase(it);
+            if (keep && b.device == device && b.bytes <= kArrayIdle / 2 && cudaDeviceSynchronize() == cudaSuccess) {
+                g_arr_idle.push_back(b);
+                g_arr_idle_bytes += b.bytes;
+                arrays_trim(kArrayIdle);
+                kept = true;
+            }
+        }
+    }
+    if (!kept) e = cudaFree(ptr);
+    cudaSetDevice(cur);
+    return e;
+}
+
 vta_status vram_check(size_t required) {
     const char* env = std::getenv("VTA_MEM_CHECK");
     if (env && (env[0] == '0' || env[0] == 'f' || env[0] == 'F')) return VTA_OK;
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return VTA_OK;
     const size_t headroom = size_t(64) << 20;
+    if (required + headroom > free_b) {
+        // give the idle result blocks back and look again
+        std::lock_guard<std::mutex> lock(g_arr_mu);
+        if (!g_arr_idle.empty()) {
+            arrays_trim(0);
+            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return VTA_OK;
+        }
+    }
     if (required + headroom > free_b) {
         char buf[160];
         std::snprintf(buf, sizeof buf, "out of memory: required=%zu free=%zu headroom=%zu", required, free_b,
@@ -1496,6 +1588,22 @@ float* pinned_device_view(const void* p, size_t bytes) {
     return reinterpret_cast<float*>(it->second.dev + off);
 }
 
+// The context's device buffer for inputs (and into-host outputs), at least
+// `need` bytes.  Calls that return device arrays use it for up to kIoInputs
+// bytes of inputs.
+constexpr size_t kIoInputs = size_t(64) << 20;
+static vta_status io_reserve(vta_ctx* ctx, size_t need) {
+    if (need <= ctx->io_bytes) return VTA_OK;
+    VTA_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (ctx->io) cudaFree(ctx->io);
+    ctx->io = nullptr;
+    ctx->io_bytes = 0;
+    VTA_TRY(vram_check(need));
+    VTA_CUDA_TRY(cudaMalloc(&ctx->io, need));
+    ctx->io_bytes = need;
+    return VTA_OK;
+}
+
 // host inputs -> device outputs (`out_dev` non-null: caller's device buffers;
 // `out_host` non-null: copy results into host buffers of out_len floats)
 static vta_status batch_host(vta_ctx* ctx, Ind ind, const float* const* hin, size_t len,
@@ -1526,39 +1634,35 @@ static vta_status batch_host(vta_ctx* ctx, Ind ind, const float* const* hin, siz
             if (!direct[k]) ++n_staged;
         }
     }
-    // into-host calls with the cached policy keep one device buffer for the
-    // inputs and outputs in the context (grown when too small), so repeated
-    // calls do not pay a cudaMalloc / cudaFree of their outputs each time
+    // with the cached policy the context keeps one device buffer (grown when too
+    // small) for the inputs, and for the outputs of into-host calls, so repeated
+    // calls do not pay a cudaMalloc / cudaFree of them each time
     const bool cached = out_host && ctx->policy.host_io == 0;
+    const bool in_kept = cached || (ctx->policy.host_io == 0 && in_bytes <= kIoInputs);
     float* d_in = nullptr;
     float* d_out[3] = {nullptr, nullptr, nullptr};
     std::unique_ptr<void, void (*)(void*)> in_guard(nullptr, [](void* p) { cudaFree(p); });
-    if (cached) {
-        const size_t in_al = (in_bytes + 255) & ~size_t(255);
-        const size_t out_al = (out_bytes + 255) & ~size_t(255);
-        const size_t need = in_al + out_al * n_staged;
-        if (need > ctx->io_bytes) {
-            VTA_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-            if (ctx->io) cudaFree(ctx->io);
-            ctx->io = nullptr;
-            ctx->io_bytes = 0;
-            VTA_TRY(vram_check(need));
-            VTA_CUDA_TRY(cudaMalloc(&ctx->io, need));
-            ctx->io_bytes = need;
-        }
+    const size_t in_al = (in_bytes + 255) & ~size_t(255);
+    const size_t out_al = (out_bytes + 255) & ~size_t(255);
+    if (in_kept) {
+        VTA_TRY(io_reserve(ctx, in_al + (cached ? out_al * n_staged : 0)));
         char* base = static_cast<char*>(ctx->io);
         d_in = reinterpret_cast<float*>(base);
-        for (int k = 0, j = 0; k < nout; ++k)
+        for (int k = 0, j = 0; cached && k < nout; ++k)
             if (!direct[k]) d_out[k] = reinterpret_cast<float*>(base + in_al + out_al * j++);
-    } else {
-        VTA_TRY(vram_check(out_bytes * n_staged + in_bytes));
-        VTA_CUDA_TRY(cudaMalloc((void**)&d_in, in_bytes));
-        in_guard.reset(d_in);
+    }
+    if (!cached) {
+        VTA_TRY(vram_check(out_bytes * n_staged + (in_kept ? 0 : in_bytes)));
+        if (!in_kept) {
+            VTA_CUDA_TRY(cudaMalloc((void**)&d_in, in_bytes));
+            in_guard.reset(d_in);
+        }
         for (int k = 0; k < nout; ++k) {
             if (direct[k]) continue;
-            cudaError_t e = cudaMalloc((void**)&d_out[k], out_bytes);
+            cudaError_t e = array_alloc(ctx->device, out_bytes, (void**)&d_out[k]);
             if (e != cudaSuccess) {
-                for (int j = 0; j < k; ++j) cudaFree(d_out[j]);
+                for (int j = 0; j < k; ++j)
+                    if (d_out[j]) array_free(ctx->device, d_out[j]);
                 return cuda_fail(e, "cudaMalloc(output)");
             }
         }
@@ -1585,7 +1689,7 @@ static vta_status batch_host(vta_ctx* ctx, Ind ind, const float* const* hin, siz
     if (s != VTA_OK || out_host) {
         if (!cached)
             for (int k = 0; k < nout; ++k)
-                if (d_out[k]) cudaFree(d_out[k]);
+                if (d_out[k]) array_free(ctx->device, d_out[k]);
         if (s != VTA_OK) return s;
     } else {
         for (int k = 0; k < nout; ++k) *out_arr[k] = vta_device_array{d_out[k], nc, len, ctx->device};
@@ -1642,10 +1746,19 @@ static vta_status tm_host(vta_ctx* ctx, Ind ind, const float* const* hin, size_t
         if (!hin[k]) return fail(VTA_ERR_INVALID_INPUT, "null input pointer");
     VTA_TRY(tm_validate_host(ind, hin, cols, rows, c));
     const size_t elems = cols * rows;
-    VTA_TRY(vram_check(elems * sizeof(float) * (nin + nout)));
+    const size_t in_bytes = elems * sizeof(float) * nin;
+    const bool in_kept = ctx->policy.host_io == 0 && in_bytes <= kIoInputs;
     float* d_in = nullptr;
-    VTA_CUDA_TRY(cudaMalloc((void**)&d_in, elems * sizeof(float) * nin));
-    std::unique_ptr<void, void (*)(void*)> in_guard(d_in, [](void* p) { cudaFree(p); });
+    std::unique_ptr<void, void (*)(void*)> in_guard(nullptr, [](void* p) { cudaFree(p); });
+    if (in_kept) {
+        VTA_TRY(io_reserve(ctx, in_bytes));
+        d_in = static_cast<float*>(ctx->io);
+    }
+    VTA_TRY(vram_check(elems * sizeof(float) * nout + (in_kept ? 0 : in_bytes)));
+    if (!in_kept) {
+        VTA_CUDA_TRY(cudaMalloc((void**)&d_in, in_bytes));
+        in_guard.reset(d_in);
+    }
     DevIn din{};
     for (int k = 0; k < nin; ++k) {
         din.p[k] = d_in + (size_t)k * elems;
@@ -1653,9 +1766,9 @@ static vta_status tm_host(vta_ctx* ctx, Ind ind, const float* const* hin, size_t
     }
     float* d_out[3] = {nullptr, nullptr, nullptr};
     for (int k = 0; k < nout; ++k) {
-        cudaError_t e = cudaMalloc((void**)&d_out[k], elems * sizeof(float));
+        cudaError_t e = array_alloc(ctx->device, elems * sizeof(float), (void**)&d_out[k]);
         if (e != cudaSuccess) {
-            for (int j = 0; j < k; ++j) cudaFree(d_out[j]);
+            for (int j = 0; j < k; ++j) array_free(ctx->device, d_out[j]);
             return cuda_fail(e, "cudaMalloc(output)");
         }
     }
@@ -1663,7 +1776,7 @@ static vta_status tm_host(vta_ctx* ctx, Ind ind, const float* const* hin, size_t
     if (s == VTA_OK) s = sync(ctx);
     cudaStreamSynchronize(ctx->stream);
     if (s != VTA_OK) {
-        for (int k = 0; k < nout; ++k) cudaFree(d_out[k]);
+        for (int k = 0; k < nout; ++k) array_free(ctx->device, d_out[k]);
         return s;
     }
     for (int k = 0; k < nout; ++k) *out_arr[k] = vta_device_array{d_out[k], rows, cols, ctx->device};
@@ -2086,6 +2199,7 @@ vta_status vta_ctx_create(int device_id, vta_ctx** out) {
     }
     const char* pol = std::getenv("VTA_WMA_BATCH");
     if (pol) vta_ctx_set_policy(c, "wma_batch", pol);
+    g_contexts.fetch_add(1);
     *out = c;
     return VTA_OK;
 }
@@ -2109,6 +2223,10 @@ vta_status vta_ctx_destroy(vta_ctx* ctx) {
     if (g_cur == ctx) g_cur = nullptr;
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
+    if (g_contexts.fetch_sub(1) == 1) {  // the last one
+        std::lock_guard<std::mutex> lock(g_arr_mu);
+        arrays_trim(0);
+    }
     return VTA_OK;
 }
 
@@ -2266,11 +2384,7 @@ size_t vta_ctx_scratch_bytes(vta_ctx* ctx) { return ctx ? ctx->scratch_bytes : 0
 
 vta_status vta_device_array_free(vta_device_array* a) {
     if (!a || !a->ptr) return VTA_OK;
-    int cur = 0;
-    cudaGetDevice(&cur);
-    cudaSetDevice(a->device);
-    cudaError_t e = cudaFree(a->ptr);
-    cudaSetDevice(cur);
+    const cudaError_t e = array_free(a->device, a->ptr);
     a->ptr = nullptr;
     a->rows = a->cols = 0;
     if (e != cudaSuccess) return cuda_fail(e, "cudaFree");

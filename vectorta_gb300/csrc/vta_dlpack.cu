@@ -59,13 +59,8 @@ struct Manager {
 
 void release(Manager* m) {
     if (!m) return;
-    if (m->data) {
-        int cur = 0;
-        cudaGetDevice(&cur);
-        cudaSetDevice(m->device);
-        cudaFree(m->data);
-        cudaSetDevice(cur);
-    }
+    // (a tensor given away goes back to the driver, not to this library's pool)
+    if (m->data) vta::array_free(m->device, m->data, false);
     std::free(m);
 }
 

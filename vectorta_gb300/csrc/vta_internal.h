@@ -33,6 +33,10 @@ vta_status cuda_fail(cudaError_t e, const char* what);
         if (_s != VTA_OK) return _s;         \
     } while (0)
 
+// Frees a result array handed to a caller (or another cudaMalloc pointer);
+// keep: its block may stay with the library for the next result.
+cudaError_t array_free(int device, void* ptr, bool keep = true);
+
 // Checks the launch that was just enqueued (and counts it).
 vta_status check_launch(const char* kernel);
 // The sticky / asynchronous error state after non-kernel work (a stream
