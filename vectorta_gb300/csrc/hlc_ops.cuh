@@ -13,6 +13,9 @@
 //   step(in, t, o1) -> o0        process t (any phase), outputs for t
 //   stepv(t, h, l, c, o1) -> o0  the same with the inputs of t given
 //   step_run(h, l, c, o1) -> o0  stepv for t >= run_from() without phase checks
+//   terms, step_terms / seed_terms, last_bar  (ADX, SuperTrend) step_run and stepv
+//                                in two parts: what depends on the bars alone,
+//                                and the rest
 //   (ADX also: wide_ok(h, l, c) and step_run<true> for tiles of up to 32 steps
 //   whose sums stay normal, with DX by the hardware reciprocal)
 // `In` provides H(t), L(t), C(t).  The arithmetic of each op is that of the
@@ -143,7 +146,8 @@ struct PAtr {
 // The arithmetic is the sequential time-major kernel's (k_adx).
 struct PAdx {
     static constexpr bool kTwo = false;
-    int p, f, dx_count;
+    static constexpr bool kFirstTr = false;
+    int p, f;
     float rp, omr, pm1;
     float atr, pdm, mdm, dx_sum, adx, ph, pl, pc;
     __device__ void init(int period, float, int first) {
@@ -156,7 +160,6 @@ struct PAdx {
     __device__ int run_from() const { return f + 2 * p; }
     __device__ void start_exact() {
         atr = pdm = mdm = dx_sum = adx = ph = pl = pc = 0.f;
-        dx_count = 0;
     }
     template <class In> __device__ void prev_inputs(const In& in, int t0) {
         ph = in.H(t0 - 1);
@@ -168,71 +171,70 @@ struct PAdx {
         atr = (float)p * (ph - pl);
         pdm = mdm = 0.f;
         adx = 0.f;
-        dx_count = p;
     }
     template <class In> __device__ void load(const float* w, const In& in, int t0) {
         atr = w[0]; pdm = w[1]; mdm = w[2]; adx = w[3];
-        dx_count = p;
         prev_inputs(in, t0);
     }
     __device__ void save(float* w) const {
         w[0] = atr; w[1] = pdm; w[2] = mdm; w[3] = adx;
         w[4] = w[5] = w[6] = w[7] = 0.f;
     }
-    __device__ float dx_now() const {
-        return adx_dx(pdm, mdm, atr);
-    }
     template <class In> __device__ float step(const In& in, int t, float& o1) {
         if (t < f) return qnan();
         return stepv(t, in.H(t), in.L(t), in.C(t), o1);
     }
-    __device__ float stepv(int t, float ch, float cl, float cc, float&) {
+    __device__ float stepv(int t, float ch, float cl, float cc, float& o1) {
         if (t < f) return qnan();
+        float tr, dp, dm;
+        terms(ch, cl, cc, ph, pl, pc, tr, dp, dm);
+        last_bar(ch, cl, cc);
+        return seed_terms(t, tr, dp, dm, o1);
+    }
+    // One step of any phase on the bar's terms (selects, see adx_dx: the lanes
+    // of a sweep are in different phases).  r counts the bars after the first:
+    // sums over r = 1..p, the mean of the DX of r = p..2p-1, then running.
+    __device__ __forceinline__ float seed_terms(int t, float tr, float dp, float dm, float&) {
         const int r = t - f;
-        float v = qnan();
-        if (r > 0) {
-            const float tr = fmaxf(fmaxf(ch - cl, fabsf(ch - pc)), fabsf(cl - pc));
-            const float up = ch - ph, down = pl - cl;
-            const float dp = (up > down && up > 0.f) ? up : 0.f;
-            const float dm = (down > up && down > 0.f) ? down : 0.f;
-            if (r <= p) {
-                atr += tr; pdm += dp; mdm += dm;
-                if (r == p) {
-                    dx_sum = dx_now();
-                    dx_count = 1;
-                }
-            } else {
-                atr = atr * omr + tr;
-                pdm = pdm * omr + dp;
-                mdm = mdm * omr + dm;
-                const float dx = dx_now();
-                if (dx_count < p) {
-                    dx_sum += dx;
-                    dx_count += 1;
-                    if (dx_count == p) { adx = dx_sum * rp; v = adx; }
-                } else {
-                    adx = (adx * pm1 + dx) * rp;
-                    v = adx;
-                }
-            }
-        }
-        ph = ch; pl = cl; pc = cc;
-        return v;
+        const bool live = r > 0;
+        const float keep = r <= p ? 1.f : omr;  // x * 1 + y is the plain sum
+        atr = fmaf(atr, keep, live ? tr : 0.f);
+        pdm = fmaf(pdm, keep, live ? dp : 0.f);
+        mdm = fmaf(mdm, keep, live ? dm : 0.f);
+        const float dx = adx_dx(pdm, mdm, atr);
+        dx_sum = r == p ? dx : dx_sum + dx;  // read at r = 2p - 1 only
+        const float run = fmaf(adx, pm1, dx) * rp;
+        const bool mean = r == 2 * p - 1 && r > p, late = r >= 2 * p;
+        adx = mean ? dx_sum * rp : late ? run : adx;
+        return mean || late ? adx : qnan();
+    }
+    // What a running step takes from the bars alone: TR, +DM, -DM.  They are the
+    // same for every combo of a sweep, so a warp of combos forms them once per
+    // bar (k_hlc_chunk.cu, k_adx_scan.cu).
+    static __device__ __forceinline__ void terms(float ch, float cl, float, float ph, float pl, float pc, float& tr,
+                                                 float& dp, float& dm) {
+        tr = fmaxf(fmaxf(ch - cl, fabsf(ch - pc)), fabsf(cl - pc));
+        const float up = ch - ph, down = pl - cl;
+        dp = (up > down && up > 0.f) ? up : 0.f;
+        dm = (down > up && down > 0.f) ? down : 0.f;
     }
     // stepv for t >= run_from(): the running update alone; WIDE: the steps
     // of a tile for which wide_ok held on every lane at its start
     template <bool WIDE = false>
-    __device__ __forceinline__ float step_run(float ch, float cl, float cc, float&) {
-        const float tr = fmaxf(fmaxf(ch - cl, fabsf(ch - pc)), fabsf(cl - pc));
-        const float up = ch - ph, down = pl - cl;
-        const float dp = (up > down && up > 0.f) ? up : 0.f;
-        const float dm = (down > up && down > 0.f) ? down : 0.f;
+    __device__ __forceinline__ float step_terms(float tr, float dp, float dm, float&) {
         atr = atr * omr + tr;
         pdm = pdm * omr + dp;
         mdm = mdm * omr + dm;
         adx = (adx * pm1 + (WIDE ? adx_dx_wide(pdm, mdm) : adx_dx(pdm, mdm, atr))) * rp;
-        ph = ch; pl = cl; pc = cc;
         return adx;
+    }
+    __device__ __forceinline__ void last_bar(float ch, float cl, float cc) { ph = ch; pl = cl; pc = cc; }
+    template <bool WIDE = false>
+    __device__ __forceinline__ float step_run(float ch, float cl, float cc, float& o1) {
+        float tr, dp, dm;
+        terms(ch, cl, cc, ph, pl, pc, tr, dp, dm);
+        last_bar(ch, cl, cc);
+        return step_terms<WIDE>(tr, dp, dm, o1);
     }
     static constexpr bool kWide = true;
     __device__ bool wide_ok(float xh, float xl, float xc) const {
@@ -245,6 +247,7 @@ struct PAdx {
 // The arithmetic is the sequential time-major kernel's (k_supertrend).
 struct PSuperTrend {
     static constexpr bool kTwo = true;
+    static constexpr bool kFirstTr = true;  // the first valid bar's TR is high - low
     int p, f;
     float alpha, fac, atr, pub, plb, last_close, pc;
     bool upper;
@@ -287,58 +290,46 @@ struct PSuperTrend {
     __device__ float stepv(int t, float hi, float lo, float cl, float& v1) {
         v1 = qnan();
         if (t < f) return qnan();
-        float tr = hi - lo;
-        if (t != f) {
-            const float hc = fabsf(hi - pc);
-            if (hc > tr) tr = hc;
-            const float lc = fabsf(lo - pc);
-            if (lc > tr) tr = lc;
-        }
-        pc = cl;
-        const int warm = f + p - 1;
-        float v0 = qnan();
-        if (t < warm) {
-            tr_sum += (double)tr;
-        } else if (t == warm) {
-            tr_sum += (double)tr;
-            atr = (float)(tr_sum / (double)p);
-            const float hl2 = (hi + lo) * 0.5f;
-            pub = hl2 + fac * atr;
-            plb = hl2 - fac * atr;
-            last_close = cl;
-            if (cl <= pub) { v0 = pub; upper = true; }
-            else { v0 = plb; upper = false; }
-            v1 = 0.f;
-        } else {
-            atr = fmaf(-alpha, atr, atr) + alpha * tr;
-            const float hl2 = (hi + lo) * 0.5f;
-            const float ub = fmaf(fac, atr, hl2);
-            const float lb = fmaf(-fac, atr, hl2);
-            float cub = ub, clb = lb;
-            if (last_close <= pub) cub = fminf(cub, pub);
-            if (last_close >= plb) clb = fmaxf(clb, plb);
-            if (upper) {
-                if (cl <= cub) { v0 = cub; v1 = 0.f; }
-                else { v0 = clb; v1 = 1.f; upper = false; }
-            } else {
-                if (cl >= clb) { v0 = clb; v1 = 0.f; }
-                else { v0 = cub; v1 = 1.f; upper = true; }
-            }
-            pub = cub; plb = clb; last_close = cl;
-        }
-        return v0;
+        float tr, hl2, c;
+        terms(hi, lo, cl, 0.f, 0.f, pc, tr, hl2, c);
+        if (t == f) tr = hi - lo;
+        last_bar(hi, lo, cl);
+        return seed_terms(t, tr, hl2, c, v1);
     }
-    // stepv for t >= run_from(): the running update alone
-    template <bool WIDE = false>  // (no division: one form)
-    __device__ __forceinline__ float step_run(float hi, float lo, float cl, float& v1) {
-        float tr = hi - lo;
+    // One step of any phase on the bar's terms (tr at the first valid bar is
+    // high - low: the caller's)
+    __device__ __forceinline__ float seed_terms(int t, float tr, float hl2, float cl, float& v1) {
+        const int warm = f + p - 1;
+        v1 = qnan();
+        if (t < f) return qnan();
+        if (t > warm) return step_terms(tr, hl2, cl, v1);
+        tr_sum += (double)tr;
+        if (t < warm) return qnan();
+        atr = (float)(tr_sum / (double)p);
+        // (product and sum rounded one by one, as the sequential kernel does)
+        const float band = __fmul_rn(fac, atr);
+        pub = __fadd_rn(hl2, band);
+        plb = __fsub_rn(hl2, band);
+        last_close = cl;
+        upper = cl <= pub;
+        v1 = 0.f;
+        return upper ? pub : plb;
+    }
+    // What a running step takes from the bars alone: TR, (high + low) / 2, close
+    static __device__ __forceinline__ void terms(float hi, float lo, float cl, float, float, float pc, float& tr,
+                                                 float& hl2, float& c) {
+        tr = hi - lo;
         const float hc = fabsf(hi - pc);
         if (hc > tr) tr = hc;
         const float lc = fabsf(lo - pc);
         if (lc > tr) tr = lc;
-        pc = cl;
+        hl2 = (hi + lo) * 0.5f;
+        c = cl;
+    }
+    // stepv for t >= run_from(): the running update alone
+    template <bool WIDE = false>  // (no division: one form)
+    __device__ __forceinline__ float step_terms(float tr, float hl2, float cl, float& v1) {
         atr = fmaf(-alpha, atr, atr) + alpha * tr;
-        const float hl2 = (hi + lo) * 0.5f;
         float cub = fmaf(fac, atr, hl2), clb = fmaf(-fac, atr, hl2);
         if (last_close <= pub) cub = fminf(cub, pub);
         if (last_close >= plb) clb = fmaxf(clb, plb);
@@ -349,6 +340,14 @@ struct PSuperTrend {
         v1 = hold ? 0.f : 1.f;
         pub = cub; plb = clb; last_close = cl;
         return upper ? cub : clb;
+    }
+    __device__ __forceinline__ void last_bar(float, float, float cl) { pc = cl; }
+    template <bool WIDE = false>
+    __device__ __forceinline__ float step_run(float hi, float lo, float cl, float& v1) {
+        float tr, hl2, c;
+        terms(hi, lo, cl, 0.f, 0.f, pc, tr, hl2, c);
+        last_bar(hi, lo, cl);
+        return step_terms(tr, hl2, c, v1);
     }
 };
 

@@ -12,10 +12,15 @@
 // (bit for bit) from its predecessor's end state.  Results are therefore
 // bit-identical to the sequential kernels.
 //
-// A warp owns one (group, chunk) item.  The shared inputs of each 32-step tile
-// are loaded once per warp (lane j loads step tb + j, one coalesced 128-byte
-// row per array) and broadcast step by step with shuffles; outputs are staged
-// per warp in shared memory and written as 32 rows x 128 bytes.
+// A warp owns one (group, chunk) item.  What a step takes from the bars alone
+// (TR, +DM, -DM; TR, (high + low) / 2, close) is the same for every combo, so
+// each lane forms it for one bar of a 32-step tile and the warp reads it back
+// from shared memory, four steps per 16-byte broadcast load; the next tile's
+// bars are on their way meanwhile.  Outputs are staged per warp in shared
+// memory and written as 32 rows x 128 bytes, unrolled.  Seeding steps are
+// selects, no branches: a 400-period seeding run is 900 of them in one chain.
+// Bound by the chain of one or two warps per scheduler (about 16 instructions
+// a step): ADX periods 2..97 on 1M bars 361 -> 177 us with these four.
 #include <algorithm>
 #include <type_traits>
 
@@ -48,7 +53,7 @@ template <class Op>
 __global__ void __launch_bounds__(kCW * 32) k_hlc_chunk(HlcChunkArgs a) {
     __shared__ float stage0[kCW][32][33];
     __shared__ float stage1[kCW][Op::kTwo ? 32 : 1][33];
-    __shared__ float4 xin[kCW][3][8];  // a running tile's high, low and close
+    __shared__ float4 xin[kCW][3][8];  // a running tile's terms
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int item = blockIdx.x * kCW + warp;
     if (item >= a.n_items) return;
@@ -76,77 +81,109 @@ __global__ void __launch_bounds__(kCW * 32) k_hlc_chunk(HlcChunkArgs a) {
     // from rf on every lane of the warp is in its running phase
     const int rf = __reduce_max_sync(0xffffffffu, op.run_from());
     // tiles of 32 steps over [tb0, tend); with `emit` the outputs go to the rows
-    auto tiles = [&](int tb0, int tend, bool emit) {
+    // (the next tile's bars are loaded while this one is worked on)
+    const int rows = min(32, a.n_combos - g * 32);
+    auto tiles = [&](int tb0, int tend, auto emit_tag) {
+        constexpr bool emit = decltype(emit_tag)::value;
+        float nh = 0.f, nl = 0.f, nc = 0.f;
+        auto fetch = [&](int t) {
+            if (t < tend) {
+                nh = __ldg(a.h + t);
+                nl = __ldg(a.l + t);
+                nc = __ldg(a.c + t);
+            }
+        };
+        fetch(tb0 + lane);
+        // the bar before the tile (unused before the first valid bar)
+        float lh = 0.f, ll = 0.f, lcl = 0.f;
+        if (tb0 > 0 && tb0 < tend) {
+            lh = __ldg(a.h + tb0 - 1);
+            ll = __ldg(a.l + tb0 - 1);
+            lcl = __ldg(a.c + tb0 - 1);
+        }
         for (int tb = tb0; tb < tend; tb += 32) {
             const int nt = min(32, tend - tb);
             const int tj = tb + lane;
-            float xh = 0.f, xl = 0.f, xc = 0.f;
-            if (lane < nt) {
-                xh = __ldg(a.h + tj);
-                xl = __ldg(a.l + tj);
-                xc = __ldg(a.c + tj);
+            const float xh = nh, xl = nl, xc = nc;
+            fetch(tj + 32);
+            // each lane forms its bar's terms (the same for every combo); the
+            // warp reads them back from shared memory, four steps per 16-byte
+            // broadcast load in a running tile
+            float ph = __shfl_up_sync(0xffffffffu, xh, 1), pl = __shfl_up_sync(0xffffffffu, xl, 1),
+                  pc = __shfl_up_sync(0xffffffffu, xc, 1);
+            if (lane == 0) {
+                ph = lh;
+                pl = ll;
+                pc = lcl;
             }
+            float u0, u1, u2;
+            Op::terms(xh, xl, xc, ph, pl, pc, u0, u1, u2);
+            if (Op::kFirstTr && tj == a.first) u0 = xh - xl;
+            float* xs = reinterpret_cast<float*>(&xin[warp][0][0]);
+            __syncwarp();  // the previous tile's reads are done
+            xs[lane] = u0;
+            xs[32 + lane] = u1;
+            xs[64 + lane] = u2;
+            __syncwarp();
+            auto put = [&](int j, float o0, float o1) {
+                if (!emit) return;
+                stage0[warp][lane][j] = o0;
+                if (Op::kTwo) stage1[warp][lane][j] = o1;
+            };
             if (tb >= rf && nt == 32) {
-                // the tile's bars from shared memory, four steps per 16-byte
-                // broadcast load
-                float* xs = reinterpret_cast<float*>(&xin[warp][0][0]);
-                __syncwarp();  // the previous tile's reads are done
-                xs[lane] = xh;
-                xs[32 + lane] = xl;
-                xs[64 + lane] = xc;
-                __syncwarp();
+                bool wide = false;
+                if constexpr (HasWide<Op>::value) wide = __all_sync(0xffffffffu, op.wide_ok(xh, xl, xc));
                 auto run32 = [&](auto wide_tag) {
-#pragma unroll 2
+#pragma unroll
                     for (int q = 0; q < 8; ++q) {
-                        const float4 h4 = xin[warp][0][q], l4 = xin[warp][1][q], c4 = xin[warp][2][q];
-                        const float hv[4] = {h4.x, h4.y, h4.z, h4.w}, lv[4] = {l4.x, l4.y, l4.z, l4.w},
+                        const float4 a4 = xin[warp][0][q], b4 = xin[warp][1][q], c4 = xin[warp][2][q];
+                        const float av[4] = {a4.x, a4.y, a4.z, a4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w},
                                     cv[4] = {c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
                             float o1;
                             const float o0 =
-                                op.template step_run<decltype(wide_tag)::value>(hv[u], lv[u], cv[u], o1);
-                            if (emit) {
-                                stage0[warp][lane][4 * q + u] = o0;
-                                if (Op::kTwo) stage1[warp][lane][4 * q + u] = o1;
-                            }
+                                op.template step_terms<decltype(wide_tag)::value>(av[u], bv[u], cv[u], o1);
+                            put(4 * q + u, o0, o1);
                         }
                     }
                 };
-                bool wide = false;
-                if constexpr (HasWide<Op>::value) wide = __all_sync(0xffffffffu, op.wide_ok(xh, xl, xc));
                 if (wide)
                     run32(std::true_type{});
                 else
                     run32(std::false_type{});
             } else {
+#pragma unroll 4
                 for (int j = 0; j < nt; ++j) {
-                    const float hv = __shfl_sync(0xffffffffu, xh, j);
-                    const float lv = __shfl_sync(0xffffffffu, xl, j);
-                    const float cv = __shfl_sync(0xffffffffu, xc, j);
                     float o1;
-                    const float o0 = op.stepv(tb + j, hv, lv, cv, o1);
-                    if (emit) {
-                        stage0[warp][lane][j] = o0;
-                        if (Op::kTwo) stage1[warp][lane][j] = o1;
-                    }
+                    const float o0 = op.seed_terms(tb + j, xs[j], xs[32 + j], xs[64 + j], o1);
+                    put(j, o0, o1);
                 }
             }
+            lh = __shfl_sync(0xffffffffu, xh, nt - 1);
+            ll = __shfl_sync(0xffffffffu, xl, nt - 1);
+            lcl = __shfl_sync(0xffffffffu, xc, nt - 1);
+            op.last_bar(lh, ll, lcl);
             if (emit) {
                 __syncwarp();
-                if (lane < nt) {
+                const size_t o = (size_t)(g * 32) * a.n + tj;
+                if (nt == 32 && rows == 32) {
+#pragma unroll
                     for (int r = 0; r < 32; ++r) {
-                        const int row = g * 32 + r;
-                        if (row >= a.n_combos) break;
-                        a.out0[(size_t)row * a.n + tj] = stage0[warp][r][lane];
-                        if (Op::kTwo) a.out1[(size_t)row * a.n + tj] = stage1[warp][r][lane];
+                        a.out0[o + (size_t)r * a.n] = stage0[warp][r][lane];
+                        if (Op::kTwo) a.out1[o + (size_t)r * a.n] = stage1[warp][r][lane];
+                    }
+                } else if (lane < nt) {
+                    for (int r = 0; r < rows; ++r) {
+                        a.out0[o + (size_t)r * a.n] = stage0[warp][r][lane];
+                        if (Op::kTwo) a.out1[o + (size_t)r * a.n] = stage1[warp][r][lane];
                     }
                 }
                 __syncwarp();
             }
         }
     };
-    tiles(t0, c0, false);
+    tiles(t0, c0, std::false_type{});
     float w[8];
     const size_t sidx = (size_t)k * a.n_combos + li;
     if (k > 0 && valid) {
@@ -154,7 +191,7 @@ __global__ void __launch_bounds__(kCW * 32) k_hlc_chunk(HlcChunkArgs a) {
         store_state(a.st_start + sidx * 8, w);
         a.exact[sidx] = warm ? 0 : 1;
     }
-    tiles(c0, c1, true);
+    tiles(c0, c1, std::true_type{});
     if (valid) {
         op.save(w);
         store_state(a.st_end + sidx * 8, w);
