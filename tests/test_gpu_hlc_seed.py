@@ -37,3 +37,16 @@ def test_seeding_is_the_sequential_one(name, sweep, lead, gap):
     seq, _ = run(name, (h, l, c), sweep, ("recur_chunk", "sequential"))
     for g, s in zip(got, seq):
         assert np.array_equal(g, s, equal_nan=True)
+
+
+@pytest.mark.parametrize("sweep", [{"period": (1, 4, 1)}, {"period": (1, 301, 100)}])
+def test_period_one_has_no_nan(sweep):
+    # period 1 keeps nothing of the bar before: +DM + -DM is 0 on inside bars,
+    # where DX is 0
+    d = datagen.ohlcv(9_001, seed=95, nan_lead=20)
+    cols = tuple(np.asarray(d[k], np.float32) for k in ("high", "low", "close"))
+    (got,), _ = run("adx", cols, sweep)
+    (seq,), _ = run("adx", cols, sweep, ("recur_chunk", "sequential"))
+    assert np.array_equal(np.isnan(got), np.isnan(seq))
+    # period 1 is DX itself: full divide or hardware reciprocal, two ulps of 100
+    assert np.nanmax(np.abs(got[0] - seq[0])) <= 2e-5

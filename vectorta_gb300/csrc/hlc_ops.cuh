@@ -58,17 +58,18 @@ __device__ __forceinline__ float rcp_approx_ftz(float x) {
 
 // Whether up to 32 running ADX steps from this state keep atr and
 // pdm + mdm normal and nonzero, given the inputs of those steps and of the
-// bar before them (x*, p*): the sums shrink by at most omr^32 >= 2^-32 and
+// bar before them (x*, p*): the sums shrink by at most omr^32 >= 2^-32 from
+// period 2 on (period 1 keeps nothing of a bar: its sums may be 0) and
 // grow by at most 32 x 2^100 when every price is within 2^98 in magnitude,
 // so sums in [2^-60, 2^100] at the start stay within [2^-92, 2^106].  On such
 // steps DX = |pdm - mdm| / (pdm + mdm) 100 needs none of adx_dx's guards
 // (adx_dx_wide).  NaN prices or sums fail the test.
-__device__ __forceinline__ bool adx_wide_ok(float atr, float pdm, float mdm, float xh, float xl, float xc,
+__device__ __forceinline__ bool adx_wide_ok(float omr, float atr, float pdm, float mdm, float xh, float xl, float xc,
                                             float ph, float pl, float pc) {
     const float s = pdm + mdm;
     const bool in_range = fabsf(xh) <= 0x1p98f && fabsf(xl) <= 0x1p98f && fabsf(xc) <= 0x1p98f &&
                           fabsf(ph) <= 0x1p98f && fabsf(pl) <= 0x1p98f && fabsf(pc) <= 0x1p98f;
-    return in_range && atr >= 0x1p-60f && atr <= 0x1p100f && s >= 0x1p-60f && s <= 0x1p100f;
+    return omr >= 0.5f && in_range && atr >= 0x1p-60f && atr <= 0x1p100f && s >= 0x1p-60f && s <= 0x1p100f;
 }
 __device__ __forceinline__ float adx_dx_wide(float pdm, float mdm) {
     return fabsf(pdm - mdm) * rcp_approx_ftz(pdm + mdm) * 100.f;
@@ -238,7 +239,7 @@ struct PAdx {
     }
     static constexpr bool kWide = true;
     __device__ bool wide_ok(float xh, float xl, float xc) const {
-        return adx_wide_ok(atr, pdm, mdm, xh, xl, xc, ph, pl, pc);
+        return adx_wide_ok(omr, atr, pdm, mdm, xh, xl, xc, ph, pl, pc);
     }
 };
 

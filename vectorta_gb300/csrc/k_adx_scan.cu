@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a) {
         // DX by the hardware reciprocal where the sums stay normal over
         // these steps (hlc::adx_wide_ok)
         const bool wide = PASS != PASS_AGG1 &&
-                          __all_sync(0xffffffffu, hlc::adx_wide_ok(atr, pdm, mdm, xh, xl, xc, ph, pl, pc));
+                          __all_sync(0xffffffffu, hlc::adx_wide_ok(ln.omr, atr, pdm, mdm, xh, xl, xc, ph, pl, pc));
         float u0, u1, u2;
         hlc::PAdx::terms(xh, xl, xc, h1, l1, c1p, u0, u1, u2);
         float* xs = reinterpret_cast<float*>(&xin[warp][0][0]);
