@@ -17,15 +17,19 @@
 //          and the second level from a zero state;
 //   CARRY2 per lane: chunk-entry ADX, adx_{k+1} = (pm1 rp)^L adx_k + b_k;
 //   EMIT   per (group, chunk): both levels from their entry states, outputs.
-// The seeding run (chunk 0, up to the group's s0) is k_hlc_chunk's exact
-// chunk-0 item.  Outputs differ from one sequential f32 pass by the rounding
+// The seeding run (chunk 0, up to the group's s0) is the exact chunk-0 item of
+// k_hlc_chunk.cu.  AGG1 needs no state, so the seeding items run in its launch;
+// the sweep's short-period groups, which depend on nothing here, run beside
+// EMIT: their chains leave issue slots that EMIT's stores wait in.  399 ADX
+// periods on 1M bars 707 -> 685 us, 101 periods of 100..400 on 200k bars
+// 182 -> 164 (own launch before the scan -> beside its passes).
+// Outputs differ from one sequential f32 pass by the rounding
 // of the composed carries (a few 1e-7 relative); a NaN bar enters the sums
 // through the same NaN-skipping max and comparisons as in the sequential
 // pass.
 #include <algorithm>
-#include <type_traits>
 
-#include "hlc_ops.cuh"
+#include "hlc_item.cuh"
 #include "vta_internal.h"
 
 namespace vta {
@@ -82,11 +86,18 @@ enum { PASS_AGG1 = 0, PASS_AGG2 = 1, PASS_EMIT = 2 };
 // AGG2 281 -> 147 (both bound by issue), EMIT 472 -> 243 (1.28 GB written, 5.3
 // TB/s).
 template <int PASS>
-__global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a) {
-    __shared__ float stage[kSW][32][33];
-    __shared__ float4 xin[kSW][3][8];  // a tile's TR, +DM and -DM
+__global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a, HlcChunkArgs c) {
+    __shared__ hlc::ItemSmem<hlc::PAdx> smem[kSW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int item = blockIdx.x * kSW + warp;
+    auto& sm = smem[warp];
+    int item = blockIdx.x * kSW + warp;
+    if (PASS != PASS_AGG2) {  // the pass's warm-restart items first
+        if (item < c.n_items) {
+            hlc::run_item<hlc::PAdx>(c, item, sm);
+            return;
+        }
+        item -= c.n_items;
+    }
     if (item >= a.n_items) return;
     const int2 it = a.items[item];
     const int gi = it.x, k = it.y;
@@ -139,7 +150,7 @@ __global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a) {
                           __all_sync(0xffffffffu, hlc::adx_wide_ok(ln.omr, atr, pdm, mdm, xh, xl, xc, ph, pl, pc));
         float u0, u1, u2;
         hlc::PAdx::terms(xh, xl, xc, h1, l1, c1p, u0, u1, u2);
-        float* xs = reinterpret_cast<float*>(&xin[warp][0][0]);
+        float* xs = reinterpret_cast<float*>(&sm.xin[0][0]);
         __syncwarp();  // the previous tile's reads are done
         xs[lane] = u0;
         xs[32 + lane] = u1;
@@ -155,13 +166,13 @@ __global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a) {
                 const float dx = WIDE ? hlc::adx_dx_wide(pdm, mdm) : hlc::adx_dx(pdm, mdm, atr);
                 adx = (adx * ln.pm1 + dx) * ln.rp;
             }
-            if (PASS == PASS_EMIT) stage[warp][lane][j] = adx;
+            if (PASS == PASS_EMIT) sm.stage0[lane][j] = adx;
         };
         auto steps = [&](auto wide_tag) {
             if (nt == 32) {
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const float4 t4 = xin[warp][0][q], p4 = xin[warp][1][q], m4 = xin[warp][2][q];
+                    const float4 t4 = sm.xin[0][q], p4 = sm.xin[1][q], m4 = sm.xin[2][q];
                     step(4 * q, t4.x, p4.x, m4.x, wide_tag);
                     step(4 * q + 1, t4.y, p4.y, m4.y, wide_tag);
                     step(4 * q + 2, t4.z, p4.z, m4.z, wide_tag);
@@ -183,9 +194,9 @@ __global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a) {
             float* o = a.out + (size_t)(g * 32) * a.n + tb + lane;
             if (nt == 32 && rows == 32) {
 #pragma unroll
-                for (int r = 0; r < 32; ++r) o[(size_t)r * a.n] = stage[warp][r][lane];
+                for (int r = 0; r < 32; ++r) o[(size_t)r * a.n] = sm.stage0[r][lane];
             } else if (lane < nt) {
-                for (int r = 0; r < rows; ++r) o[(size_t)r * a.n] = stage[warp][r][lane];
+                for (int r = 0; r < rows; ++r) o[(size_t)r * a.n] = sm.stage0[r][lane];
             }
             __syncwarp();
         }
@@ -289,20 +300,27 @@ __global__ void __launch_bounds__(128) k_adx_carry(AdxScanArgs a) {
 
 }  // namespace
 
-vta_status launch_adx_scan(const AdxScanArgs& a, cudaStream_t st) {
-    if (a.n_items <= 0) return VTA_OK;
-    const unsigned blocks = ceil_div(a.n_items, kSW);
+vta_status launch_adx_scan(const AdxScanArgs& a, const HlcChunkArgs& c, int n_seed, cudaStream_t st) {
     const unsigned cblocks = ceil_div((size_t)a.n_slots * 32, 128);  // a warp per lane slot
-    k_adx_scan<PASS_AGG1><<<blocks, kSW * 32, 0, st>>>(a);
+    HlcChunkArgs seed = c, rest = c;
+    seed.n_items = n_seed;
+    rest.items += n_seed;
+    rest.n_items -= n_seed;
+    auto blocks = [&](int extra) { return ceil_div((size_t)a.n_items + extra, kSW); };
+    ktimer_begin(st);
+    k_adx_scan<PASS_AGG1><<<blocks(seed.n_items), kSW * 32, 0, st>>>(a, seed);
     VTA_TRY(check_launch("k_adx_scan<agg1>"));
     k_adx_carry<1><<<cblocks, 128, 0, st>>>(a);
     VTA_TRY(check_launch("k_adx_carry<1>"));
-    k_adx_scan<PASS_AGG2><<<blocks, kSW * 32, 0, st>>>(a);
+    k_adx_scan<PASS_AGG2><<<blocks(0), kSW * 32, 0, st>>>(a, seed);
     VTA_TRY(check_launch("k_adx_scan<agg2>"));
     k_adx_carry<2><<<cblocks, 128, 0, st>>>(a);
     VTA_TRY(check_launch("k_adx_carry<2>"));
-    k_adx_scan<PASS_EMIT><<<blocks, kSW * 32, 0, st>>>(a);
-    return check_launch("k_adx_scan<emit>");
+    k_adx_scan<PASS_EMIT><<<blocks(rest.n_items), kSW * 32, 0, st>>>(a, rest);
+    VTA_TRY(check_launch("k_adx_scan<emit>"));
+    VTA_TRY(launch_hlc_fixup(c, st));
+    ktimer_end(st);
+    return VTA_OK;
 }
 
 }  // namespace vta

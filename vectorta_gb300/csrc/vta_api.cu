@@ -1052,7 +1052,7 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
             int max_nch = 1;
             bool chunked = false;
             std::vector<int> adx_groups, adx_s0;  // groups on the exact scan and their s0
-            int adx_L = 0;
+            int adx_L = 0, n_seed = 0;
             if (ctx->policy.recur_chunk != 1) {
                 // warm length per group: 32 p steps shrink the guessed state's
                 // error by (1 - 1/p)^(32 p) < e^-32, far below an f32 ulp, so the
@@ -1123,9 +1123,13 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
                     chunked = chunked || nch > 1;
                     for (int k = 0; k < nch; ++k) items.push_back(make_int2(g, k));
                 }
-                // longest items first (chunk + warm steps), so the long warm
-                // runs of large-period groups do not trail at the end
+                // the scan's seeding items, then the longest first (chunk +
+                // warm steps), so the long warm runs of large-period groups
+                // do not trail at the end
+                n_seed = (int)adx_groups.size();
                 std::stable_sort(items.begin(), items.end(), [&](const int2& x, const int2& y) {
+                    const bool sx = is_scan(x.x), sy = is_scan(y.x);
+                    if (sx != sy) return sx;
                     return (long long)gchunk[x.x] + gwarm[x.x] > (long long)gchunk[y.x] + gwarm[y.x];
                 });
             }
@@ -1200,8 +1204,7 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
                 c.out0 = out[0];
                 c.out1 = ind == I_SUPERTREND ? out[1] : nullptr;
                 ctx->last_kernel = ind == I_ADX ? "adx_chunked" : "supertrend_chunked";
-                VTA_TRY(launch_hlc_chunk(c, st));
-                if (adx_groups.empty()) return VTA_OK;
+                if (adx_groups.empty()) return launch_hlc_chunk(c, st);
                 AdxScanArgs x{};
                 x.h = in.p[0]; x.l = in.p[1]; x.c = in.p[2];
                 x.n = n;
@@ -1227,8 +1230,7 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
                 x.agg2 = ar.take<float>((size_t)scan_nch * scan_slots);
                 x.carry2 = ar.take<float>((size_t)scan_nch * scan_slots);
                 x.out = out[0];
-                VTA_TRY(launch_adx_scan(x, st));
-                ktimer_end(st);  // the call's timing covers the scan too
+                VTA_TRY(launch_adx_scan(x, c, n_seed, st));
                 ctx->last_kernel = "adx_chunked(" + std::to_string(adx_groups.size()) + " of " + std::to_string(G) +
                                    " groups on the exact scan, L=" + std::to_string(adx_L) + ")";
                 return VTA_OK;

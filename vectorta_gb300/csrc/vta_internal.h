@@ -406,9 +406,10 @@ struct HlcChunkArgs {
     int max_chunks;
 };
 vta_status launch_hlc_chunk(const HlcChunkArgs& a, cudaStream_t st);
+vta_status launch_hlc_fixup(const HlcChunkArgs& a, cudaStream_t st);  // its last two kernels
 // Exact chunked scan of batch ADX for 32-combo groups with long periods
 // (k_adx_scan.cu).  Group gi (combos groups[gi] * 32 ..) is seeded by
-// k_hlc_chunk's exact chunk-0 item over [0, group_s0[gi]); its chunks k >= 1
+// the exact chunk-0 item over [0, group_s0[gi]); its chunks k >= 1
 // start at group_s0[gi] + (k - 1) L.  State slots: [chunk][n_slots], slot =
 // gi * 32 + lane.
 struct AdxScanArgs {
@@ -432,7 +433,9 @@ struct AdxScanArgs {
     float* carry2;
     float* out;             // [n_combos][n]
 };
-vta_status launch_adx_scan(const AdxScanArgs& a, cudaStream_t st);
+// c: the sweep's warm-restart items, the n_seed seeding items of the scan's
+// groups first; runs them all
+vta_status launch_adx_scan(const AdxScanArgs& a, const HlcChunkArgs& c, int n_seed, cudaStream_t st);
 vta_status launch_supertrend(const HlcArgs& a, cudaStream_t st);
 
 // ------------------------------------------------- prefix-sum windows ------
