@@ -1135,8 +1135,17 @@ __device__ __forceinline__ float4* agg_slot(const RecurArgs& a, int chunk, int l
 // Staging rows are 66 floats (8-byte aligned float2 reads); rows 16..31 swap
 // the two floats of each pair (column c is stored at c ^ 1), so the per-step
 // scalar writes of the 32 lanes fall in 32 distinct banks.
-constexpr int kSeg = 64;
-constexpr int kStageW = kSeg + 2;
+//
+// Rows that do not all start at a 32-byte sector (n % 8 != 0) are CUT at the
+// sectors instead: row r writes [seg0 - m, seg0 + 64 - m), m = its segment's
+// offset into a sector, so a chunk has two partial sectors per row, not one or
+// two per segment (the L2 merges partial sectors at about half the write
+// rate).  The last m values of the segment before wait in kCarry columns in
+// front of the row.  Bound by the flush: about twice the
+// instructions of the whole-segment form.
+constexpr size_t kCutBytes = (size_t)64 << 20;
+constexpr int kSeg = 64, kCarry = 8;
+constexpr int kStageW = kSeg + 2, kCutW = kCarry + kStageW;
 
 // ------------------------------------------------------- warm-up tiles ----
 // Tiles in which some combos are still warming up.  All combos of a batch
@@ -1354,9 +1363,9 @@ __device__ __forceinline__ void warm_tile(Op& op, int f, int tb, int nt, float x
 
 // One warp's 32 lanes (combos 32 group .. 32 group + 31) over [c0, c1): AGG
 // returns the lane's record, EMIT starts from the state `cv` where the lane is
-// running and writes the outputs.  stage: 32 x kStageW floats, xin: 16 float4
-// of the warp's own (EMIT only).
-template <class Op, int PASS>
+// running and writes the outputs.  stage: 32 x (CUT ? kCutW : kStageW) floats,
+// xin: 16 float4 of the warp's own (EMIT only).
+template <class Op, int PASS, bool CUT>
 __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int c0, int c1, const float4 cv,
                                              float* stage, float4* xin) {
     const int lane = threadIdx.x & 31;
@@ -1412,7 +1421,8 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
     // this lane's staging row (batch EMIT): the current 64-step segment starts
     // at seg0, the tile at column off = tb - seg0 (0 or 32), swizzle sw
     const int sw = (lane >> 4) & 1;
-    const bool vec2 = PASS == PASS_EMIT && (a.n & 1) == 0 && (c0 & 1) == 0 &&
+    constexpr int W = CUT ? kCutW : kStageW, C0 = CUT ? kCarry : 0;
+    const bool vec2 = !CUT && PASS == PASS_EMIT && (a.n & 1) == 0 && (c0 & 1) == 0 &&
                       (reinterpret_cast<uintptr_t>(a.out) & 7) == 0;
     // writes a completed segment of the warp's 32 rows (tile [tb, te))
     auto flush = [&](int seg0, int off, int te) {
@@ -1422,22 +1432,62 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
         const int rows = min(32, a.n_lanes - row0);
         const int len = te - seg0;
         float* ob = a.out + (size_t)row0 * a.n + seg0;
-        if (vec2 && len == kSeg) {
+        if (CUT) {
+            const int m0 = (int)(reinterpret_cast<uintptr_t>(ob) >> 2);
+            const bool first = seg0 == c0, last = te == c1;
+            const float* sr = stage + kCarry + lane;
+            float* op = ob + lane;
+            if (!first && !last && rows == 32) {
+                // m repeats every 8 rows
+                int m[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) m[k] = (m0 + k * a.n) & 7;
+                op += lane;
+                sr += lane;
+#pragma unroll
+                for (int i = 0; i < 32; i += 8) {
+                    float2 v[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int x = i < 16 ? 0 : m[k] & 1 ? -1 : 1;  // the row's swizzle
+                        v[k] = make_float2(sr[(i + k) * W + x - m[k]], sr[(i + k) * W + 1 - x - m[k]]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; ++k, op += a.n) *reinterpret_cast<float2*>(op - m[k]) = v[k];
+                }
+            } else {  // a chunk's first segment has no carry, its last leaves none
+#pragma unroll 4
+                for (int r = 0; r < rows; ++r, sr += W, op += a.n) {
+                    const int m = (m0 + r * a.n) & 7, odd = (lane - m) & 1;
+                    const int x = (r >> 4) & 1 ? 1 - 2 * odd : 0;
+                    const int e = lane - m, lo = first ? 0 : -kCarry, hi = last ? len : kSeg - m;
+                    if (e >= lo && e < hi) op[-m] = sr[x - m];
+                    if (e + 32 < hi) op[32 - m] = sr[32 + x - m];
+                    if (e + 64 < hi) op[64 - m] = sr[64 + x - m];
+                }
+            }
+            __syncwarp();
+            if (te != c1) {  // the segment's last columns become the next one's carry
+                float2* row = reinterpret_cast<float2*>(stage + lane * W);
+#pragma unroll
+                for (int i = 0; i < kCarry / 2; ++i) row[i] = row[kSeg / 2 + i];
+            }
+        } else if (vec2 && len == kSeg) {
             // rows 0..15 as staged, rows 16..31 with each pair swapped back
             const int r16 = min(rows, 16);
             float* op = ob + 2 * lane;
 #pragma unroll 4
             for (int r = 0; r < r16; ++r, op += a.n)
-                *reinterpret_cast<float2*>(op) = *reinterpret_cast<const float2*>(stage + r * kStageW + 2 * lane);
+                *reinterpret_cast<float2*>(op) = *reinterpret_cast<const float2*>(stage + r * W + 2 * lane);
 #pragma unroll 4
             for (int r = 16; r < rows; ++r, op += a.n) {
-                const float2 v = *reinterpret_cast<const float2*>(stage + r * kStageW + 2 * lane);
+                const float2 v = *reinterpret_cast<const float2*>(stage + r * W + 2 * lane);
                 *reinterpret_cast<float2*>(op) = make_float2(v.y, v.x);
             }
         } else {
             for (int h = lane; h < len; h += 32) {
 #pragma unroll 4
-                for (int r = 0; r < rows; ++r) ob[(size_t)r * a.n + h] = stage[r * kStageW + (h ^ ((r >> 4) & 1))];
+                for (int r = 0; r < rows; ++r) ob[(size_t)r * a.n + h] = stage[r * W + (h ^ ((r >> 4) & 1))];
             }
         }
         __syncwarp();
@@ -1448,7 +1498,7 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
         const int te = min(tb + 32, c1);
         const int seg0 = c0 + ((tb - c0) & ~(kSeg - 1));
         const int off = tb - seg0;
-        float* srow = stage + lane * kStageW + off;
+        float* srow = stage + lane * W + C0 + off;
         // ---- general path: per-step phase logic
         rsi_fast_exit(op);  // (a no-op: general tiles come before the fast ones)
         // the tile's inputs in registers (one coalesced load per lane);
@@ -1499,7 +1549,7 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
         const int te = min(tb + 32, c1);
         const int seg0 = c0 + ((tb - c0) & ~(kSeg - 1));
         const int off = tb - seg0;
-        float* srow = stage + lane * kStageW + off;
+        float* srow = stage + lane * W + C0 + off;
         // ---- fast path: every lane running and past warm-up
         if (te - tb == 32) {
             // the tile's inputs in registers, one coalesced load per lane
@@ -1545,11 +1595,11 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
     return agg_record(op, active, seeded_ever, steps, c0, c1);
 }
 
-template <class Op, int PASS>
+template <class Op, int PASS, bool CUT = false>
 __global__ void __launch_bounds__(kWarps * 32)
 k_recur(RecurArgs a) {
     // (AGG stages the chunk's inputs in it)
-    __shared__ __align__(16) float stage[kWarps][32][PASS == PASS_EMIT ? kStageW : 33];
+    __shared__ __align__(16) float stage[kWarps][32][PASS == PASS_AGG ? 33 : CUT ? kCutW : kStageW];
     // per warp: a fast tile's broadcast inputs (EMIT), 2 x 32 floats
     __shared__ float4 xin[kWarps][PASS == PASS_EMIT ? 16 : 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1591,7 +1641,7 @@ k_recur(RecurArgs a) {
     if (group * 32 >= a.n_lanes) return;
     float4 cv = make_float4(0.f, 0.f, 0.f, 0.f);
     if (PASS == PASS_EMIT && valid) cv = __ldg(reinterpret_cast<const float4*>(a.carry) + (size_t)chunk * a.n_lanes + li);
-    const float4 g = recur_span<Op, PASS>(a, group, c0, c1, cv, &stage[warp][0][0], &xin[warp][0]);
+    const float4 g = recur_span<Op, PASS, CUT>(a, group, c0, c1, cv, &stage[warp][0][0], &xin[warp][0]);
     if (PASS == PASS_AGG && valid) *agg_slot(a, chunk, li) = g;
 }
 
@@ -1981,7 +2031,7 @@ __global__ void __launch_bounds__(32 * kOneWarps) k_recur_one(RecurArgs a) {
     float4* xi = xin + q * 16;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 g = make_float4(0.f, 0.f, 0.f, kBeforeSeed);
-    if (c1 < a.n) g = recur_span<Op, PASS_AGG>(a, group, c0, c1, zero, st, xi);  // (nobody reads the last record)
+    if (c1 < a.n) g = recur_span<Op, PASS_AGG, false>(a, group, c0, c1, zero, st, xi);  // (nobody reads the last record)
     rec[threadIdx.x] = g;
     // the transition of a full chunk, while other warps still aggregate
     constexpr int N = Op::NS;
@@ -2016,7 +2066,7 @@ __global__ void __launch_bounds__(32 * kOneWarps) k_recur_one(RecurArgs a) {
     cv.x = S[0].hi + S[0].lo;
     if (N > 1) cv.y = S[N > 1 ? 1 : 0].hi + S[N > 1 ? 1 : 0].lo;
     if (N > 2) cv.z = S[N > 2 ? 2 : 0].hi + S[N > 2 ? 2 : 0].lo;
-    recur_span<Op, PASS_EMIT>(a, group, c0, c1, cv, st, xi);
+    recur_span<Op, PASS_EMIT, false>(a, group, c0, c1, cv, st, xi);
 }
 
 template <class Op>
@@ -2046,7 +2096,16 @@ vta_status run(const RecurArgs& a, cudaStream_t st) {
         emit = k_recur_tm<Op, PASS_EMIT>;
     } else {
         agg = k_recur<Op, PASS_AGG>;
-        emit = k_recur<Op, PASS_EMIT>;
+        // Cut stores where the rows do not all start at a 16-byte boundary and
+        // the outputs are beyond what the L2 merges before it writes them back.
+        // us of a call, as they fall / cut: 399 EMAs on 500,001 bars 367 / 231
+        // (185 on 500,000), RSIs 383 / 249 (210), 199 DEMAs on 200,001 102 / 82
+        // (70), ATRs on 500,001 249 / 200; 80 MB of RSIs 58.1 / 56.3; 8 MB of
+        // EMAs 24.6 / 26.6.  Rows at 16-byte boundaries (n % 8 == 4): EMA 241 /
+        // 221, DEMA 80 / 81, ATR 194 / 199.
+        const bool cut = (a.n % 4 != 0 || reinterpret_cast<uintptr_t>(a.out) % 16 != 0) &&
+                         (size_t)a.n_lanes * a.n * sizeof(float) >= kCutBytes;
+        emit = cut ? k_recur<Op, PASS_EMIT, true> : k_recur<Op, PASS_EMIT>;
     }
     if (n_chunks > 1) {
         agg<<<grid, kWarps * 32, 0, st>>>(a);
