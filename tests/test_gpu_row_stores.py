@@ -42,3 +42,25 @@ def test_recurrence_rows(name, extra, chunk):
     for g, w in zip(got, want):
         assert g.shape[1] == n
         assert np.array_equal(g, w[:, :n], equal_nan=True)
+
+
+@pytest.mark.parametrize("gap", [None, 40_000])
+@pytest.mark.parametrize("extra", [0, 1, 2, 5])
+@pytest.mark.parametrize("name,n0,hi", [("bollinger_bands", 92_001, 254), ("sma", 200_001, 704), ("stddev", 92_001, 254)])
+def test_prefix_window_rows(name, n0, hi, extra, gap):
+    # a shifted tile may take its reference value one to seven bars away: the
+    # rows agree to a few roundings of one f32 result
+    n = n0 + extra
+    pad = (n + 7) // 8 * 8
+    sweep = {"period": (5, hi, 1), "devup": (2.0, 2.0, 0.0), "devdn": (2.0, 2.0, 0.0), "nbdev": (1.0, 1.0, 0.0)}
+    (x,) = inputs(pad, name)
+    if gap:
+        x = x.copy()
+        x[gap] = np.nan
+    want = run(name, (x,), sweep, None)
+    got = run(name, (np.ascontiguousarray(x[:n]),), sweep, None)
+    for g, w in zip(got, want):
+        w = w[:, :n]
+        assert np.array_equal(np.isnan(g), np.isnan(w))
+        d = np.abs(g - w)
+        assert np.nanmax(d / np.maximum(np.abs(w), 1.0)) <= 1e-5

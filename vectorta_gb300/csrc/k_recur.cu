@@ -1143,7 +1143,6 @@ __device__ __forceinline__ float4* agg_slot(const RecurArgs& a, int chunk, int l
 // rate).  The last m values of the segment before wait in kCarry columns in
 // front of the row.  Bound by the flush: about twice the
 // instructions of the whole-segment form.
-constexpr size_t kCutBytes = (size_t)64 << 20;
 constexpr int kSeg = 64, kCarry = 8;
 constexpr int kStageW = kSeg + 2, kCutW = kCarry + kStageW;
 

@@ -201,7 +201,7 @@ __device__ __forceinline__ void fast_outputs(const float2 (&q1)[4], const float2
     for (int k = 0; k < 4; ++k) {
         const int tk = t + k * kPwThreads;
         if (!FULL && (tk >= n || tk < warm)) {
-            if (tk < n) {
+            if (tk >= 0 && tk < n) {
                 r0[k * kPwThreads] = qnan();
                 if (K == WK_BB) { r1[k * kPwThreads] = qnan(); r2[k * kPwThreads] = qnan(); }
             }
@@ -231,24 +231,37 @@ __device__ __forceinline__ void fast_outputs(const float2 (&q1)[4], const float2
     }
 }
 
+// Rows of n floats from `out`: how far into a 32-byte sector row c starts, and
+// after how many rows that repeats.  A row cut at its sectors is written
+// [t0 - m, t0 + tile - m) by the tile at t0.
+__device__ __forceinline__ int row_shift(const float* out, int n, int c) {
+    return (int)((reinterpret_cast<uintptr_t>(out) >> 2) + (unsigned)c * (unsigned)n) & 7;
+}
+__device__ __forceinline__ int row_classes(int n) { return n & 1 ? 8 : n & 2 ? 4 : n & 4 ? 2 : 1; }
+
 constexpr int kPwComboGroup = 256;  // combos whose constants share memory holds at a time
 static_assert(kPwComboGroup <= kPwThreads, "one thread per combo of a group");
 
-template <int K>
+template <int K, bool CUT>
 __device__ void fast_tile(const PrefixWinArgs& a, const float2* s1, const float2* s2, int pmax, int t0,
                           float r0, int cb, int ce, float4* cc) {
     static_assert(kPwPer == 4, "fast_outputs is written for 4 outputs per thread");
     float2 q1[4], q2[4];
     float xt[4];
     const int tid = threadIdx.x;
+    // rows that start m floats into a sector take the tile's times m earlier
+    auto load_t = [&](int m) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int l = pmax + tid + k * kPwThreads;
-        const int t = t0 + tid + k * kPwThreads;
-        q1[k] = s1[l];
-        q2[k] = K == WK_SMA ? make_float2(0.f, 0.f) : s2[l];
-        xt[k] = (K == WK_ZSCORE && t < a.n) ? __fsub_rn(__ldg(a.x + t), r0) : 0.f;  // y(t)
-    }
+        for (int k = 0; k < 4; ++k) {
+            const int l = pmax + tid + k * kPwThreads - m;
+            const int t = t0 + tid + k * kPwThreads - m;
+            q1[k] = s1[l];
+            q2[k] = K == WK_SMA ? make_float2(0.f, 0.f) : s2[l];
+            xt[k] = (K == WK_ZSCORE && t >= 0 && t < a.n) ? __fsub_rn(__ldg(a.x + t), r0) : 0.f;  // y(t)
+        }
+    };
+    const int classes = CUT ? row_classes(a.n) : 1;
+    if (!CUT) load_t(0);
     const bool tail = t0 + kPwTile > a.n;
     for (int g0 = cb; g0 < ce; g0 += kPwComboGroup) {
         const int gn = min(kPwComboGroup, ce - g0);
@@ -259,18 +272,24 @@ __device__ void fast_tile(const PrefixWinArgs& a, const float2* s1, const float2
                                    a.k2 ? __ldg(a.k2 + c) : 1.f);
         }
         __syncthreads();
-        for (int j = 0; j < gn; ++j) {
-            const float4 k4 = cc[j];
-            const int p = __float_as_int(k4.x);
-            const int warm = a.first + p - 1;
-            const size_t o = (size_t)(g0 + j) * a.n + t0 + tid;
-            const int sh = pmax - p + tid;
-            float* o1 = a.out1 ? a.out1 + o : nullptr;
-            float* o2 = a.out2 ? a.out2 + o : nullptr;
-            if (!tail && t0 >= warm)  // the whole tile is past this combo's warm-up
-                fast_outputs<K, true>(q1, q2, xt, s1 + sh, s2 + sh, k4, r0, a.out0 + o, o1, o2, t0 + tid, a.n, warm);
-            else
-                fast_outputs<K, false>(q1, q2, xt, s1 + sh, s2 + sh, k4, r0, a.out0 + o, o1, o2, t0 + tid, a.n, warm);
+        for (int cls = 0; cls < classes; ++cls) {
+            const int m = CUT ? row_shift(a.out0, a.n, g0 + cls) : 0;
+            if (CUT) load_t(m);
+            for (int j = cls; j < gn; j += classes) {
+                const float4 k4 = cc[j];
+                const int p = __float_as_int(k4.x);
+                const int warm = a.first + p - 1;
+                const ptrdiff_t o = (ptrdiff_t)(g0 + j) * a.n + t0 + tid - m;
+                const int sh = pmax - p + tid - m;
+                float* o1 = a.out1 ? a.out1 + o : nullptr;
+                float* o2 = a.out2 ? a.out2 + o : nullptr;
+                if (!tail && t0 - m >= warm)  // the whole tile is past this combo's warm-up
+                    fast_outputs<K, true>(q1, q2, xt, s1 + sh, s2 + sh, k4, r0, a.out0 + o, o1, o2, t0 + tid - m, a.n,
+                                          warm);
+                else
+                    fast_outputs<K, false>(q1, q2, xt, s1 + sh, s2 + sh, k4, r0, a.out0 + o, o1, o2, t0 + tid - m,
+                                           a.n, warm);
+            }
         }
     }
 }
@@ -278,6 +297,7 @@ __device__ void fast_tile(const PrefixWinArgs& a, const float2* s1, const float2
 // Block (tile, g): the tile's kPwTile times for the combos [g cpb, (g + 1)
 // cpb); a tile's prefix is rebuilt by each of its combo groups (a few percent
 // of a group's work), so the grid fills the GPU in whole waves.
+template <bool CUT>
 __global__ void __launch_bounds__(kPwThreads)
 k_prefix_window_batch(PrefixWinArgs a, int pmax, int cpb) {
     extern __shared__ float2 psm[];
@@ -285,6 +305,7 @@ k_prefix_window_batch(PrefixWinArgs a, int pmax, int cpb) {
     const int cb = blockIdx.y * cpb, ce = min(a.n_combos, cb + cpb);
     __shared__ DS wsum1[kPwThreads / 32], wsum2[kPwThreads / 32];
     const int t0 = blockIdx.x * kPwTile;
+    pmax += CUT ? 8 : 0;  // (the shifted rows' slots)
     const int span = kPwTile + pmax;
     const int base = t0 - pmax;  // global index of slot 0
     const bool two = a.kind != WK_SMA;
@@ -378,10 +399,10 @@ k_prefix_window_batch(PrefixWinArgs a, int pmax, int cpb) {
             }
             __syncthreads();
             switch (a.kind) {
-                case WK_SMA: fast_tile<WK_SMA>(a, s1, s2, pmax, t0, r0, cb, ce, cc); break;
-                case WK_STDDEV: fast_tile<WK_STDDEV>(a, s1, s2, pmax, t0, r0, cb, ce, cc); break;
-                case WK_ZSCORE: fast_tile<WK_ZSCORE>(a, s1, s2, pmax, t0, r0, cb, ce, cc); break;
-                default: fast_tile<WK_BB>(a, s1, s2, pmax, t0, r0, cb, ce, cc); break;
+                case WK_SMA: fast_tile<WK_SMA, CUT>(a, s1, s2, pmax, t0, r0, cb, ce, cc); break;
+                case WK_STDDEV: fast_tile<WK_STDDEV, CUT>(a, s1, s2, pmax, t0, r0, cb, ce, cc); break;
+                case WK_ZSCORE: fast_tile<WK_ZSCORE, CUT>(a, s1, s2, pmax, t0, r0, cb, ce, cc); break;
+                default: fast_tile<WK_BB, CUT>(a, s1, s2, pmax, t0, r0, cb, ce, cc); break;
             }
             return;
         }
@@ -390,15 +411,23 @@ k_prefix_window_batch(PrefixWinArgs a, int pmax, int cpb) {
     const int first_nan = a.n - a.bad[0], first_inf = a.n - a.bad[1];
     float2 p1t[kPwPer], p2t[kPwPer];
     float xt[kPwPer];
+    int m = 0;  // the loaded times' shift (row_shift)
+    auto load_t = [&] {
 #pragma unroll
-    for (int k = 0; k < kPwPer; ++k) {
-        const int l = pmax + threadIdx.x + k * kPwThreads;  // local index of t
-        const int t = t0 + threadIdx.x + k * kPwThreads;
-        p1t[k] = s1[l];
-        p2t[k] = two ? s2[l] : z;
-        xt[k] = (a.kind == WK_ZSCORE && t < a.n) ? __fsub_rn(a.x[t], r0) : 0.f;
-    }
+        for (int k = 0; k < kPwPer; ++k) {
+            const int l = pmax + threadIdx.x + k * kPwThreads - m;  // local index of t
+            const int t = t0 + threadIdx.x + k * kPwThreads - m;
+            p1t[k] = s1[l];
+            p2t[k] = two ? s2[l] : z;
+            xt[k] = (a.kind == WK_ZSCORE && t >= 0 && t < a.n) ? __fsub_rn(a.x[t], r0) : 0.f;
+        }
+    };
+    load_t();
     for (int c = cb; c < ce; ++c) {
+        if (CUT && row_shift(a.out0, a.n, c) != m) {
+            m = row_shift(a.out0, a.n, c);
+            load_t();
+        }
         const int p = a.periods[c];
         const int warm = a.first + p - 1;
         const int poison = min(first_nan, first_inf < a.n ? first_inf + p : a.n);
@@ -409,15 +438,16 @@ k_prefix_window_batch(PrefixWinArgs a, int pmax, int cpb) {
         float* row0 = a.out0 + (size_t)c * a.n;
 #pragma unroll
         for (int k = 0; k < kPwPer; ++k) {
-            const int t = t0 + threadIdx.x + k * kPwThreads;
+            const int t = t0 + threadIdx.x + k * kPwThreads - m;
             if (t >= a.n) break;
+            if (t < 0) continue;
             const size_t o = (size_t)c * a.n + t;
             if (t < warm || t >= poison) {
                 row0[t] = qnan();
                 if (a.kind == WK_BB) { a.out1[o] = qnan(); a.out2[o] = qnan(); }
                 continue;
             }
-            const int lb = pmax + threadIdx.x + k * kPwThreads - p;  // local index of t - p
+            const int lb = pmax + threadIdx.x + k * kPwThreads - m - p;  // local index of t - p
             const DS w1 = ds_sub2(p1t[k], s1[lb]);
             const DS w2 = two ? ds_sub2_ge(p2t[k], s2[lb]) : DS{0.f, 0.f};
             WinOut r = window_eval(a.kind, w1, w2, pf, inv_p, inv_p2, xt[k], k1, k2);
@@ -1184,20 +1214,36 @@ static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_
 }
 
 vta_status launch_prefix_window_batch(const PrefixWinArgs& a, int pmax, size_t smem_optin, cudaStream_t st) {
-    const size_t smem = (size_t)(kPwTile + pmax) * sizeof(float2) * (a.kind == WK_SMA ? 1 : 2);
-    if (smem + 2 * (kPwThreads / 32) * sizeof(DS) > smem_optin)
+    const size_t fixed = 2 * (kPwThreads / 32) * sizeof(DS), slot = sizeof(float2) * (a.kind == WK_SMA ? 1 : 2);
+    size_t smem = (size_t)(kPwTile + pmax) * slot;
+    // Large outputs whose rows do not start at 16-byte boundaries: rows shifted
+    // to the sectors, every output alike.  The shifted tiles read their
+    // prefixes once per class of rows, which a short sweep does not repay.  us
+    // of a call, as they fall / cut: 250 Bollinger rows on 200,001 bars 177 /
+    // 122 (200,000: 107), on 100,001 90 / 78, on 50,001 51.5 / 51.1, on 30,001
+    // 31.6 / 34.3; SMA rows 404 / 297 (399 on 1,000,001 bars), 124 / 116 (299
+    // on 500,001), 46 / 53 (199 on 200,001); StdDev, bound by arithmetic, 183 /
+    // 200 (299 on 500,001).
+    const auto at = [](const float* o) { return reinterpret_cast<uintptr_t>(o) % 32; };
+    const int outs = a.kind == WK_BB ? 3 : 1;
+    const bool cut = (a.kind == WK_SMA || a.kind == WK_BB) && (a.n % 4 != 0 || at(a.out0) % 16 != 0) &&
+                     (outs == 1 || (at(a.out1) == at(a.out0) && at(a.out2) == at(a.out0))) &&
+                     (size_t)a.n_combos * a.n * sizeof(float) * outs >= (outs == 1 ? 8 : 4) * kCutBytes &&
+                     smem + 8 * slot + fixed <= smem_optin;
+    const auto kernel = cut ? k_prefix_window_batch<true> : k_prefix_window_batch<false>;
+    if (cut) smem += 8 * slot;
+    if (smem + fixed > smem_optin)
         return fail(VTA_ERR_LAUNCH_CONFIG_TOO_LARGE, "prefix window: period too large");
     VTA_CUDA_TRY(cudaMemsetAsync(a.bad, 0, 2 * sizeof(int), st));
     if (a.first < a.n) {
         k_first_bad<<<std::min<int>(ceil_div(a.n - a.first, 256), 4 * kNumSMs), 256, 0, st>>>(a.x, a.n, a.first, a.bad);
         VTA_TRY(check_launch("k_first_bad"));
     }
-    VTA_CUDA_TRY(cudaFuncSetAttribute(k_prefix_window_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const long long tiles = ceil_div(a.n, kPwTile);
-    const int cpb = wave_combos(k_prefix_window_batch, kPwThreads, smem, tiles, a.n_combos);
+    VTA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const long long tiles = ceil_div(a.n + (cut ? 7 : 0), kPwTile);
+    const int cpb = wave_combos(kernel, kPwThreads, smem, tiles, a.n_combos);
     ktimer_begin(st);
-    k_prefix_window_batch<<<dim3((unsigned)tiles, (unsigned)ceil_div(a.n_combos, cpb)), kPwThreads, smem, st>>>(a, pmax,
-                                                                                                              cpb);
+    kernel<<<dim3((unsigned)tiles, (unsigned)ceil_div(a.n_combos, cpb)), kPwThreads, smem, st>>>(a, pmax, cpb);
     ktimer_end(st);
     return check_launch("k_prefix_window_batch");
 }
