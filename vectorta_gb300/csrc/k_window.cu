@@ -1190,8 +1190,18 @@ __global__ void k_percentile(PnrArgs a) {
 // Combos per block for a grid of `tiles` time tiles x combo groups: the
 // grid in (nearly) whole waves of the kernel's resident blocks, counting a
 // group's per-tile set-up (prefix or table rebuild) as ~4 combos of work.
+//
+// `drift`: where that makes long blocks (over 24 combos) of a series with a
+// tile per SM or more, a few waves of shorter blocks instead, the least of
+// (waves + 1) x (combos + 6).  Blocks of one full wave set up and store in
+// step, each row of the whole series at a time; shorter ones drift apart.  us
+// of a call, one wave / a few, prefix windows: 299 SMAs on 180k, 300k and 600k
+// bars 70 / 53, 100 / 73, 188 / 131, 250 Bollinger rows 129 / 103, 196 / 155,
+// 379 / 291; below a tile per SM the reverse (80k: 27.8 / 30.5, StdDev on 120k
+// 49 / 53), and for the min/max kernels throughout (100 Williams %R on 1M bars
+// 92 / 131).
 template <class K>
-static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_combos) {
+static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_combos, bool drift = false) {
     int per_sm = 0, dev = 0, sms = kNumSMs;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess) {
         cudaGetLastError();
@@ -1199,18 +1209,24 @@ static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_
     }
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long slots = (long long)std::max(1, per_sm) * sms;
-    int best_g = 1;
-    double best = 1e300;
-    for (int g = 1; g <= 16 && g <= n_combos; ++g) {
-        const int cpb = (n_combos + g - 1) / g;
-        const long long blocks = tiles * ((n_combos + cpb - 1) / cpb);
-        const double cost = (double)((blocks + slots - 1) / slots) * (cpb + 4);
-        if (cost < best * 0.98) {
-            best = cost;
-            best_g = g;
+    const int gmax = std::min(drift ? 24 : 16, n_combos);
+    auto pick = [&](bool waves) {
+        int best_cpb = n_combos;
+        double best = 1e300;
+        for (int g = 1; g <= gmax; ++g) {
+            const int cpb = (n_combos + g - 1) / g;
+            const long long blocks = tiles * ((n_combos + cpb - 1) / cpb);
+            const double cost = waves ? (double)((blocks + slots - 1) / slots) * (cpb + 4)
+                                      : ((double)blocks / slots + 1.) * (cpb + 6);
+            if (cost < best * (waves ? 0.98 : 1.)) {
+                best = cost;
+                best_cpb = cpb;
+            }
         }
-    }
-    return (n_combos + best_g - 1) / best_g;
+        return best_cpb;
+    };
+    const int cpb = pick(true);
+    return drift && cpb > 24 && tiles >= sms ? pick(false) : cpb;
 }
 
 vta_status launch_prefix_window_batch(const PrefixWinArgs& a, int pmax, size_t smem_optin, cudaStream_t st) {
@@ -1220,8 +1236,8 @@ vta_status launch_prefix_window_batch(const PrefixWinArgs& a, int pmax, size_t s
     // to the sectors, every output alike.  The shifted tiles read their
     // prefixes once per class of rows, which a short sweep does not repay.  us
     // of a call, as they fall / cut: 250 Bollinger rows on 200,001 bars 177 /
-    // 122 (200,000: 107), on 100,001 90 / 78, on 50,001 51.5 / 51.1, on 30,001
-    // 31.6 / 34.3; SMA rows 404 / 297 (399 on 1,000,001 bars), 124 / 116 (299
+    // 111 (200,000: 102), on 100,001 90 / 78, on 50,001 51.5 / 51.1, on 30,001
+    // 31.6 / 34.3; SMA rows 404 / 270 (399 on 1,000,001 bars), 124 / 116 (299
     // on 500,001), 46 / 53 (199 on 200,001); StdDev, bound by arithmetic, 183 /
     // 200 (299 on 500,001).
     const auto at = [](const float* o) { return reinterpret_cast<uintptr_t>(o) % 32; };
@@ -1241,7 +1257,7 @@ vta_status launch_prefix_window_batch(const PrefixWinArgs& a, int pmax, size_t s
     }
     VTA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long long tiles = ceil_div(a.n + (cut ? 7 : 0), kPwTile);
-    const int cpb = wave_combos(kernel, kPwThreads, smem, tiles, a.n_combos);
+    const int cpb = wave_combos(kernel, kPwThreads, smem, tiles, a.n_combos, true);
     ktimer_begin(st);
     kernel<<<dim3((unsigned)tiles, (unsigned)ceil_div(a.n_combos, cpb)), kPwThreads, smem, st>>>(a, pmax, cpb);
     ktimer_end(st);
