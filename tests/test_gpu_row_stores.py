@@ -64,3 +64,54 @@ def test_prefix_window_rows(name, n0, hi, extra, gap):
         assert np.array_equal(np.isnan(g), np.isnan(w))
         d = np.abs(g - w)
         assert np.nanmax(d / np.maximum(np.abs(w), 1.0)) <= 1e-5
+
+
+@pytest.mark.parametrize("gap", [None, 700])
+@pytest.mark.parametrize("n", [1, 3, 29, 251, 253, 254, 257, 505, 1_537, 1_638, 2_047])
+@pytest.mark.parametrize("rows", [130, 35, 2])
+def test_tensor_core_rows(rows, n, gap):
+    # four tensor maps and 252-bar time tiles against the CUDA-core kernel, at
+    # the bound the two kernels are held to on aligned rows
+    (x,) = inputs(n, "wma")
+    x = np.where(np.isnan(x), np.float32(50), x) if n < 600 else x.copy()
+    if gap and gap < n:
+        x[gap] = np.nan
+    sweep = {"period": (1, min(rows, n - int(np.isnan(x[0])) * 33), 1)}
+    res = []
+    for policy in ("plain", "tc_fp16x3"):
+        ind = V.CLASSES["swma"](0)
+        ind.set_policy("wma_batch", policy)
+        res.append(ind.batch_dev(x, sweep=sweep).to_host())
+        assert policy == "plain" or ind.last_kernel == "wwma_tc_fp16x3"
+    w, g = res
+    assert np.array_equal(np.isnan(g), np.isnan(w))
+    d = np.abs(g - w) / np.abs(w)
+    assert np.all(np.isnan(d)) or np.nanmax(d) < 2e-6
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 5])
+@pytest.mark.parametrize("n", [2_048, 2_049])
+@pytest.mark.parametrize("name", ["wma", "ema", "sma"])
+def test_outputs_at_any_float(name, n, offset):
+    # rows written inside a larger buffer: nothing outside them changes
+    import torch
+    (x,) = inputs(n, name)
+    sweep = {"period": (5, 74, 1)}
+    rows = 70
+    ind = V.CLASSES[name](0)
+    if name == "wma":
+        ind.set_policy("wma_batch", "tc_fp16x3")
+    want = ind.batch_dev(x, sweep=sweep).to_host()
+    xd = torch.from_numpy(x).cuda()
+    buf = torch.full((rows * n + 64,), 7.0, device="cuda")
+    out = buf[16 + offset:16 + offset + rows * n]
+    torch.cuda.synchronize()
+    ind.batch_device(xd, n, 33, sweep, out)
+    ind.synchronize()
+    got = out.cpu().numpy().reshape(rows, n)
+    if name == "wma":
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+        assert np.nanmax(np.abs(got - want) / np.abs(want)) < 2e-6
+    else:
+        assert np.array_equal(got, want, equal_nan=True)
+    assert bool((buf[:16 + offset] == 7.0).all()) and bool((buf[16 + offset + rows * n:] == 7.0).all())

@@ -48,6 +48,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include <climits>
 
@@ -67,8 +68,24 @@ constexpr int kMaxK = 272;       // largest tile K whose whole A tile the shared
 constexpr int kSliceK = 256;     // K slice of a larger tile: its A slice and strip part are
                                  // copied per (item, slice) and its MMAs accumulate in TMEM
 constexpr int kStripBufs = 3;    // strip buffers: copies for items i+1 and i+2 in flight during item i
-constexpr int kStageLd = 36;     // epilogue staging row stride (floats) of the st.global path
 constexpr int kStageTma = 32 * 32 * 4;  // epilogue staging per warp for a TMA store (bytes)
+// Output rows of any length.  A tensor map's row stride is a multiple of 16
+// bytes, so rows of n floats need n % 4 == 0.  Other lengths are written
+// through four maps (PERM): map q holds the rows c = q (mod 4), whose stride 4 n
+// is a multiple of 16 bytes, from the 16-byte boundary at or before row q, m_q
+// floats before its start.  The combos of a tile are permuted so that the 32
+// accumulator rows of an epilogue warp are of one q (row 32 q + i: combo 4 i +
+// q), and a warp writes the columns from s_q = -m_q (mod 4) on, which start at
+// a boundary.  A time tile then writes 252 columns of its 256 (kNPerm), so the
+// windows of the four classes meet without a gap.  The s_q outputs before the
+// first window and those after a row's last whole 16 bytes (a map ends there:
+// TMA clips no finer) are stored one by one.
+// 232 ALMA rows on 200,001 bars 115 -> 82 us (200,000: 74), on 500,003 261 ->
+// 157 (500,000: 135); scalar stores of 16-byte strides before.
+constexpr int kNPerm = kN - 4;
+struct OutMaps {
+    CUtensorMap m[4];
+};
 constexpr uint32_t kTmemCols = 512;
 constexpr unsigned long long kWaitNs = 2000000000ull;  // 2 s per wait
 
@@ -81,9 +98,9 @@ __host__ __device__ constexpr uint32_t instr_desc(uint32_t ab_type) { return tc:
 // need them are few; kept out of line so the hot epilogue loop stays small).
 // A NaN at or after the first valid bar poisons the windows that hold it
 // (nan_mode 0: the bit words of the NaN bars, 32 bars a word, are searched over
-// the window) or every later output (nan_mode 1).  `swz` selects the
-// 128-byte-swizzled staging layout of the TMA store path.
-__device__ __noinline__ void mask_staged(float* row, bool swz, int lane, int tb, int warm, int p, bool has_nan,
+// the window) or every later output (nan_mode 1).  The staging is 128-byte
+// swizzled.
+__device__ __noinline__ void mask_staged(float* row, int lane, int tb, int warm, int p, bool has_nan,
                                          int n, int nan_mode, int first_nan, const uint32_t* nan_bits) {
     for (int j = 0; j < 32; ++j) {
         const int t = tb + j;
@@ -99,8 +116,7 @@ __device__ __noinline__ void mask_staged(float* row, bool swz, int lane, int tb,
             }
         }
         if (bad) {
-            const int pos = swz ? ((((j >> 2) ^ (lane & 7)) << 2) | (j & 3)) : j;
-            row[pos] = qnan();
+            row[(((j >> 2) ^ (lane & 7)) << 2) | (j & 3)] = qnan();
         }
     }
 }
@@ -129,6 +145,7 @@ struct RowArgs {
     float* row_scale;           // [tiles*128] 2^-e_r
     float* row_sum;             // [tiles*128] sum of the f32 weights
     int blocks, kcap;           // blocks of the launch that form rows; weights the staging holds per row
+    int perm;                   // rows in the order of the four maps
 };
 
 // A lane owns whole octets of the row (8 columns = one 16-byte piece of a core
@@ -142,12 +159,13 @@ __device__ void prep_row(const RowArgs& a, int row, wts::DS* raw) {
     const int K = a.tile_k[m];
     uint16_t* hi = a.packed + a.tile_off[m];
     uint16_t* lo = hi + (size_t)kM * K;
-    const bool live = row < a.n_combos;
-    const int p = live ? a.periods[row] : 0;
+    const int c = a.perm ? m * kM + 4 * (r & 31) + (r >> 5) : row;  // the row's combo
+    const bool live = c < a.n_combos;
+    const int p = live ? a.periods[c] : 0;
     const int lead = K - p;  // zero columns before the window
     wts::DS inv{0.f, 0.f};
     if (live) {
-        const wts::RowConst rc = wts::row_const(a.kind, a.pa, a.pb, row);
+        const wts::RowConst rc = wts::row_const(a.kind, a.pa, a.pb, c);
         wts::DS s{0.f, 0.f};
         for (int i = lane; i < p; i += 32) {
             const wts::DS w = wts::raw_weight(a.kind, i, p, rc);
@@ -218,17 +236,18 @@ struct StripArgs {
     int n, first;
     int kmax;
     int jmax;                 // strip blocks of 8 shifts: Kmax/8 + 31
+    int step;                 // bars from one time tile to the next (kN or kNPerm)
     uint8_t* strips_hi;       // [n_time_tiles][jmax * 8 * 16]
     uint8_t* strips_lo;
     float* ref;               // [n_time_tiles] centring value r
     float* xscale;            // [n_time_tiles] 2^-e_x
     int* tile_nan;            // [n_time_tiles] first NaN bar at or after `first` (INT_MAX: none)
-    uint32_t* nan_bits;       // [n_time_tiles * 8] the NaN bars
+    uint32_t* nan_bits;       // [n_time_tiles * 8] the NaN bars (of bars [g kN, g kN + kN): tile_nan, too)
 };
 
 template <int VARIANT>
 __device__ void prep_strip(const StripArgs& a, int g, uint8_t* sm) {
-    const int t0 = g * kN;
+    const int t0 = g * a.step;
     const int base = t0 - a.kmax + 1;
     const int L = a.jmax * 8 + 8;  // linear values needed
     float* xf = reinterpret_cast<float*>(sm);
@@ -236,10 +255,10 @@ __device__ void prep_strip(const StripArgs& a, int g, uint8_t* sm) {
     uint16_t* ll = lh + ((L + 7) & ~7);
     __shared__ float red[4];
     __shared__ int bad[4];
-    // the tile's NaN bars
+    // the NaN bars
     int nan_at = INT_MAX;
     for (int i = threadIdx.x; i < kN; i += kPrepThreads) {
-        const int t = t0 + i;
+        const int t = g * kN + i;
         const bool nan = t >= a.first && t < a.n && isnan(a.x[t]);
         const uint32_t bits = __ballot_sync(0xffffffffu, nan);
         if ((threadIdx.x & 31) == 0) a.nan_bits[t >> 5] = bits;
@@ -340,6 +359,7 @@ struct TcArgs {
     const int* warm_extra;  // [n_combos] extra warm-up steps (null: 0)
     float* out;
     int n_time_tiles;     // time tiles per combo tile
+    int step;             // bars from one time tile to the next
     int items;            // combo tiles x time tiles, combo-tile major
     int nchunks;          // items are cut into nchunks near-equal runs; CTA b takes b, b+G, ...
     int* err;             // error word in mapped host memory (0 = ok)
@@ -389,8 +409,8 @@ struct ItemIter {
     }
 };
 
-template <int VARIANT, bool TMA_STORE>
-__global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_constant__ CUtensorMap tmap_out) {
+template <int VARIANT, bool PERM>
+__global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_constant__ OutMaps maps) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // layout (capacities for the largest tile K): A hi | A lo | strip[kStripBufs] hi |
     // strip[kStripBufs] lo | staging (1024-aligned) | ctl
@@ -407,8 +427,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
     for (int j = 0; j < kStripBufs; ++j) strip_lo[j] = p + (size_t)j * strip_cap;
     p += kStripBufs * (size_t)strip_cap;
     p = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
-    float* stage = reinterpret_cast<float*>(p);  // [8 epilogue warps][32][kStageLd] or [8][4 KB swizzled]
-    p += (size_t)8 * 32 * kStageLd * sizeof(float);
+    uint8_t* stage = p;  // [8 epilogue warps][4 KB swizzled]
+    p += (size_t)8 * kStageTma;
     SmemCtl* ctl = reinterpret_cast<SmemCtl*>(p);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -595,9 +615,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
         const int q4 = warp & 3;
         const int half = (warp - 1) >> 2;
         const int r = q4 * 32 + lane;  // accumulator row = combo within tile
-        int cur_mt = -1, p = 1, warm = 0, rbase = 0;
+        int cur_mt = -1, c = 0, p = 1, warm = 0, rbase = 0;
         float rscale = 0.f, rsum = 0.f;
-        const bool vec_ok = (a.n & 3) == 0;
         // the first NaN bar, from the time tiles' (while the first operands load)
         int nan_at = INT_MAX;
         for (int g = tid - 32; g < a.n_time_tiles; g += kEpiThreads) nan_at = min(nan_at, __ldg(a.tile_nan + g));
@@ -606,23 +625,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
         const int first_nan = ctl->first_nan;
         const bool has_nan = first_nan != INT_MAX;
-        float* st = TMA_STORE ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(stage) + (size_t)(warp - 1) * kStageTma)
-                              : stage + (size_t)(warp - 1) * 32 * kStageLd;
+        uint8_t* row8 = stage + (size_t)(warp - 1) * kStageTma + lane * 128;  // this lane's staging row
+        // PERM: the class's rows, and where its rows start (m_q) and its windows (s_q)
+        const int mq = PERM ? (int)((reinterpret_cast<uintptr_t>(a.out) >> 2) + (unsigned)q4 * (unsigned)a.n) & 3 : 0;
+        const int sq = (4 - mq) & 3;
+        const int rows_q = PERM ? (a.n_combos - q4 + 3) >> 2 : a.n_combos;
+        const int tail = PERM ? (a.n + mq) & 3 : 0;  // outputs past the map
         ItemIter it;
         it.start(a, blockIdx.x);
         for (int i = 0; i < ntiles; ++i, it.advance(a)) {
             const int b = i & 1;
             const int mt = it.tile(a);
             const int g = it.time_tile(a);
-            const int t0 = g * kN;
+            const int t0 = g * a.step;
             if (mt != cur_mt) {
                 cur_mt = mt;
-                const int c = mt * kM + r;
+                c = mt * kM + (PERM ? 4 * lane + q4 : r);
                 p = c < a.n_combos ? a.periods[c] : 1;
                 warm = a.first + p - 1 + (a.warm_extra && c < a.n_combos ? a.warm_extra[c] : 0);
                 rscale = a.row_scale[(size_t)mt * kM + r];
                 rsum = a.row_sum[(size_t)mt * kM + r];
-                rbase = mt * kM + q4 * 32;  // first combo of this warp's rows
+                rbase = PERM ? mt * 32 : mt * kM + q4 * 32;  // first row of this warp's in its map
             }
             const float ref = __ldg(a.ref + g), xs = __ldg(a.xscale + g);
             // one lane waits, the warp follows (tcgen05.ld is warp-collective)
@@ -642,81 +665,93 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
             // tiles past every row's warm-up with a NaN-free series need no masks
             const bool plain = !has_nan && __all_sync(0xffffffffu, t0 >= warm);
             const uint32_t tbase = tmem + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(b * kN + half * 128);
+            // stages 32 of the values z at s on (128-byte swizzle: 16-byte chunk
+            // j4 of the row goes to chunk j4 ^ (lane & 7))
+            auto put = [&](const float* z, auto s_tag) {
+                constexpr int S = decltype(s_tag)::value;
+#pragma unroll
+                for (int j4 = 0; j4 < 8; ++j4)
+                    *reinterpret_cast<float4*>(row8 + ((j4 ^ (lane & 7)) << 4)) =
+                        make_float4(z[4 * j4 + S], z[4 * j4 + S + 1], z[4 * j4 + S + 2], z[4 * j4 + S + 3]);
+            };
+            auto put_at = [&](const float* z) {
+                switch (sq) {
+                    case 0: put(z, std::integral_constant<int, 0>{}); break;
+                    case 1: put(z, std::integral_constant<int, 1>{}); break;
+                    case 2: put(z, std::integral_constant<int, 2>{}); break;
+                    default: put(z, std::integral_constant<int, 3>{}); break;
+                }
+            };
             // the TMEM load of block k + 1 is issued before block k is staged, so
-            // it overlaps the wait for the previous block's TMA store
-            uint32_t v[32];
+            // it overlaps the wait for the previous block's TMA store.  PERM: a
+            // block is 32 of 36 columns, the four before (second half of the
+            // tile) or after (first half) its own loaded with it
+            const uint32_t tfour = tbase + (half ? (uint32_t)-4 : 32u);
+            uint32_t v[32], u[4];
             TC_LD32(tbase, v);
+            if (PERM) TC_LD4(tfour, u);
 #pragma unroll 1
             for (int k = 0; k < 4; ++k) {
                 TC_WAIT_LD32(v);
-                const int cb = half * 128 + k * 32;
-                float y[32];
+                if (PERM) TC_TIE4(u);
+                const int tc = t0 + half * 128 + k * 32 + (PERM ? sq - (half ? 4 : 0) : 0);  // the block's first time
+                float y[PERM ? 40 : 32];  // PERM: u at 0 (second half) or 36 (first), v at 4
 #pragma unroll
-                for (int j = 0; j < 32; ++j) y[j] = fmaf(__uint_as_float(v[j]), scale, off);
-                if (k < 3) TC_LD32(tbase + (uint32_t)((k + 1) * 32), v);
-                if constexpr (TMA_STORE) {
-                    // the staging block is rewritten: wait until the previous
-                    // block's store has read it
-                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    __syncwarp();
-                    // 128-byte swizzle: 16-byte chunk j4 of row `lane` goes to chunk j4 ^ (lane & 7)
-                    uint8_t* row8 = reinterpret_cast<uint8_t*>(st) + lane * 128;
+                for (int j = 0; j < 32; ++j) y[(PERM ? 4 : 0) + j] = fmaf(__uint_as_float(v[j]), scale, off);
+                if (PERM) {
 #pragma unroll
-                    for (int j4 = 0; j4 < 8; ++j4)
-                        *reinterpret_cast<float4*>(row8 + ((j4 ^ (lane & 7)) << 4)) =
-                            make_float4(y[4 * j4], y[4 * j4 + 1], y[4 * j4 + 2], y[4 * j4 + 3]);
-                    if (!plain)
-                        mask_staged(reinterpret_cast<float*>(row8), true, lane, t0 + cb, warm, p, has_nan, a.n,
-                                    a.nan_mode, first_nan, a.nan_bits);
-                    // the TMA engine writes the 32 x 32 block (clipping rows / times past the ends)
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) {
-                        asm volatile(
-                            "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
-                                reinterpret_cast<uint64_t>(&tmap_out)),
-                            "r"(t0 + cb), "r"(rbase), "r"(smem_u32(st))
-                            : "memory");
-                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    }
-                    __syncwarp();
-                } else {
-#pragma unroll
-                    for (int j4 = 0; j4 < 8; ++j4)
-                        *reinterpret_cast<float4*>(st + lane * kStageLd + 4 * j4) =
-                            make_float4(y[4 * j4], y[4 * j4 + 1], y[4 * j4 + 2], y[4 * j4 + 3]);
-                    if (!plain)
-                        mask_staged(st + lane * kStageLd, false, lane, t0 + cb, warm, p, has_nan, a.n, a.nan_mode,
-                                    first_nan, a.nan_bits);
-                    __syncwarp();
-                    // 8 lanes per row: each store instruction writes 4 rows x 128 B
-                    const int c4 = lane & 7;
-                    const int tcol = t0 + cb + 4 * c4;
-#pragma unroll
-                    for (int kk = 0; kk < 8; ++kk) {
-                        const int rr = 4 * kk + (lane >> 3);
-                        const int cr = rbase + rr;
-                        if (cr < a.n_combos) {
-                            const float4 yv = *reinterpret_cast<const float4*>(st + rr * kStageLd + 4 * c4);
-                            float* o = a.out + (size_t)cr * a.n + tcol;
-                            if (vec_ok && tcol + 4 <= a.n) {
-                                *reinterpret_cast<float4*>(o) = yv;
-                            } else {
-                                if (tcol < a.n) o[0] = yv.x;
-                                if (tcol + 1 < a.n) o[1] = yv.y;
-                                if (tcol + 2 < a.n) o[2] = yv.z;
-                                if (tcol + 3 < a.n) o[3] = yv.w;
-                            }
-                        }
-                    }
-                    __syncwarp();
+                    for (int j = 0; j < 4; ++j) y[j] = y[36 + j] = fmaf(__uint_as_float(u[j]), scale, off);
                 }
+                if (k < 3) {
+                    TC_LD32(tbase + (uint32_t)((k + 1) * 32), v);
+                    if (PERM) TC_LD4(tfour + (uint32_t)((k + 1) * 32), u);
+                }
+                // the staging block is rewritten: wait until the previous
+                // block's store has read it
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                __syncwarp();
+                if constexpr (PERM) {
+                    if (g == 0 && half == 0 && k == 0 && sq > 0) {  // the outputs before the first window
+                        put(y + 4, std::integral_constant<int, 0>{});
+                        if (!plain)
+                            mask_staged(reinterpret_cast<float*>(row8), lane, 0, warm, p, has_nan, a.n, a.nan_mode,
+                                        first_nan, a.nan_bits);
+                        const float* head = reinterpret_cast<const float*>(row8 + ((lane & 7) << 4));
+                        for (int t = 0; t < min(sq, a.n); ++t)
+                            if (c < a.n_combos) a.out[(size_t)c * a.n + t] = head[t];
+                    }
+                    if (half)
+                        put_at(y);
+                    else
+                        put_at(y + 4);
+                } else {
+                    put(y, std::integral_constant<int, 0>{});
+                }
+                if (!plain)
+                    mask_staged(reinterpret_cast<float*>(row8), lane, tc, warm, p, has_nan, a.n, a.nan_mode, first_nan,
+                                a.nan_bits);
+                if (PERM && (unsigned)(a.n - tail - tc) < 32u && c < a.n_combos) {
+                    const float* end = reinterpret_cast<const float*>(row8 + ((((a.n - tail - tc) >> 2) ^ (lane & 7)) << 4));
+                    for (int i = 0; i < tail; ++i) a.out[(size_t)c * a.n + a.n - tail + i] = end[i];
+                }
+                // the TMA engine writes the 32 x 32 block (clipping rows / times past the ends)
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0 && (!PERM || (rbase < rows_q && tc + mq < a.n + mq - tail))) {
+                    asm volatile(
+                        "cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                            reinterpret_cast<uint64_t>(&maps.m[PERM ? q4 : 0])),
+                        "r"(tc + mq), "r"(rbase), "r"(smem_u32(row8))
+                        : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+                __syncwarp();
             }
             tc_fence_before();
             mbar_arrive(&ctl->acc_empty[b]);
             if (tr) a.trace[i * TR_N + TR_E_END] = now_ns();
         }
-        if (TMA_STORE && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
 
     // drain: the last committed MMAs must have completed before TMEM is freed
@@ -746,7 +781,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
 // tiles run in kSliceK slices).
 size_t smem_bytes_for(int K) {
     const int J = K / 8 + kN / 8 - 1;
-    return (size_t)kM * K * 2 * 2 + 2 * kStripBufs * (size_t)J * 128 + 1024 + (size_t)8 * 32 * kStageLd * sizeof(float) +
+    return (size_t)kM * K * 2 * 2 + 2 * kStripBufs * (size_t)J * 128 + 1024 + (size_t)8 * kStageTma +
            sizeof(SmemCtl) + 128;
 }
 
@@ -772,7 +807,34 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     const int ka = std::min(kbig, kMaxK);
     const size_t smem = std::max<size_t>(smem_bytes_for(ka), 160 * 1024);
     if (smem > ctx->smem_optin) return fail(VTA_ERR_NOT_IMPLEMENTED, "tcgen05 path: shared memory");
-    const int n_time_tiles = (a.n + kN - 1) / kN;
+    // rows at 16-byte boundaries: one tensor map; any others: four
+    const bool perm = a.n % 4 != 0 || (reinterpret_cast<uintptr_t>(a.out) & 15) != 0;
+    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+    if (!encode) {
+        cudaDriverEntryPointQueryResult q;
+        void* fn = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) ==
+                cudaSuccess && q == cudaDriverEntryPointSuccess)
+            encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+        cudaGetLastError();
+    }
+    OutMaps maps;
+    std::memset(&maps, 0, sizeof maps);
+    bool mapped = encode != nullptr;
+    for (int q = 0; q < (perm ? 4 : 1) && mapped; ++q) {
+        const uintptr_t row = reinterpret_cast<uintptr_t>(a.out) + (size_t)q * a.n * sizeof(float);
+        const int mq = (int)(row >> 2) & 3, by = perm ? 4 : 1;
+        const cuuint64_t dims[2] = {(cuuint64_t)(perm ? std::max(4, (a.n + mq) & ~3) : a.n), (cuuint64_t)std::max(1, (a.n_combos - q + by - 1) / by)};
+        const cuuint64_t strides[1] = {(cuuint64_t)a.n * by * sizeof(float)};
+        const cuuint32_t box[2] = {32, 32};
+        const cuuint32_t estr[2] = {1, 1};
+        mapped = encode(&maps.m[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, reinterpret_cast<void*>(row - 4 * mq), dims,
+                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    }
+    if (!mapped) return fail(VTA_ERR_NOT_IMPLEMENTED, "tcgen05 path: tensor map of the outputs");
+    const int step = perm ? kNPerm : kN;
+    const int n_time_tiles = (a.n + step - 1) / step;
     const int jmax = kbig / 8 + kN / 8 - 1;
     const size_t strip_tile = (size_t)jmax * 128;
     // preparation: shared memory of a strip (its linear values, split) or of a
@@ -817,8 +879,8 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     VTA_TRY(const_upload(ctx, toff.data(), toff.size(), const_cast<long long*>(d_toff), &d_toff));
     const int rows = n_tiles_m * kM;
     RowArgs ra{a.kind, a.periods, a.pa, a.pb, a.n_combos, d_tk, d_toff, d_packed, d_rs, d_rsum,
-               (int)ceil_div(rows, kPrepRows), kbig};
-    StripArgs sa{a.x, a.n, a.first, kbig, jmax, d_sh, d_sl, d_ref, d_xs, d_tnan, d_nbits};
+               (int)ceil_div(rows, kPrepRows), kbig, perm ? 1 : 0};
+    StripArgs sa{a.x, a.n, a.first, kbig, jmax, step, d_sh, d_sl, d_ref, d_xs, d_tnan, d_nbits};
     auto prep = variant == 1 ? k_wwma_prep<1> : k_wwma_prep<0>;
     if (psmem > 48 * 1024)
         VTA_CUDA_TRY(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem));
@@ -872,36 +934,15 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     // every chunk must hold at least one item (the CTAs' item walk assumes it)
     k = std::min<long long>(k, std::max<long long>(1, items / G));
     t.n_time_tiles = n_time_tiles;
+    t.step = step;
     t.items = (int)items;
     t.nchunks = G * k;
     dim3 grid((unsigned)G);
-    // TMA store path when rows are 16-byte aligned (len % 4 == 0); st.global otherwise
-    CUtensorMap tmap;
-    std::memset(&tmap, 0, sizeof tmap);
-    bool use_tma = (a.n % 4) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
-    if (use_tma) {
-        static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-        if (!encode) {
-            cudaDriverEntryPointQueryResult q;
-            void* fn = nullptr;
-            if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) ==
-                    cudaSuccess && q == cudaDriverEntryPointSuccess)
-                encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-            cudaGetLastError();
-        }
-        const cuuint64_t dims[2] = {(cuuint64_t)a.n, (cuuint64_t)a.n_combos};
-        const cuuint64_t strides[1] = {(cuuint64_t)a.n * sizeof(float)};
-        const cuuint32_t box[2] = {32, 32};
-        const cuuint32_t estr[2] = {1, 1};
-        use_tma = encode && encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, a.out, dims, strides, box, estr,
-                                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    }
-    auto kern = variant == 1 ? (use_tma ? k_wwma_tc<1, true> : k_wwma_tc<1, false>)
-                             : (use_tma ? k_wwma_tc<0, true> : k_wwma_tc<0, false>);
+    auto kern = variant == 1 ? (perm ? k_wwma_tc<1, true> : k_wwma_tc<1, false>)
+                             : (perm ? k_wwma_tc<0, true> : k_wwma_tc<0, false>);
     VTA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ktimer_begin(st);
-    kern<<<grid, kThreads, smem, st>>>(t, tmap);
+    kern<<<grid, kThreads, smem, st>>>(t, maps);
     ktimer_end(st);
     VTA_TRY(check_launch("k_wwma_tc"));
     // the error word is read where the host next waits for this work (tc_error,

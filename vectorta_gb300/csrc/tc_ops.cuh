@@ -88,6 +88,13 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
           "=r"(r[29]), "=r"(r[30]), "=r"(r[31])                                                              \
         : "r"(taddr))
 
+#define TC_LD4(taddr, r)                                                                                 \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"                            \
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])                                        \
+                 : "r"(taddr))
+// (after the wait of another load of this thread: ties the four registers to it)
+#define TC_TIE4(r) asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])::"memory")
+
 // Waits for this thread's tcgen05.ld to complete; the 32 destination registers
 // are operands, so no use of them can be scheduled before the wait.
 #define TC_WAIT_LD32(r)                                                                                   \
