@@ -115,3 +115,20 @@ def test_outputs_at_any_float(name, n, offset):
     else:
         assert np.array_equal(got, want, equal_nan=True)
     assert bool((buf[:16 + offset] == 7.0).all()) and bool((buf[16 + offset + rows * n:] == 7.0).all())
+
+
+@pytest.mark.parametrize("extra", [0, 1, 2, 5, 6])
+def test_adx_scan_rows(extra):
+    # same chunks, same carries: only the stores differ
+    n = 280_001 + extra
+    pad = (n + 7) // 8 * 8
+    d = datagen.ohlcv(pad, seed=74, nan_lead=33)
+    cols = tuple(np.asarray(d[k], np.float32) for k in ("high", "low", "close"))
+    res = []
+    for m in (pad, n):
+        ind = V.CLASSES["adx"](0)
+        ind.set_policy("scan_chunk", "1056")
+        res.append(ind.batch_dev(*(np.ascontiguousarray(c[:m]) for c in cols),
+                                 sweep={"period": (160, 409, 1)}).to_host())
+        assert "exact scan" in ind.last_kernel
+    assert np.array_equal(res[1], res[0][:, :n], equal_nan=True)

@@ -78,6 +78,59 @@ struct Lane {
 enum { PASS_AGG1 = 0, PASS_AGG2 = 1, PASS_EMIT = 2 };
 
 
+// A warp's staging: a row per lane, CUT behind 8 columns of the tile before; odd
+// row stride, so a row's and a column's accesses both fall in 32 banks.
+template <bool CUT> struct ScanSmem {
+    static constexpr int kLead = CUT ? 8 : 0;
+    float stage[32][kLead + 33];
+    float4 xin[3][8];  // a tile's TR, +DM and -DM
+};
+template <bool CUT> union WarpSmem {
+    ScanSmem<CUT> scan;
+    hlc::ItemSmem<hlc::PAdx> item;
+};
+
+// Stores a staged tile of nt steps: row r at o + r n.  CUT (large outputs whose
+// rows do not start at 32-byte sectors): each row from its sector boundary on,
+// the last m values of the tile before waiting in the kLead columns; `first`
+// and `last` tile of a chunk.
+template <bool CUT>
+__device__ __forceinline__ void store_tile(float* o, int n, int rows, ScanSmem<CUT>& sm, int nt, bool first,
+                                           bool last) {
+    constexpr int kLead = ScanSmem<CUT>::kLead;
+    auto& stage = sm.stage;
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    if constexpr (CUT) {
+        const int m0 = (int)(reinterpret_cast<uintptr_t>(o) >> 2);
+        o += lane;
+        if (!first && !last && rows == 32) {
+#pragma unroll
+            for (int r = 0; r < 32; ++r, o += n) {
+                const int m = (m0 + r * n) & 7;
+                o[-m] = stage[r][kLead + lane - m];
+            }
+        } else {
+#pragma unroll 4
+            for (int r = 0; r < rows; ++r, o += n) {
+                const int m = (m0 + r * n) & 7, e = lane - m;
+                if ((!first || e >= 0) && e < nt) o[-m] = stage[r][kLead + e];
+                if (last && e + 32 < nt) o[32 - m] = stage[r][kLead + 32 + e];
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 1; i < kLead; ++i) stage[lane][i] = stage[lane][32 + i];
+    } else if (nt == 32 && rows == 32) {
+        o += lane;
+#pragma unroll
+        for (int r = 0; r < 32; ++r) o[(size_t)r * n] = stage[r][kLead + lane];
+    } else if (lane < nt) {
+        for (int r = 0; r < rows; ++r) o[(size_t)r * n + lane] = stage[r][kLead + lane];
+    }
+    __syncwarp();
+}
+
 // One (group, chunk >= 1) item per warp; lane = combo of the group.  A step is
 // the three first-level updates plus DX and the second level: the bar's own
 // terms come from shared memory (formed once per bar by the lane that loaded
@@ -85,15 +138,15 @@ enum { PASS_AGG1 = 0, PASS_AGG2 = 1, PASS_EMIT = 2 };
 // by 32 unrolled 128-byte stores.  320 periods on 1M bars: AGG1 221 -> 74 us,
 // AGG2 281 -> 147 (both bound by issue), EMIT 472 -> 243 (1.28 GB written, 5.3
 // TB/s).
-template <int PASS>
+template <int PASS, bool CUT = false>
 __global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a, HlcChunkArgs c) {
-    __shared__ hlc::ItemSmem<hlc::PAdx> smem[kSW];
+    __shared__ WarpSmem<CUT> smem[kSW];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    auto& sm = smem[warp];
+    ScanSmem<CUT>& sm = smem[warp].scan;
     int item = blockIdx.x * kSW + warp;
     if (PASS != PASS_AGG2) {  // the pass's warm-restart items first
         if (item < c.n_items) {
-            hlc::run_item<hlc::PAdx>(c, item, sm);
+            hlc::run_item<hlc::PAdx>(c, item, smem[warp].item);
             return;
         }
         item -= c.n_items;
@@ -166,7 +219,7 @@ __global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a, HlcChunkAr
                 const float dx = WIDE ? hlc::adx_dx_wide(pdm, mdm) : hlc::adx_dx(pdm, mdm, atr);
                 adx = (adx * ln.pm1 + dx) * ln.rp;
             }
-            if (PASS == PASS_EMIT) sm.stage0[lane][j] = adx;
+            if (PASS == PASS_EMIT) sm.stage[lane][ScanSmem<CUT>::kLead + j] = adx;
         };
         auto steps = [&](auto wide_tag) {
             if (nt == 32) {
@@ -189,17 +242,8 @@ __global__ void __launch_bounds__(kSW * 32) k_adx_scan(AdxScanArgs a, HlcChunkAr
         ph = __shfl_sync(0xffffffffu, xh, nt - 1);
         pl = __shfl_sync(0xffffffffu, xl, nt - 1);
         pc = __shfl_sync(0xffffffffu, xc, nt - 1);
-        if (PASS == PASS_EMIT) {
-            __syncwarp();
-            float* o = a.out + (size_t)(g * 32) * a.n + tb + lane;
-            if (nt == 32 && rows == 32) {
-#pragma unroll
-                for (int r = 0; r < 32; ++r) o[(size_t)r * a.n] = sm.stage0[r][lane];
-            } else if (lane < nt) {
-                for (int r = 0; r < rows; ++r) o[(size_t)r * a.n] = sm.stage0[r][lane];
-            }
-            __syncwarp();
-        }
+        if (PASS == PASS_EMIT)
+            store_tile<CUT>(a.out + (size_t)(g * 32) * a.n + tb, a.n, rows, sm, nt, tb == c0, tb + nt == c1);
     }
     if (PASS == PASS_AGG1) a.agg1[si] = make_float4(atr, pdm, mdm, 0.f);
     if (PASS == PASS_AGG2) a.agg2[si] = adx;
@@ -316,7 +360,8 @@ vta_status launch_adx_scan(const AdxScanArgs& a, const HlcChunkArgs& c, int n_se
     VTA_TRY(check_launch("k_adx_scan<agg2>"));
     k_adx_carry<2><<<cblocks, 128, 0, st>>>(a);
     VTA_TRY(check_launch("k_adx_carry<2>"));
-    k_adx_scan<PASS_EMIT><<<blocks(rest.n_items), kSW * 32, 0, st>>>(a, rest);
+    const auto emit = a.cut ? k_adx_scan<PASS_EMIT, true> : k_adx_scan<PASS_EMIT, false>;
+    emit<<<blocks(rest.n_items), kSW * 32, 0, st>>>(a, rest);
     VTA_TRY(check_launch("k_adx_scan<emit>"));
     VTA_TRY(launch_hlc_fixup(c, st));
     ktimer_end(st);

@@ -1230,6 +1230,11 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
                 x.agg2 = ar.take<float>((size_t)scan_nch * scan_slots);
                 x.carry2 = ar.take<float>((size_t)scan_nch * scan_slots);
                 x.out = out[0];
+                // us of a call, rows as they fall / cut: 399 periods on 500,001
+                // bars 539 / 444, on 500,004 461 / 443 (500,000: 417), 301 on
+                // 100,001 167 / 179; the warm-restart groups' chains only lose
+                // (99 periods on 200,001 159 / 184)
+                x.cut = n % 8 != 0 && (size_t)nc * n * sizeof(float) >= 4 * kCutBytes;
                 VTA_TRY(launch_adx_scan(x, c, n_seed, st));
                 ctx->last_kernel = "adx_chunked(" + std::to_string(adx_groups.size()) + " of " + std::to_string(G) +
                                    " groups on the exact scan, L=" + std::to_string(adx_L) + ")";

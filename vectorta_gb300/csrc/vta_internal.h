@@ -381,6 +381,11 @@ struct HlcArgs {
     float* out1;           // changed
 };
 vta_status launch_adx(const HlcArgs& a, cudaStream_t st);
+// Outputs from which batch rows that do not start at 32-byte sectors are stored
+// cut at the sectors: beyond this the L2 no longer merges all partial sectors
+// before it writes them back (at about half rate)
+constexpr size_t kCutBytes = (size_t)64 << 20;
+
 // Batch ADX (kind 0) / SuperTrend (kind 1) cut into time chunks with verified
 // warm restarts (k_hlc_chunk.cu); bit-identical to the sequential kernels.
 struct HlcChunkArgs {
@@ -432,6 +437,7 @@ struct AdxScanArgs {
     float4* carry1;
     float* carry2;
     float* out;             // [n_combos][n]
+    bool cut;               // the scan's rows stored cut at sectors (see kCutBytes)
 };
 // c: the sweep's warm-restart items, the n_seed seeding items of the scan's
 // groups first; runs them all
@@ -440,11 +446,6 @@ vta_status launch_supertrend(const HlcArgs& a, cudaStream_t st);
 
 // ------------------------------------------------- prefix-sum windows ------
 enum WinKind { WK_SMA = 0, WK_STDDEV = 1, WK_ZSCORE = 2, WK_BB = 3 };
-// Outputs from which batch rows that do not start at 32-byte sectors are stored
-// cut at the sectors: beyond this the L2 no longer merges all partial sectors
-// before it writes them back (at about half rate)
-constexpr size_t kCutBytes = (size_t)64 << 20;
-
 struct PrefixWinArgs {
     int kind;
     const float* x;
