@@ -1134,7 +1134,9 @@ __device__ __forceinline__ float4* agg_slot(const RecurArgs& a, int chunk, int l
 // pattern reaches ~6.9 TB/s where 128-byte row segments reach ~6.2 TB/s.
 // Staging rows are 66 floats (8-byte aligned float2 reads); rows 16..31 swap
 // the two floats of each pair (column c is stored at c ^ 1), so the per-step
-// scalar writes of the 32 lanes fall in 32 distinct banks.
+// scalar writes of the 32 lanes fall in 32 distinct banks.  The stores are
+// marked evict-first (nothing of the call reads them back): 999 EMAs on 1M bars
+// 648 -> 635 us, 399 on 500k 185 -> 177.
 //
 // Rows that do not all start at a 32-byte sector (n % 8 != 0) are CUT at the
 // sectors instead: row r writes [seg0 - m, seg0 + 64 - m), m = its segment's
@@ -1452,7 +1454,7 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
                         v[k] = make_float2(sr[(i + k) * W + x - m[k]], sr[(i + k) * W + 1 - x - m[k]]);
                     }
 #pragma unroll
-                    for (int k = 0; k < 8; ++k, op += a.n) *reinterpret_cast<float2*>(op - m[k]) = v[k];
+                    for (int k = 0; k < 8; ++k, op += a.n) __stcs(reinterpret_cast<float2*>(op - m[k]), v[k]);
                 }
             } else {  // a chunk's first segment has no carry, its last leaves none
 #pragma unroll 4
@@ -1477,11 +1479,11 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
             float* op = ob + 2 * lane;
 #pragma unroll 4
             for (int r = 0; r < r16; ++r, op += a.n)
-                *reinterpret_cast<float2*>(op) = *reinterpret_cast<const float2*>(stage + r * W + 2 * lane);
+                __stcs(reinterpret_cast<float2*>(op), *reinterpret_cast<const float2*>(stage + r * W + 2 * lane));
 #pragma unroll 4
             for (int r = 16; r < rows; ++r, op += a.n) {
                 const float2 v = *reinterpret_cast<const float2*>(stage + r * W + 2 * lane);
-                *reinterpret_cast<float2*>(op) = make_float2(v.y, v.x);
+                __stcs(reinterpret_cast<float2*>(op), make_float2(v.y, v.x));
             }
         } else {
             for (int h = lane; h < len; h += 32) {

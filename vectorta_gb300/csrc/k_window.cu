@@ -187,7 +187,9 @@ __device__ __forceinline__ float rsqrt_approx(float v) {
     return r;
 }
 
-// One combo's outputs at this thread's kPwPer times of a clean tile.
+// One combo's outputs at this thread's kPwPer times of a clean tile, stored
+// evict-first (250 Bollinger rows on 200k bars 102 -> 99 us, 399 SMAs on 500k
+// 133 -> 125).
 // q1[k], q2[k]: split prefix at t; b1, b2: split prefix array shifted to t - p.
 template <int K, bool FULL>
 __device__ __forceinline__ void fast_outputs(const float2 (&q1)[4], const float2 (&q2)[4], const float (&xt)[4],
@@ -202,31 +204,31 @@ __device__ __forceinline__ void fast_outputs(const float2 (&q1)[4], const float2
         const int tk = t + k * kPwThreads;
         if (!FULL && (tk >= n || tk < warm)) {
             if (tk >= 0 && tk < n) {
-                r0[k * kPwThreads] = qnan();
-                if (K == WK_BB) { r1[k * kPwThreads] = qnan(); r2[k * kPwThreads] = qnan(); }
+                __stcs(r0 + k * kPwThreads, qnan());
+                if (K == WK_BB) { __stcs(r1 + k * kPwThreads, qnan()); __stcs(r2 + k * kPwThreads, qnan()); }
             }
             continue;
         }
         const float2 v1 = b1[k * kPwThreads];
         const float d1h = __fsub_rn(q1[k].x, v1.x), d1l = __fsub_rn(q1[k].y, v1.y);
         if (K == WK_SMA) {
-            r0[k * kPwThreads] = __fadd_rn(ref, __fmul_rn(__fadd_rn(d1h, d1l), inv_p));
+            __stcs(r0 + k * kPwThreads, __fadd_rn(ref, __fmul_rn(__fadd_rn(d1h, d1l), inv_p)));
             continue;
         }
         const float2 v2 = b2[k * kPwThreads];
         const float D = window_d(d1h, d1l, __fsub_rn(q2[k].x, v2.x), __fsub_rn(q2[k].y, v2.y), pf);
         const float r = rsqrt_approx(fmaxf(D, 1.17549435e-38f));
         if (K == WK_STDDEV) {
-            r0[k * kPwThreads] = D > 0.f ? __fmul_rn(__fmul_rn(D, r), cc.z) : 0.f;
+            __stcs(r0 + k * kPwThreads, D > 0.f ? __fmul_rn(__fmul_rn(D, r), cc.z) : 0.f);
         } else if (K == WK_ZSCORE) {
             const float dev = __fsub_rn(xt[k], __fmul_rn(__fadd_rn(d1h, d1l), inv_p));
-            r0[k * kPwThreads] = D > 0.f ? __fmul_rn(__fmul_rn(dev, r), cc.z) : qnan();
+            __stcs(r0 + k * kPwThreads, D > 0.f ? __fmul_rn(__fmul_rn(dev, r), cc.z) : qnan());
         } else {
             const float mean = __fadd_rn(ref, __fmul_rn(__fadd_rn(d1h, d1l), inv_p));
             const float sd = __fmul_rn(__fmul_rn(fmaxf(D, 0.f), r), inv_p);
-            r1[k * kPwThreads] = mean;
-            r0[k * kPwThreads] = fmaf(cc.z, sd, mean);
-            r2[k * kPwThreads] = fmaf(-cc.w, sd, mean);
+            __stcs(r1 + k * kPwThreads, mean);
+            __stcs(r0 + k * kPwThreads, fmaf(cc.z, sd, mean));
+            __stcs(r2 + k * kPwThreads, fmaf(-cc.w, sd, mean));
         }
     }
 }
@@ -606,13 +608,13 @@ __device__ __forceinline__ void minmax_clean(const MinMaxArgs& a, const float* m
             const float hmax = fmaxf(mz[k * THREADS], mw[k * THREADS]);
             const float lmin = fminf(nz[k * THREADS], nw[k * THREADS]);
             if (KIND == MM_DONCHIAN) {
-                r0[k * THREADS] = valid ? hmax : qnan();
-                r1[k * THREADS] = valid ? fmaf(hmax - lmin, 0.5f, lmin) : qnan();
-                r2[k * THREADS] = valid ? lmin : qnan();
+                __stcs(r0 + k * THREADS, valid ? hmax : qnan());
+                __stcs(r1 + k * THREADS, valid ? fmaf(hmax - lmin, 0.5f, lmin) : qnan());
+                __stcs(r2 + k * THREADS, valid ? lmin : qnan());
             } else {
                 const float den = hmax - lmin;
                 const float v = den == 0.f ? 0.f : fmaf(-100.f, __fdividef(hmax - cl[k], den), 0.f);
-                r0[k * THREADS] = valid ? v : qnan();
+                __stcs(r0 + k * THREADS, valid ? v : qnan());
             }
         };
         if (full && t0 >= ct.y) {  // the whole tile is valid for this combo (uniform branch)
@@ -630,7 +632,7 @@ __device__ __forceinline__ void minmax_clean(const MinMaxArgs& a, const float* m
                 for (int k = 0; k < PER; ++k) {
                     const float hmax = fmaxf(mz[k * THREADS], mw[k * THREADS]);
                     const float lmin = fminf(nz[k * THREADS], nw[k * THREADS]);
-                    r0[k * THREADS] = willr_wide(hmax, lmin, cl[k]);
+                    __stcs(r0 + k * THREADS, willr_wide(hmax, lmin, cl[k]));
                 }
             } else {
 #pragma unroll
@@ -882,13 +884,13 @@ __global__ void __launch_bounds__(THREADS) k_minmax_ap(MinMaxArgs a, int tile, i
         // value of slot k (finite prices: the fast divide is within 2 ulp)
         auto emit = [&](int k, bool valid) {
             if (KIND == MM_DONCHIAN) {
-                r0[k * THREADS] = valid ? hm[k] : qnan();
-                r1[k * THREADS] = valid ? fmaf(hm[k] - lm[k], 0.5f, lm[k]) : qnan();
-                r2[k * THREADS] = valid ? lm[k] : qnan();
+                __stcs(r0 + k * THREADS, valid ? hm[k] : qnan());
+                __stcs(r1 + k * THREADS, valid ? fmaf(hm[k] - lm[k], 0.5f, lm[k]) : qnan());
+                __stcs(r2 + k * THREADS, valid ? lm[k] : qnan());
             } else {
                 const float den = hm[k] - lm[k];
                 const float v = den == 0.f ? 0.f : fmaf(-100.f, __fdividef(hm[k] - cl[k], den), 0.f);
-                r0[k * THREADS] = valid ? v : qnan();
+                __stcs(r0 + k * THREADS, valid ? v : qnan());
             }
         };
         if (full && t0 >= warm) {  // the whole tile is valid for this combo (uniform branch)
@@ -901,7 +903,7 @@ __global__ void __launch_bounds__(THREADS) k_minmax_ap(MinMaxArgs a, int tile, i
             }
             if (fast) {
 #pragma unroll
-                for (int k = 0; k < PER; ++k) r0[k * THREADS] = willr_wide(hm[k], lm[k], cl[k]);
+                for (int k = 0; k < PER; ++k) __stcs(r0 + k * THREADS, willr_wide(hm[k], lm[k], cl[k]));
             } else {
 #pragma unroll
                 for (int k = 0; k < PER; ++k) emit(k, true);
