@@ -30,6 +30,7 @@
 #include <algorithm>
 
 #include "hlc_item.cuh"
+#include "period_coefs.cuh"
 #include "vta_internal.h"
 
 namespace vta {
@@ -69,8 +70,8 @@ __device__ __forceinline__ D2s ds_pow(D2s b, long long n) {
 struct Lane {
     float omr, pm1, rp;
     __device__ void init(int p) {
-        rp = (float)(1.0 / (double)p);
-        omr = (float)(1.0 - 1.0 / (double)p);
+        rp = coef::wilder(p);
+        omr = coef::wilder_keep(p);
         pm1 = (float)p - 1.f;
     }
 };

@@ -19,6 +19,7 @@
 #include <climits>
 
 #include "vta_internal.h"
+#include "period_coefs.cuh"
 
 namespace vta {
 namespace {
@@ -182,9 +183,8 @@ struct OpEma {
     Acc wsum;
     int wcnt;
     __device__ void init(int p, int first) {
-        double a = 2.0 / ((double)p + 1.0);
-        alpha = (float)a;
-        beta = (float)(1.0 - a);
+        alpha = coef::ema(p);
+        beta = coef::ema_keep(p);
         f = first; s = first + p - 1; warm = first;
         wsum.zero(); wcnt = 0;
     }
@@ -240,9 +240,8 @@ struct OpDema {
     float alpha, a, e1, e2, xf;
     int f, s, warm;
     __device__ void init(int p, int first) {
-        double al = 2.0 / ((double)p + 1.0);
-        alpha = (float)al;
-        a = (float)(1.0 - al);
+        alpha = coef::ema(p);
+        a = coef::ema_keep(p);
         f = first; s = first; warm = first + p - 1;
     }
     template <class In> __device__ void accum(const In& in, int t) { xf = in.X(t); }
@@ -286,9 +285,8 @@ struct OpTema {
     float per, per1, e1, e2, e3;
     int f, s, warm, start2, p1;
     __device__ void init(int p, int first) {
-        double pd = 2.0 / ((double)p + 1.0);
-        per = (float)pd;
-        per1 = (float)(1.0 - pd);
+        per = coef::ema(p);
+        per1 = coef::ema_keep(p);
         p1 = p - 1;
         f = first; start2 = first + p1; s = first + 2 * p1; warm = first + 3 * p1;
         e1 = e2 = e3 = 0.f;
@@ -378,10 +376,9 @@ struct OpRsi {
     Acc sg, sl;
     bool wnan, sc;
     __device__ void init(int p, int first) {
-        double ip = 1.0 / (double)p;
-        inv_p = (float)ip;
+        inv_p = coef::wilder(p);
         pf = (float)p;
-        beta = (float)(1.0 - ip);
+        beta = coef::wilder_keep(p);
         f = first; s = first + p; warm = s;
         sg.zero(); sl.zero(); wnan = false; sc = false;
     }
@@ -451,7 +448,7 @@ struct OpWilders {
     Acc wsum;
     __device__ void init(int p_, int first) {
         p = p_;
-        alpha = (float)(1.0 / (double)p);
+        alpha = coef::wilder(p);
         f = first; s = first + p - 1; warm = s;
         wsum.zero();
     }
@@ -499,7 +496,7 @@ struct OpAtr {
     Acc wsum;
     __device__ void init(int p_, int first) {
         p = p_;
-        alpha = (float)(1.0 / (double)p);
+        alpha = coef::wilder(p);
         f = first; s = first + p - 1; warm = s;
         wsum.zero();
     }
@@ -803,9 +800,9 @@ __device__ bool agg_fast_block(const RecurArgs& a, int chunk, int c0, int c1, fl
     float* s0 = smem;
     float* s1 = smem + kAggTile;
     const int li = blockIdx.x * blockDim.x + threadIdx.x;
-    const double p = li < a.n_lanes ? (double)a.periods[li] : 1.0;
-    const float b = (float)(1.0 - 1.0 / p);       // RSI
-    const float al = (float)(2.0 / (p + 1.0));   // the EMAs
+    const int p = li < a.n_lanes ? a.periods[li] : 1;
+    const float b = coef::wilder_keep(p);  // RSI
+    const float al = coef::ema(p);         // the EMAs
     float z[NZ];
 #pragma unroll
     for (int q = 0; q < NZ; ++q) z[q] = 0.f;
@@ -1006,7 +1003,7 @@ __device__ bool agg_seed_fast(const RecurArgs& a, float* xs, int c1, int cap) {
         acc[0].add(acc[1].hi); acc[0].add(acc[1].lo);
         acc[2].add(acc[3].hi); acc[2].add(acc[3].lo);
         acc[0].add(acc[2].hi); acc[0].add(acc[2].lo);
-        const float al = (float)(2.0 / ((double)p + 1.0));
+        const float al = coef::ema(p);
         CascadeBlock<1> cb;
         cb.init(al);
         float y[1] = {acc[0].f() / (float)p};
@@ -1042,8 +1039,8 @@ __device__ bool agg_seed_fast(const RecurArgs& a, float* xs, int c1, int cap) {
             if (v > xp) sg[0].add_diff(v, xp);
             else if (v < xp) sl[0].add_diff(xp, v);
         }
-        const double inv_p = (double)(float)(1.0 / (double)p);
-        const float beta = (float)(1.0 - 1.0 / (double)p), ip = (float)(1.0 / (double)p);
+        const float beta = coef::wilder_keep(p), ip = coef::wilder(p);
+        const double inv_p = (double)ip;
         float ag = (float)((sg[0].d() + sg[1].d()) * inv_p);
         float al = (float)((sl[0].d() + sl[1].d()) * inv_p);
         for (t = s + 1; t < c1; ++t) {
@@ -1057,7 +1054,7 @@ __device__ bool agg_seed_fast(const RecurArgs& a, float* xs, int c1, int cap) {
         // TEMA: e1 from x[f]; e2 joins at f + p - 1 as a copy of e1, e3 at s
         // as a copy of e2 (the op's accum), then all three run (p == 1:
         // the op copies x into e1)
-        const float per = (float)(2.0 / ((double)p + 1.0));
+        const float per = coef::ema(p);
         if (p == 1) {
             g.x = xs[c1 - 1];
         } else {
