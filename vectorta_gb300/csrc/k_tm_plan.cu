@@ -33,7 +33,6 @@
 namespace vta {
 namespace {
 
-constexpr int kPlanWarps = 4;
 __device__ __forceinline__ float qnan() { return __int_as_float(0x7fc00000); }
 
 struct TmIn {

@@ -49,6 +49,7 @@ vta_status launch_plan_first(const PlanArgs& a, int* first_hlc, int* first_c, cu
 vta_status launch_tm_plan(const PlanArgs& a, int blocks, cudaStream_t st);
 vta_status launch_tm_fixup(const PlanArgs& a, cudaStream_t st);
 // CTAs of the persistent launch that fit on the device at once.
+constexpr int kPlanWarps = 4;  // warps of a CTA
 int tm_plan_blocks(int num_sms);
 
 }  // namespace vta
