@@ -200,6 +200,8 @@ vta_status plan_enqueue(vta_tm_plan* P, int n_jobs, cudaStream_t st, bool with_f
 using TuneKey = std::tuple<int, int, int, int>;
 std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tune;
+// a mixed plan's chunks by its jobs' keys and own chunks (tune_mix)
+std::map<std::pair<std::vector<TuneKey>, std::vector<int>>, std::vector<int>> g_tune_mix;
 bool g_tune_loaded = false;
 
 int log2_bucket(long long v) {
@@ -252,51 +254,70 @@ vta_status time_run(vta_tm_plan* P, int n_jobs, float* ms) {
 }
 
 // Chunks are picked for each job alone, where short ones fill the GPU although
-// their warm-up takes more steps than they emit.  Together the jobs may fill it:
-// a plan of more than an item per scheduler is also timed with the chunks
-// shorter than their warm-up lengthened to it, and keeps the faster (ATR, ADX,
-// SuperTrend and percentile(50) of ragged series, us: 200 x 20,000 rows, chunks
-// 512, 256, 256 / all 512: 189 / 148; 512 x 20,000 295 / 261; 128 x 12,000 135 /
-// 98; 1,000 x 2,500 142 / 175).
-vta_status tune_mix(vta_tm_plan* P, const std::vector<int>& all) {
+// entering a chunk (a recurrence's warm-up, a percentile's first window) takes
+// more steps than it emits.  Together the jobs may fill it: a plan of more than
+// an item per scheduler is also timed with the recurrences' chunks lengthened to
+// half their warm-up, the whole, or twice it, the percentiles' to two windows,
+// and both, and keeps the fastest (ATR, ADX, SuperTrend and percentile(50) of
+// ragged series, us, as picked / kept: 200 x 20,000 rows 190 / 148, 512 x 20,000
+// 295 / 260, 128 x 12,000 135 / 98).  `keys`: the jobs' tuning keys; the choice
+// is kept for the process.
+vta_status tune_mix(vta_tm_plan* P, const std::vector<int>& all, const std::vector<TuneKey>& keys) {
     const int n = (int)all.size(), maxlen = *std::max_element(P->lens.begin(), P->lens.end());
-    std::vector<int> own(n), longer(n);
-    for (int j = 0; j < n; ++j) {
-        const PlanJob& J = P->jobs[j];
-        own[j] = longer[j] = J.chunk;
-        while (plan_job_recurrent(J.kind) && longer[j] < J.warm && longer[j] < maxlen) longer[j] *= 2;
-    }
-    if (longer == own) return VTA_OK;
-    auto use = [&](const std::vector<int>& chunks) {
-        for (int j = 0; j < n; ++j) VTA_TRY(plan_states(P, j, chunks[j]));
+    auto lengthened = [&](const std::vector<int>& own, int quarter_warm, bool windows) {
+        std::vector<int> c = own;
+        for (int j = 0; j < n; ++j) {
+            const PlanJob& J = P->jobs[j];
+            const int to = plan_job_recurrent(J.kind) ? J.warm / 4 * quarter_warm : windows ? 2 * J.period : 0;
+            while (c[j] < to && c[j] < maxlen) c[j] *= 2;
+        }
+        return c;
+    };
+    auto use = [&](const std::vector<int>& c) {
+        for (int j = 0; j < n; ++j) VTA_TRY(plan_states(P, j, c[j]));
         VTA_TRY(plan_items(P, all));
         return plan_upload_jobs(P, all);
     };
-    auto best = [&](float* ms) {  // of three
-        *ms = 1e30f;
+    std::vector<int> own(n);
+    for (int j = 0; j < n; ++j) own[j] = P->jobs[j].chunk;
+    {
+        std::lock_guard<std::mutex> lock(g_tune_mu);
+        const auto it = g_tune_mix.find({keys, own});
+        if (it != g_tune_mix.end()) return use(std::vector<int>(it->second));
+    }
+    std::vector<std::vector<int>> tried;
+    std::vector<int> best;
+    float best_ms = 1e30f;
+    for (int v = 0; v < 8; ++v) {
+        static const int kWarm[] = {0, 2, 4, 8};
+        const std::vector<int> c = lengthened(own, kWarm[v >> 1], v & 1);
+        if (std::find(tried.begin(), tried.end(), c) != tried.end()) continue;
+        tried.push_back(c);
+        VTA_TRY(use(c));
         for (int i = 0; i < 3; ++i) {
-            float one = 0.f;
-            VTA_TRY(time_run(P, n, &one));
-            *ms = std::min(*ms, one);
+            float ms = 0.f;
+            VTA_TRY(time_run(P, n, &ms));
+            if (ms < best_ms) {
+                best_ms = ms;
+                best = c;
+            }
         }
-        return VTA_OK;
-    };
-    float ms_own = 0.f, ms_longer = 0.f;
-    VTA_TRY(plan_upload_jobs(P, all));
-    VTA_TRY(best(&ms_own));
-    VTA_TRY(use(longer));
-    VTA_TRY(best(&ms_longer));
-    return ms_longer < ms_own ? VTA_OK : use(own);
+    }
+    {
+        std::lock_guard<std::mutex> lock(g_tune_mu);
+        g_tune_mix[{keys, own}] = best;
+    }
+    return use(best);
 }
 
 // Times job j alone with each candidate chunk length (second of two runs)
 // and returns the fastest.
 vta_status tune_job(vta_tm_plan* P, int j, int* best) {
-    static const int kRec[] = {256, 512, 1024, 2048, 4096, 8192, 16384};
-    static const int kPnr[] = {128, 256, 512, 1024};
+    static const int kRec[] = {128, 256, 512, 1024, 2048, 4096, 8192, 16384};
+    static const int kPnr[] = {32, 64, 128, 256, 512, 1024};
     const bool rec = plan_job_recurrent(P->jobs[j].kind);
     const int* cand = rec ? kRec : kPnr;
-    const int nc = rec ? 7 : 4;
+    const int nc = rec ? 8 : 6;
     const int maxlen = *std::max_element(P->lens.begin(), P->lens.end());
     float best_ms = 1e30f;
     *best = cand[0];
@@ -400,11 +421,13 @@ vta_status plan_create(vta_ctx* ctx, const float* h, const float* l, const float
     VTA_TRY(launch_plan_first(a0, P->d_first_hlc, P->d_first_c, st));
     // chunk length per job: policy, cache, or timed now
     const int maxlen = *std::max_element(P->lens.begin(), P->lens.end());
+    std::vector<TuneKey> keys;
     for (size_t j = 0; j < n_jobs; ++j) {
         int chunk = ctx->policy.tm_chunk;
         if (chunk < 0) chunk = std::max(maxlen, 1);
         if (chunk == 0) {
             const TuneKey key{P->jobs[j].kind, P->jobs[j].period, log2_bucket(maxlen), log2_bucket((long long)cols)};
+            keys.push_back(key);
             {
                 std::lock_guard<std::mutex> lock(g_tune_mu);
                 tune_load_locked();
@@ -423,7 +446,8 @@ vta_status plan_create(vta_ctx* ctx, const float* h, const float* l, const float
     std::vector<int> all(n_jobs);
     for (size_t j = 0; j < n_jobs; ++j) all[j] = (int)j;
     VTA_TRY(plan_items(P, all));
-    if (n_jobs > 1 && ctx->policy.tm_chunk == 0 && P->n_items > 4 * ctx->num_sms) VTA_TRY(tune_mix(P, all));
+    if (n_jobs > 1 && ctx->policy.tm_chunk == 0 && P->n_items > 4 * ctx->num_sms)
+        VTA_TRY(tune_mix(P, all, keys));
     VTA_TRY(plan_upload_jobs(P, all));
     VTA_CUDA_TRY(cudaStreamSynchronize(st));
 
