@@ -702,7 +702,7 @@ def gpu_bench_plan(args, wl):
         "clocks": clk.summary(),
         "roofline": {"bound": "hbm", "achieved": alg / (g_ms / 1e3) / 1e9, "peak": hbm, "unit": "GB/s",
                      "frac": alg / (g_ms / 1e3) / 1e9 / hbm, "traffic": TRAFFIC.get(wl["name"]),
-                     "kernel": "tm plan graph (k_plan_first + k_tm_plan + k_tm_fixup)", "peak_source": src,
+                     "kernel": "tm plan graph (k_first_valid_tm + k_tm_plan + k_tm_fixup)", "peak_source": src,
                      "bytes_per_launch": alg, "ms_per_launch": g_ms},
         "kernel_ms_per_call": {"plan_graph": g_ms}, "outputs_per_step": out_per_step, "e2e": e2e,
         "plan": {"create_s": create_s, "tuned": info["tuned"], "chunk": info["chunk"][:len(jobs)],
