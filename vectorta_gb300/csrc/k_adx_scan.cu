@@ -108,13 +108,13 @@ __device__ __forceinline__ void store_tile(float* o, int n, int rows, ScanSmem<C
         if (!first && !last && rows == 32) {
 #pragma unroll
             for (int r = 0; r < 32; ++r, o += n) {
-                const int m = (m0 + r * n) & 7;
+                const int m = (int)((unsigned)m0 + (unsigned)r * (unsigned)n) & 7;
                 o[-m] = stage[r][kLead + lane - m];
             }
         } else {
 #pragma unroll 4
             for (int r = 0; r < rows; ++r, o += n) {
-                const int m = (m0 + r * n) & 7, e = lane - m;
+                const int m = (int)((unsigned)m0 + (unsigned)r * (unsigned)n) & 7, e = lane - m;
                 if ((!first || e >= 0) && e < nt) o[-m] = stage[r][kLead + e];
                 if (last && e + 32 < nt) o[32 - m] = stage[r][kLead + 32 + e];
             }

@@ -1482,7 +1482,7 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
                 // m repeats every 8 rows
                 int m[8];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) m[k] = (m0 + k * a.n) & 7;
+                for (int k = 0; k < 8; ++k) m[k] = (int)((unsigned)m0 + (unsigned)k * (unsigned)a.n) & 7;
                 op += lane;
                 sr += lane;
 #pragma unroll
@@ -1499,7 +1499,7 @@ __device__ __forceinline__ float4 recur_span(const RecurArgs& a, int group, int 
             } else {  // a chunk's first segment has no carry, its last leaves none
 #pragma unroll 4
                 for (int r = 0; r < rows; ++r, sr += W, op += a.n) {
-                    const int m = (m0 + r * a.n) & 7, odd = (lane - m) & 1;
+                    const int m = (int)((unsigned)m0 + (unsigned)r * (unsigned)a.n) & 7, odd = (lane - m) & 1;
                     const int x = (r >> 4) & 1 ? 1 - 2 * odd : 0;
                     const int e = lane - m, lo = first ? 0 : -kCarry, hi = last ? len : kSeg - m;
                     if (e >= lo && e < hi) op[-m] = sr[x - m];
