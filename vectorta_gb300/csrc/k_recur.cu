@@ -1717,14 +1717,12 @@ struct TmBatch {
     }
 };
 
+// One warp's 32 series over the rows [c0, c1): AGG returns the lane's record,
+// EMIT starts from the state `cv` where the lane is running and writes the
+// outputs.
 template <class Op, int PASS>
-__global__ void __launch_bounds__(kWarps * 32) k_recur_tm(RecurArgs a) {
-    const int li = blockIdx.x * (kWarps * 32) + threadIdx.x;
+__device__ __forceinline__ float4 tm_span(const RecurArgs& a, int li, int c0, int c1, const float4 cv) {
     const bool valid = li < a.n_lanes;
-    const int chunk = blockIdx.y;
-    int c0, c1;
-    recur_chunk_bounds(a, chunk, c0, c1);
-    if (c0 >= a.n || (li & ~31) >= a.n_lanes) return;  // (whole warps)
     const int p = a.period, first = valid ? a.first_tm[li] : a.n;
     Op op;
     op.init(p > 0 ? p : 1, first);
@@ -1740,7 +1738,6 @@ __global__ void __launch_bounds__(kWarps * 32) k_recur_tm(RecurArgs a) {
             if (PASS == PASS_AGG) {
                 op.zero();
             } else {
-                const float4 cv = reinterpret_cast<const float4*>(a.carry)[(size_t)chunk * a.n_lanes + li];
                 op.set(0, cv.x);
                 if (Op::NS > 1) op.set(1, cv.y);
                 if (Op::NS > 2) op.set(2, cv.z);
@@ -1790,7 +1787,21 @@ __global__ void __launch_bounds__(kWarps * 32) k_recur_tm(RecurArgs a) {
         before = cur.x[kTmRows - 1];
         cur = nxt;
     }
-    if (PASS == PASS_AGG && valid) *agg_slot(a, chunk, li) = agg_record(op, active, seeded_ever, steps, c0, c1);
+    return agg_record(op, active, seeded_ever, steps, c0, c1);
+}
+
+template <class Op, int PASS>
+__global__ void __launch_bounds__(kWarps * 32) k_recur_tm(RecurArgs a) {
+    const int li = blockIdx.x * (kWarps * 32) + threadIdx.x;
+    const int chunk = blockIdx.y;
+    int c0, c1;
+    recur_chunk_bounds(a, chunk, c0, c1);
+    if (c0 >= a.n || (li & ~31) >= a.n_lanes) return;  // (whole warps)
+    float4 cv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (PASS == PASS_EMIT && li < a.n_lanes)
+        cv = reinterpret_cast<const float4*>(a.carry)[(size_t)chunk * a.n_lanes + li];
+    const float4 g = tm_span<Op, PASS>(a, li, c0, c1, cv);
+    if (PASS == PASS_AGG && li < a.n_lanes) *agg_slot(a, chunk, li) = g;
 }
 
 // Carry-in of every chunk: an exclusive scan, over the chunks of one lane, of
@@ -2058,6 +2069,41 @@ constexpr int kOneWarps = 16;
 constexpr int kOneMax = 2048, kOneMaxTemaP = 64;
 constexpr size_t kOneSmem = (size_t)kOneWarps * (32 * kStageW * sizeof(float) + 16 * sizeof(float4) + 32 * sizeof(float4));
 
+// The state entering chunk q of a lane, from the block's records (rec[32 k +
+// lane]: chunk k's) and the transition ml of a full chunk.
+template <class Op>
+__device__ __forceinline__ float4 entry_state(const float4* rec, int q, int lane, int p, int chunk,
+                                              const D2 (&ml)[Op::NS][Op::NS]) {
+    constexpr int N = Op::NS;
+    constexpr int SH = ShapeOf<Op>::v;
+    D2 S[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) S[r] = {0.f, 0.f};
+#pragma unroll 1
+    for (int k = 0; k < q; ++k) {
+        const float4 e = rec[k * 32 + lane];
+        if (e.w == kBeforeSeed) continue;
+        AffD<N> m;
+        chunk_map<Op>(e, p, chunk, ml, m);
+        D2 t[N];
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            D2 v = m.b[r];
+#pragma unroll
+            for (int c = 0; c < N; ++c)
+                if (shape_nz(SH, r, c)) v = d2_fma(m.m[r][c], S[c], v);
+            t[r] = v;
+        }
+#pragma unroll
+        for (int r = 0; r < N; ++r) S[r] = t[r];
+    }
+    float4 cv = make_float4(0.f, 0.f, 0.f, 0.f);
+    cv.x = S[0].hi + S[0].lo;
+    if (N > 1) cv.y = S[N > 1 ? 1 : 0].hi + S[N > 1 ? 1 : 0].lo;
+    if (N > 2) cv.z = S[N > 2 ? 2 : 0].hi + S[N > 2 ? 2 : 0].lo;
+    return cv;
+}
+
 template <class Op>
 __global__ void __launch_bounds__(32 * kOneWarps) k_recur_one(RecurArgs a) {
     extern __shared__ __align__(16) float one_smem[];
@@ -2075,39 +2121,44 @@ __global__ void __launch_bounds__(32 * kOneWarps) k_recur_one(RecurArgs a) {
     if (c1 < a.n) g = recur_span<Op, PASS_AGG, false>(a, group, c0, c1, zero, st, xi);  // (nobody reads the last record)
     rec[threadIdx.x] = g;
     // the transition of a full chunk, while other warps still aggregate
-    constexpr int N = Op::NS;
-    constexpr int SH = ShapeOf<Op>::v;
     const int p = valid ? a.periods[li] : 1;
-    D2 ml[N][N];
+    D2 ml[Op::NS][Op::NS];
     trans_pow<Op>((long long)a.chunk, p, ml);
     __syncthreads();
     if (c0 >= a.n) return;
-    D2 S[N];
-#pragma unroll
-    for (int r = 0; r < N; ++r) S[r] = {0.f, 0.f};
-#pragma unroll 1
-    for (int k = 0; k < q; ++k) {
-        const float4 e = rec[k * 32 + lane];
-        if (e.w == kBeforeSeed) continue;
-        AffD<N> m;
-        chunk_map<Op>(e, p, a.chunk, ml, m);
-        D2 t[N];
-#pragma unroll
-        for (int r = 0; r < N; ++r) {
-            D2 v = m.b[r];
-#pragma unroll
-            for (int c = 0; c < N; ++c)
-                if (shape_nz(SH, r, c)) v = d2_fma(m.m[r][c], S[c], v);
-            t[r] = v;
-        }
-#pragma unroll
-        for (int r = 0; r < N; ++r) S[r] = t[r];
-    }
-    float4 cv = zero;
-    cv.x = S[0].hi + S[0].lo;
-    if (N > 1) cv.y = S[N > 1 ? 1 : 0].hi + S[N > 1 ? 1 : 0].lo;
-    if (N > 2) cv.z = S[N > 2 ? 2 : 0].hi + S[N > 2 ? 2 : 0].lo;
+    const float4 cv = entry_state<Op>(rec, q, lane, p, a.chunk, ml);
     recur_span<Op, PASS_EMIT, false>(a, group, c0, c1, cv, st, xi);
+}
+
+// The same for many series: a block takes 32 series, a warp of it a chunk of
+// their rows.  For short histories, whose call is three launches' latency; longer
+// ones need more warps than 32 per 32 series (the caller's rule has the times).
+constexpr int kTmOneWarps = 32;
+
+template <class Op>
+__global__ void __launch_bounds__(32 * kTmOneWarps) k_recur_tm_one(RecurArgs a) {
+    __shared__ float4 rec[kTmOneWarps * 32];
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;  // q: this warp's chunk
+    const int li = blockIdx.x * 32 + lane;
+    const int c0 = min(q * a.chunk, a.n), c1 = min(c0 + a.chunk, a.n);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 g = make_float4(0.f, 0.f, 0.f, kBeforeSeed);
+    if (c1 < a.n) g = tm_span<Op, PASS_AGG>(a, li, c0, c1, zero);  // (nobody reads the last record)
+    rec[threadIdx.x] = g;
+    D2 ml[Op::NS][Op::NS];
+    trans_pow<Op>((long long)a.chunk, a.period, ml);
+    __syncthreads();
+    if (c0 >= a.n) return;
+    tm_span<Op, PASS_EMIT>(a, li, c0, c1, entry_state<Op>(rec, q, lane, a.period, a.chunk, ml));
+}
+
+template <class Op>
+vta_status run_tm_one(RecurArgs a, cudaStream_t st) {
+    a.chunk = a.chunk0 = (a.n + kTmOneWarps * kTmRows - 1) / (kTmOneWarps * kTmRows) * kTmRows;
+    ktimer_begin(st);
+    k_recur_tm_one<Op><<<ceil_div(a.n_lanes, 32), 32 * kTmOneWarps, 0, st>>>(a);
+    ktimer_end(st);
+    return check_launch("k_recur_tm_one");
 }
 
 template <class Op>
@@ -2123,8 +2174,11 @@ vta_status run_one(RecurArgs a, cudaStream_t st) {
 // AGG and CARRY (more than one chunk), then EMIT
 template <class Op, bool TM>
 vta_status run(const RecurArgs& a, cudaStream_t st) {
-    if constexpr (!TM) {
-        if (a.one_launch) return run_one<Op>(a, st);
+    if (a.one_launch) {
+        if constexpr (TM)
+            return run_tm_one<Op>(a, st);
+        else
+            return run_one<Op>(a, st);
     }
     const int n_chunks = recur_n_chunks(a.n, a.chunk, a.chunk0);
     const int groups = (int)ceil_div(a.n_lanes, 32);
