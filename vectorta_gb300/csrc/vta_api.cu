@@ -635,68 +635,32 @@ vta_status upload_async(vta_ctx* ctx, void* dst, const void* src, size_t bytes, 
     return VTA_OK;
 }
 
-// Constant cache of a context (see vta_ctx::cc_*): a device buffer filled
-// front to back by uploads; an upload whose bytes match an earlier one (hash,
-// then a full compare with the host copy) reuses it.  When the buffer is full
-// it starts over: the uploads are stream-ordered copies on the context's
-// stream, behind every kernel of the earlier calls that reads the buffer
-// (a stream switch waits for the old stream).  Server slots bypass it.
+// Constant cache of a context (const_cache.h): the uploads are stream-ordered
+// copies on the context's stream, behind every kernel of the earlier calls that
+// reads the buffer (a stream switch waits for the old stream).  Server slots
+// bypass it.
 static constexpr size_t kConstCacheBytes = size_t(4) << 20;
 static constexpr size_t kConstCacheMaxItem = size_t(256) << 10;
 
-static uint64_t bytes_hash(const void* src, size_t n) {
-    const unsigned char* b = static_cast<const unsigned char*>(src);
-    uint64_t h = 0x9E3779B97F4A7C15ull ^ n;
-    size_t i = 0;
-    for (; i + 8 <= n; i += 8) {
-        uint64_t w;
-        std::memcpy(&w, b + i, 8);
-        h = (h ^ w) * 0xff51afd7ed558ccdull;
-        h ^= h >> 32;
-    }
-    for (; i < n; ++i) h = (h ^ b[i]) * 0x100000001b3ull;
-    return h;
-}
-
 vta_status const_upload_bytes(vta_ctx* ctx, const void* src, size_t bytes, void* fallback, const void** out) {
-    if (bytes == 0) {
-        *out = fallback;
-        return VTA_OK;
-    }
-    if (ctx->async_alloc || bytes > kConstCacheMaxItem) {
-        VTA_TRY(upload_async(ctx, fallback, src, bytes, ctx->stream));
-        *out = fallback;
-        return VTA_OK;
-    }
-    const uint64_t h = bytes_hash(src, bytes);
-    for (const auto& e : ctx->cc)
-        if (e.hash == h && e.bytes == bytes && std::memcmp(ctx->cc_host.data() + e.off, src, bytes) == 0) {
-            *out = static_cast<const char*>(ctx->cc_dev) + e.off;
-            return VTA_OK;
-        }
+    *out = fallback;
+    if (bytes == 0) return VTA_OK;
+    if (ctx->async_alloc || bytes > kConstCacheMaxItem) return upload_async(ctx, fallback, src, bytes, ctx->stream);
     if (!ctx->cc_dev) {
         if (vram_check(kConstCacheBytes) != VTA_OK || cudaMalloc(&ctx->cc_dev, kConstCacheBytes) != cudaSuccess) {
             cudaGetLastError();
             ctx->cc_dev = nullptr;
-            VTA_TRY(upload_async(ctx, fallback, src, bytes, ctx->stream));
-            *out = fallback;
-            return VTA_OK;
+            return upload_async(ctx, fallback, src, bytes, ctx->stream);
         }
-        ctx->cc_cap = kConstCacheBytes;
-        ctx->cc_host.resize(kConstCacheBytes);
+        ctx->cc.init(kConstCacheBytes);
     }
-    const size_t need = (bytes + 255) & ~size_t(255);
-    if (ctx->cc_used + need > ctx->cc_cap) {
-        ctx->cc_used = 0;
-        ctx->cc.clear();
+    size_t off = 0;
+    if (!ctx->cc.find(src, bytes, &off)) {
+        if (!ctx->cc.place(src, bytes, &off)) return upload_async(ctx, fallback, src, bytes, ctx->stream);
+        VTA_TRY(upload_async(ctx, static_cast<char*>(ctx->cc_dev) + off, src, bytes, ctx->stream));
+        ctx->cc.keep(off, bytes);
     }
-    const size_t off = ctx->cc_used;
-    std::memcpy(ctx->cc_host.data() + off, src, bytes);
-    char* dst = static_cast<char*>(ctx->cc_dev) + off;
-    VTA_TRY(upload_async(ctx, dst, src, bytes, ctx->stream));
-    ctx->cc.push_back({h, off, bytes});
-    ctx->cc_used = off + need;
-    *out = dst;
+    *out = static_cast<const char*>(ctx->cc_dev) + off;
     return VTA_OK;
 }
 
@@ -730,6 +694,7 @@ static vta_status upload(vta_ctx* ctx, void* dst, const void* src, size_t bytes)
 
 static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, size_t first,
                             const std::vector<Combo>& cs, float* const* out) {
+    ctx->cc.begin_call();
     cudaStream_t st = ctx->stream;
     const int n = (int)len;
     const int nc = (int)cs.size();

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/vta_gb300.h"
+#include "const_cache.h"
 
 namespace vta {
 
@@ -115,13 +116,7 @@ struct vta_ctx {
     // constant cache: small per-sweep arrays (period lists, per-combo
     // constants) uploaded once and reused by later calls with the same bytes
     void* cc_dev = nullptr;
-    size_t cc_cap = 0, cc_used = 0;
-    std::vector<unsigned char> cc_host;  // host copy of cc_dev[0, cc_used)
-    struct CcEntry {
-        uint64_t hash;
-        size_t off, bytes;
-    };
-    std::vector<CcEntry> cc;
+    vta::ConstCache cc;
     // packed weights of the tensor-core recurrence aggregates, kept across
     // calls per (kind, chunk length, periods); least recently used evicted
     struct RwEntry {
@@ -170,7 +165,9 @@ vta_status upload_async(vta_ctx* ctx, void* dst, const void* src, size_t bytes, 
 
 // Device copy of `bytes` constant bytes for this call: from the context's
 // constant cache when an earlier call uploaded the same bytes, else uploaded
-// into the cache (or, for server slots and large arrays, into `fallback`).
+// into the cache (or, for server slots, large arrays and a cache that is full
+// in this call, into `fallback`).  Valid for the kernels of the run_batch it is
+// called from.
 vta_status const_upload_bytes(vta_ctx* ctx, const void* src, size_t bytes, void* fallback, const void** out);
 // The device address of [p, p + bytes) when it lies inside one block from
 // vta_pinned_alloc, else null
