@@ -793,6 +793,11 @@ size_t smem_bytes_for(int K) {
 }  // namespace
 
 vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ctx, cudaStream_t st) {
+    // not inside a stream capture: a replay would read operands (the constant
+    // cache, the workspaces) that later calls have since replaced
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    VTA_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return fail(VTA_ERR_CUDA, "tcgen05 path: the stream is being captured");
     const int n_tiles_m = (a.n_combos + kM - 1) / kM;
     const int* per = a.periods_host;
     std::vector<int> tk(n_tiles_m);
