@@ -127,7 +127,8 @@ __device__ __noinline__ void mask_staged(float* row, int lane, int tb, int warm,
 // prefix of the NaN count, packing and strips were six launches: 38 us for 232
 // combos on 20,001 bars, now 7.3; 64 us for the 17,920-combo grid, now 25.)
 constexpr int kPrepThreads = 128;
-constexpr int kPrepRows = kPrepThreads / 32;  // weight rows per block, one warp each
+constexpr int kPrepRows = kPrepThreads / 32;  // weight rows per block at most, one warp each
+constexpr size_t kPrepStatic = 1024;  // prep_strip's own shared memory (32 bytes) up to the 1,024-aligned dynamic part
 
 // Per combo tile m (rows c = 128 m + r): K_m = roundup16(max period), the
 // weights right-aligned in K_m columns, scaled by 2^e_r so the row maximum lies
@@ -145,6 +146,7 @@ struct RowArgs {
     float* row_scale;           // [tiles*128] 2^-e_r
     float* row_sum;             // [tiles*128] sum of the f32 weights
     int blocks, kcap;           // blocks of the launch that form rows; weights the staging holds per row
+    int per_block;              // rows per block
     int perm;                   // rows in the order of the four maps
 };
 
@@ -333,8 +335,9 @@ __global__ void __launch_bounds__(kPrepThreads) k_wwma_prep(RowArgs ra, StripArg
         prep_strip<VARIANT>(sa, blockIdx.x - ra.blocks, sm);
         return;
     }
-    const int warp = threadIdx.x >> 5, row = blockIdx.x * kPrepRows + warp;
-    if (row < rows) prep_row<VARIANT>(ra, row, reinterpret_cast<wts::DS*>(sm) + (size_t)warp * ra.kcap);
+    const int warp = threadIdx.x >> 5, row = blockIdx.x * ra.per_block + warp;
+    if (warp < ra.per_block && row < rows)
+        prep_row<VARIANT>(ra, row, reinterpret_cast<wts::DS*>(sm) + (size_t)warp * ra.kcap);
 }
 
 // ------------------------------------------------------------ main kernel -
@@ -847,12 +850,16 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     const int n_time_tiles = (a.n + step - 1) / step;
     const int jmax = kbig / 8 + kN / 8 - 1;
     const size_t strip_tile = (size_t)jmax * 128;
-    // preparation: shared memory of a strip (its linear values, split) or of a
-    // block's weight rows
+    // preparation: shared memory of a strip (its linear values, split) and of a
+    // block's weight rows, 8 bytes a column each: four rows to a block where they
+    // fit (windows up to 7,232), else one, so that the strip is the limit (28,656)
     const int L = jmax * 8 + 8;
-    const size_t psmem = std::max((size_t)L * 4 + 2 * (size_t)((L + 7) & ~7) * 2 + 64,
-                                  (size_t)kPrepRows * kbig * sizeof(wts::DS));
-    if (psmem > ctx->smem_optin) return fail(VTA_ERR_NOT_IMPLEMENTED, "tcgen05 path: period above the strip limit");
+    const size_t ssmem = (size_t)L * 4 + 2 * (size_t)((L + 7) & ~7) * 2 + 64;
+    const size_t rsmem = (size_t)kbig * sizeof(wts::DS);
+    auto fits = [&](size_t b) { return b + kPrepStatic <= ctx->smem_optin; };
+    const int per_block = fits(kPrepRows * rsmem) ? kPrepRows : 1;
+    const size_t psmem = std::max(ssmem, per_block * rsmem);
+    if (!fits(psmem)) return fail(VTA_ERR_NOT_IMPLEMENTED, "tcgen05 path: period above the strip limit");
     if (!ctx->err_host) {
         VTA_CUDA_TRY(cudaHostAlloc((void**)&ctx->err_host, sizeof(int), cudaHostAllocMapped));
         *ctx->err_host = 0;
@@ -889,7 +896,7 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
     VTA_TRY(const_upload(ctx, toff.data(), toff.size(), const_cast<long long*>(d_toff), &d_toff));
     const int rows = n_tiles_m * kM;
     RowArgs ra{a.kind, a.periods, a.pa, a.pb, a.n_combos, d_tk, d_toff, d_packed, d_rs, d_rsum,
-               (int)ceil_div(rows, kPrepRows), kbig, perm ? 1 : 0};
+               (int)ceil_div(rows, per_block), kbig, per_block, perm ? 1 : 0};
     StripArgs sa{a.x, a.n, a.first, kbig, jmax, step, d_sh, d_sl, d_ref, d_xs, d_tnan, d_nbits};
     auto prep = variant == 1 ? k_wwma_prep<1> : k_wwma_prep<0>;
     if (psmem > 48 * 1024)
