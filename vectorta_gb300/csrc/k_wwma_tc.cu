@@ -94,30 +94,50 @@ __device__ __forceinline__ float qnan() { return __int_as_float(0x7fc00000); }
 // A K-major, B MN-major, N >> 3 at bit 17, M >> 4 at bit 24.
 __host__ __device__ constexpr uint32_t instr_desc(uint32_t ab_type) { return tc::instr_desc_f16(ab_type, kM, kN, 1u); }
 
-// Warm-up / NaN masks of one staged row of 32 consecutive outputs (tiles that
-// need them are few; kept out of line so the hot epilogue loop stays small).
-// A NaN at or after the first valid bar poisons the windows that hold it
-// (nan_mode 0: the bit words of the NaN bars, 32 bars a word, are searched over
-// the window) or every later output (nan_mode 1).  The staging is 128-byte
-// swizzled.
-__device__ __noinline__ void mask_staged(float* row, int lane, int tb, int warm, int p, bool has_nan,
-                                         int n, int nan_mode, int first_nan, const uint32_t* nan_bits) {
-    for (int j = 0; j < 32; ++j) {
-        const int t = tb + j;
-        bool bad = t < warm;
-        if (!bad && has_nan && t < n && t >= first_nan) {
-            bad = nan_mode != 0;
-            const int lo = t - p + 1;  // the window's first bar (>= first valid)
-            for (int w = t >> 5; !bad && w >= max(lo, first_nan) >> 5; --w) {
-                uint32_t m = nan_bits[w];
-                if (w == t >> 5) m &= 0xffffffffu >> (31 - (t & 31));
-                if (w == lo >> 5) m &= 0xffffffffu << (lo & 31);
-                bad = m != 0;
+// Warm-up / NaN masks of one staged block: lane = row, 32 consecutive outputs
+// from time tb on (whole warp; out of line so the hot epilogue loop stays
+// small).  A NaN at or after the first valid bar poisons the windows that hold
+// it (nan_mode 0) or every later output (nan_mode 1).  Which NaN bar is the
+// latest at a time is the same for every row, so each lane finds it for one of
+// the 32 times from the NaN bars' bit words (32 bars a word; a warp looks at
+// 1,024 bars a step, as far back as the warp's longest window reaches), and a
+// row compares its window with the 32 ages.  232 ALMA rows up to 240 bars on
+// 200,000 with a NaN at bar 300 800 -> 67 us, 222 up to 2,000 bars 4,094 -> 390
+// (before, each output walked its window's words; a clean series takes 63 and
+// 392).
+// The staging is 128-byte swizzled.
+__device__ __noinline__ void mask_staged(float* row, int lane, int tb, int warm, int p, int pmax, int n, int nan_mode,
+                                         int first_nan, const uint32_t* nan_bits) {
+    uint32_t bad = tb >= warm ? 0u : warm - tb >= 32 ? ~0u : (1u << (warm - tb)) - 1u;
+    if (first_nan - 31 <= tb) {  // (INT_MAX: no NaN)
+        if (nan_mode != 0) {
+            bad |= first_nan <= tb ? ~0u : ~0u << (first_nan - tb);
+        } else {
+            const int w0 = tb >> 5, t = tb + lane, w = t >> 5;
+            uint32_t m = t < n ? __ldg(nan_bits + w) & (~0u >> (31 - (t & 31))) : 0u;
+            const uint32_t m0 = __ldg(nan_bits + w0);
+            int last = m ? 32 * w + 31 - __clz((int)m) : w > w0 && m0 ? 32 * w0 + 31 - __clz((int)m0) : -1;
+            if (__any_sync(0xffffffffu, last < 0)) {  // the words before the block's first
+                const int stop = max(first_nan >> 5, (tb - pmax + 1) >> 5);
+                int prev = -1;
+                for (int hi = w0 - 1; hi >= stop && prev < 0; hi -= 32) {
+                    const int wi = hi - lane;
+                    m = wi >= stop ? __ldg(nan_bits + wi) : 0u;
+                    const unsigned any = __ballot_sync(0xffffffffu, m != 0u);
+                    if (any) prev = __shfl_sync(0xffffffffu, 32 * wi + 31 - __clz((int)m), __ffs((int)any) - 1);
+                }
+                if (last < 0) last = prev;
+            }
+            const int age = last < 0 ? INT_MAX : t - last;
+            if (__any_sync(0xffffffffu, age < pmax)) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) bad |= (__shfl_sync(0xffffffffu, age, j) < p ? 1u : 0u) << j;
             }
         }
-        if (bad) {
-            row[(((j >> 2) ^ (lane & 7)) << 2) | (j & 3)] = qnan();
-        }
+    }
+    for (; bad; bad &= bad - 1u) {
+        const int j = __ffs((int)bad) - 1;
+        row[(((j >> 2) ^ (lane & 7)) << 2) | (j & 3)] = qnan();
     }
 }
 
@@ -618,7 +638,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
         const int q4 = warp & 3;
         const int half = (warp - 1) >> 2;
         const int r = q4 * 32 + lane;  // accumulator row = combo within tile
-        int cur_mt = -1, c = 0, p = 1, warm = 0, rbase = 0;
+        int cur_mt = -1, c = 0, p = 1, pmax = 1, warm = 0, rbase = 0;
         float rscale = 0.f, rsum = 0.f;
         // the first NaN bar, from the time tiles' (while the first operands load)
         int nan_at = INT_MAX;
@@ -650,6 +670,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
                 cur_mt = mt;
                 c = mt * kM + (PERM ? 4 * lane + q4 : r);
                 p = c < a.n_combos ? a.periods[c] : 1;
+                pmax = __reduce_max_sync(0xffffffffu, p);
                 warm = a.first + p - 1 + (a.warm_extra && c < a.n_combos ? a.warm_extra[c] : 0);
                 rscale = a.row_scale[(size_t)mt * kM + r];
                 rsum = a.row_sum[(size_t)mt * kM + r];
@@ -722,8 +743,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
                     if (g == 0 && half == 0 && k == 0 && sq > 0) {  // the outputs before the first window
                         put(y + 4, std::integral_constant<int, 0>{});
                         if (!plain)
-                            mask_staged(reinterpret_cast<float*>(row8), lane, 0, warm, p, has_nan, a.n, a.nan_mode,
-                                        first_nan, a.nan_bits);
+                            mask_staged(reinterpret_cast<float*>(row8), lane, 0, warm, p, pmax, a.n, a.nan_mode, first_nan,
+                                        a.nan_bits);
                         const float* head = reinterpret_cast<const float*>(row8 + ((lane & 7) << 4));
                         for (int t = 0; t < min(sq, a.n); ++t)
                             if (c < a.n_combos) a.out[(size_t)c * a.n + t] = head[t];
@@ -736,7 +757,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_wwma_tc(TcArgs a, const __grid_
                     put(y, std::integral_constant<int, 0>{});
                 }
                 if (!plain)
-                    mask_staged(reinterpret_cast<float*>(row8), lane, tc, warm, p, has_nan, a.n, a.nan_mode, first_nan,
+                    mask_staged(reinterpret_cast<float*>(row8), lane, tc, warm, p, pmax, a.n, a.nan_mode, first_nan,
                                 a.nan_bits);
                 if (PERM && (unsigned)(a.n - tail - tc) < 32u && c < a.n_combos) {
                     const float* end = reinterpret_cast<const float*>(row8 + ((((a.n - tail - tc) >> 2) ^ (lane & 7)) << 4));
