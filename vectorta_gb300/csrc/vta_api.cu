@@ -151,7 +151,8 @@ static cudaError_t array_alloc(int device, size_t bytes, void** out) {
 }
 
 // Frees a result array (or any other cudaMalloc pointer) of `device`; keep:
-// its block may stay for the next result.
+// its block may stay for the next result.  An idle block is not the caller's
+// any more: freeing it again is the error that a second cudaFree gives.
 cudaError_t array_free(int device, void* ptr, bool keep) {
     int cur = 0;
     cudaGetDevice(&cur);
@@ -160,6 +161,11 @@ cudaError_t array_free(int device, void* ptr, bool keep) {
     bool kept = false;
     {
         std::lock_guard<std::mutex> lock(g_arr_mu);
+        for (const ArrayBlock& b : g_arr_idle)
+            if (b.ptr == ptr) {
+                cudaSetDevice(cur);
+                return cudaErrorInvalidValue;
+            }
         auto it = g_arr_live.find(ptr);
         if (it != g_arr_live.end()) {
             const ArrayBlock b = it->second;
