@@ -111,7 +111,7 @@ static std::mutex g_arr_mu;
 static std::map<void*, ArrayBlock> g_arr_live;   // handed out
 static std::vector<ArrayBlock> g_arr_idle;       // oldest first
 static size_t g_arr_idle_bytes = 0;
-static std::atomic<int> g_contexts{0};
+static std::atomic<int> g_contexts{0};  // (read under g_arr_mu: the last one's end empties the pool after it)
 
 // Gives idle blocks back until at most `keep` bytes remain (g_arr_mu held).
 static void arrays_trim(size_t keep) {
@@ -170,7 +170,8 @@ cudaError_t array_free(int device, void* ptr, bool keep) {
         if (it != g_arr_live.end()) {
             const ArrayBlock b = it->second;
             g_arr_live.erase(it);
-            if (keep && b.device == device && b.bytes <= kArrayIdle / 2 && cudaDeviceSynchronize() == cudaSuccess) {
+            if (keep && g_contexts.load() > 0 && b.device == device && b.bytes <= kArrayIdle / 2 &&
+                cudaDeviceSynchronize() == cudaSuccess) {
                 g_arr_idle.push_back(b);
                 g_arr_idle_bytes += b.bytes;
                 arrays_trim(kArrayIdle);
