@@ -106,80 +106,115 @@ struct ArrayBlock {
     void* ptr;
     size_t bytes;
     int device;
+    bool freeing;  // being freed: not the caller's any more, not idle yet
 };
-static std::mutex g_arr_mu;
+static std::mutex g_arr_mu;  // (held for the lists alone, never over a call that may wait for a device)
 static std::map<void*, ArrayBlock> g_arr_live;   // handed out
 static std::vector<ArrayBlock> g_arr_idle;       // oldest first
 static size_t g_arr_idle_bytes = 0;
 static std::atomic<int> g_contexts{0};  // (read under g_arr_mu: the last one's end empties the pool after it)
 
-// Gives idle blocks back until at most `keep` bytes remain (g_arr_mu held).
-static void arrays_trim(size_t keep) {
+// Takes the oldest idle blocks off the list until at most `keep` bytes remain
+// (g_arr_mu held); arrays_release then gives them back.
+static std::vector<ArrayBlock> arrays_take(size_t keep) {
+    std::vector<ArrayBlock> out;
+    while (!g_arr_idle.empty() && g_arr_idle_bytes > keep) {
+        out.push_back(g_arr_idle.front());
+        g_arr_idle_bytes -= out.back().bytes;
+        g_arr_idle.erase(g_arr_idle.begin());
+    }
+    return out;
+}
+static void arrays_release(const std::vector<ArrayBlock>& blocks) {
+    if (blocks.empty()) return;
     int cur = 0;
     cudaGetDevice(&cur);
-    while (!g_arr_idle.empty() && g_arr_idle_bytes > keep) {
-        const ArrayBlock b = g_arr_idle.front();
-        g_arr_idle.erase(g_arr_idle.begin());
-        g_arr_idle_bytes -= b.bytes;
+    for (const ArrayBlock& b : blocks) {
         cudaSetDevice(b.device);
         cudaFree(b.ptr);
     }
     cudaSetDevice(cur);
 }
+// Gives all idle blocks back; whether there were any.
+static bool arrays_trim() {
+    std::vector<ArrayBlock> out;
+    {
+        std::lock_guard<std::mutex> lock(g_arr_mu);
+        out = arrays_take(0);
+    }
+    arrays_release(out);
+    return !out.empty();
+}
 
 // A block of at least `bytes` on the current device `device`.
 static cudaError_t array_alloc(int device, size_t bytes, void** out) {
-    std::lock_guard<std::mutex> lock(g_arr_mu);
-    const size_t most = bytes + bytes / 4 + (size_t(64) << 10);
-    for (size_t i = g_arr_idle.size(); i-- > 0;) {
-        const ArrayBlock b = g_arr_idle[i];
-        if (b.device != device || b.bytes < bytes || b.bytes > most) continue;
-        g_arr_idle.erase(g_arr_idle.begin() + (long)i);
-        g_arr_idle_bytes -= b.bytes;
-        g_arr_live[b.ptr] = b;
-        *out = b.ptr;
-        return cudaSuccess;
+    {
+        std::lock_guard<std::mutex> lock(g_arr_mu);
+        const size_t most = bytes + bytes / 4 + (size_t(64) << 10);
+        for (size_t i = g_arr_idle.size(); i-- > 0;) {
+            const ArrayBlock b = g_arr_idle[i];
+            if (b.device != device || b.bytes < bytes || b.bytes > most) continue;
+            g_arr_idle.erase(g_arr_idle.begin() + (long)i);
+            g_arr_idle_bytes -= b.bytes;
+            g_arr_live[b.ptr] = b;
+            *out = b.ptr;
+            return cudaSuccess;
+        }
     }
     cudaError_t e = cudaMalloc(out, bytes);
-    if (e != cudaSuccess && !g_arr_idle.empty()) {
+    if (e != cudaSuccess && arrays_trim()) {
         cudaGetLastError();
-        arrays_trim(0);
         e = cudaMalloc(out, bytes);
     }
-    if (e == cudaSuccess) g_arr_live[*out] = ArrayBlock{*out, bytes, device};
+    if (e == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(g_arr_mu);
+        g_arr_live[*out] = ArrayBlock{*out, bytes, device, false};
+    }
     return e;
 }
 
 // Frees a result array (or any other cudaMalloc pointer) of `device`; keep:
 // its block may stay for the next result.  An idle block is not the caller's
 // any more: freeing it again is the error that a second cudaFree gives.
+static cudaError_t array_free_here(int device, void* ptr, bool keep) {
+    {
+        std::lock_guard<std::mutex> lock(g_arr_mu);
+        for (const ArrayBlock& b : g_arr_idle)
+            if (b.ptr == ptr) return cudaErrorInvalidValue;
+        auto it = g_arr_live.find(ptr);
+        if (it == g_arr_live.end()) {
+            keep = false;
+        } else {
+            ArrayBlock& b = it->second;
+            if (b.freeing) return cudaErrorInvalidValue;
+            keep = keep && g_contexts.load() > 0 && b.device == device && b.bytes <= kArrayIdle / 2;
+            if (keep) b.freeing = true;
+            else g_arr_live.erase(it);
+        }
+    }
+    if (!keep) return cudaFree(ptr);
+    bool kept = cudaDeviceSynchronize() == cudaSuccess;
+    std::vector<ArrayBlock> over;
+    {
+        std::lock_guard<std::mutex> lock(g_arr_mu);
+        ArrayBlock b = g_arr_live[ptr];
+        g_arr_live.erase(ptr);
+        kept = kept && g_contexts.load() > 0;
+        if (kept) {
+            b.freeing = false;
+            g_arr_idle.push_back(b);
+            g_arr_idle_bytes += b.bytes;
+            over = arrays_take(kArrayIdle);
+        }
+    }
+    arrays_release(over);
+    return kept ? cudaSuccess : cudaFree(ptr);
+}
 cudaError_t array_free(int device, void* ptr, bool keep) {
     int cur = 0;
     cudaGetDevice(&cur);
     cudaSetDevice(device);
-    cudaError_t e = cudaSuccess;
-    bool kept = false;
-    {
-        std::lock_guard<std::mutex> lock(g_arr_mu);
-        for (const ArrayBlock& b : g_arr_idle)
-            if (b.ptr == ptr) {
-                cudaSetDevice(cur);
-                return cudaErrorInvalidValue;
-            }
-        auto it = g_arr_live.find(ptr);
-        if (it != g_arr_live.end()) {
-            const ArrayBlock b = it->second;
-            g_arr_live.erase(it);
-            if (keep && g_contexts.load() > 0 && b.device == device && b.bytes <= kArrayIdle / 2 &&
-                cudaDeviceSynchronize() == cudaSuccess) {
-                g_arr_idle.push_back(b);
-                g_arr_idle_bytes += b.bytes;
-                arrays_trim(kArrayIdle);
-                kept = true;
-            }
-        }
-    }
-    if (!kept) e = cudaFree(ptr);
+    const cudaError_t e = array_free_here(device, ptr, keep);
     cudaSetDevice(cur);
     return e;
 }
@@ -192,11 +227,7 @@ vta_status vram_check(size_t required) {
     const size_t headroom = size_t(64) << 20;
     if (required + headroom > free_b) {
         // give the idle result blocks back and look again
-        std::lock_guard<std::mutex> lock(g_arr_mu);
-        if (!g_arr_idle.empty()) {
-            arrays_trim(0);
-            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return VTA_OK;
-        }
+        if (arrays_trim() && cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return VTA_OK;
     }
     if (required + headroom > free_b) {
         char buf[160];
@@ -2209,10 +2240,7 @@ vta_status vta_ctx_destroy(vta_ctx* ctx) {
     if (g_cur == ctx) g_cur = nullptr;
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
-    if (g_contexts.fetch_sub(1) == 1) {  // the last one
-        std::lock_guard<std::mutex> lock(g_arr_mu);
-        arrays_trim(0);
-    }
+    if (g_contexts.fetch_sub(1) == 1) arrays_trim();  // the last one
     return VTA_OK;
 }
 
