@@ -1,12 +1,11 @@
 """Result arrays and the library's pool of freed blocks: freeing one twice, and
 freeing one after the last context (in a process of its own: other tests'
-contexts would keep the pool), and beside another thread's calls."""
+contexts would keep the pool), and beside another thread's stream capture."""
 import ctypes as C
 import os
 import subprocess
 import sys
 import threading
-import time
 
 import numpy as np
 import pytest
@@ -72,27 +71,32 @@ def test_no_block_outlives_the_last_context():
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
 
 
-def test_a_waiting_free_holds_up_no_other_thread():
+def test_free_beside_another_threads_capture():
     import torch
 
     x = datagen.random_walk(3000, seed=4).astype(np.float32)
-    sma, ema = V.CudaSma(0), V.CudaEma(0)
-    sweep = {"period": (2, 60, 1)}
-    ema.batch_dev(x, sweep=sweep).free()
-    a = sma.batch_dev(x, sweep=sweep)
-    hold = [ema.batch_dev(x, sweep=sweep) for _ in range(4)]  # no idle block is left for the next result
-    side = torch.cuda.Stream()
+    sma = V.CudaSma(0)
+    a = sma.batch_dev(x, sweep={"period": (2, 60, 1)})
+    y = torch.ones(1000, device="cuda")
+    ready, done = threading.Event(), threading.Event()
+
+    def free():
+        ready.wait()
+        a.free()
+        done.set()
+
+    t = threading.Thread(target=free)
+    t.start()
+    g = torch.cuda.CUDAGraph()
+    try:
+        with torch.cuda.graph(g, capture_error_mode="thread_local"):
+            z = y * 2
+            ready.set()
+            done.wait(30)
+            z = z + 1
+    finally:
+        ready.set()
+        t.join()
+    g.replay()
     torch.cuda.synchronize()
-    with torch.cuda.stream(side):
-        torch.cuda._sleep(int(1.5e9))  # 0.7 s and more
-    freed = threading.Thread(target=a.free)
-    freed.start()
-    time.sleep(0.05)
-    t = time.perf_counter()
-    r = ema.batch_dev(x, sweep=sweep)
-    took = time.perf_counter() - t
-    busy = not side.query()
-    freed.join()
-    assert busy and took < 0.3, took
-    for h in (*hold, r):
-        h.free()
+    assert torch.all(z == 3)

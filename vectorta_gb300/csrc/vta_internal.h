@@ -96,6 +96,7 @@ struct vta_ctx {
     size_t aux_bytes = 0;     // builds after the call's arena pieces are taken)
     void* io = nullptr;       // device inputs + outputs of *_batch_into_host_f32 (host_io cached)
     size_t io_bytes = 0;
+    void* mark = nullptr;     // a small allocation (see device_wait)
     void* tmp = nullptr;      // row-major staging of time-major MA-computer outputs
     size_t tmp_bytes = 0;
     void* host_stage = nullptr;  // pinned staging of small uploads, reused per call
