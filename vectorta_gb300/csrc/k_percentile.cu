@@ -379,6 +379,7 @@ __global__ void __launch_bounds__(kGrowTile) k_pnr_grow(PnrGrow a) {
 
 constexpr int kMaxSpan = 4096;              // ranks of the 64-bit bitmap form
 constexpr int kMinTile = 256, kMaxTile = 1024;
+constexpr size_t kMaxGridY = 65535;         // runs of a launch of the growing walk
 constexpr size_t kSlabBytes = size_t(128) << 20;  // ranks and values of one slab of tiles
 
 // Times per tile: the largest of 256, 512, 1024 that is at most the longest
@@ -495,11 +496,9 @@ vta_status launch_pnr_sweep(const PnrArgs& p, const PnrPlan& plan, const int4* i
     if (plan.grow) {
         w.first = p.first;
         w.items = items;
-        w.runs = runs;
         w.nwords = nwords;
         w.out = p.out;
         smem = tables + (size_t)nwords * kGrowTile * word;
-        if (plan.runs.size() > 65535) return fail(VTA_ERR_LAUNCH_CONFIG_TOO_LARGE, "percentile: too many percentages");
         VTA_CUDA_TRY(cudaFuncSetAttribute(grow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     } else {
         s.first = p.first;
@@ -532,9 +531,16 @@ vta_status launch_pnr_sweep(const PnrArgs& p, const PnrPlan& plan, const int4* i
         k_pnr_ranks<<<m, rank_threads, (size_t)g.spad * sizeof(float), st>>>(t);
         VTA_TRY(check_launch("k_pnr_ranks"));
         s.t = w.t = t;
-        if (plan.grow) grow<<<dim3(m, (unsigned)plan.runs.size()), kGrowTile, smem, st>>>(w);
-        else slide<<<s.groups * m, kSwThreads, smem, st>>>(s);
-        VTA_TRY(check_launch(plan.grow ? "k_pnr_grow" : "k_pnr_slide"));
+        if (plan.grow) {
+            for (size_t r = 0; r < plan.runs.size(); r += kMaxGridY) {
+                w.runs = runs + r;
+                grow<<<dim3(m, (unsigned)std::min(kMaxGridY, plan.runs.size() - r)), kGrowTile, smem, st>>>(w);
+                VTA_TRY(check_launch("k_pnr_grow"));
+            }
+        } else {
+            slide<<<s.groups * m, kSwThreads, smem, st>>>(s);
+            VTA_TRY(check_launch("k_pnr_slide"));
+        }
     }
     ktimer_end(st);
     return VTA_OK;
