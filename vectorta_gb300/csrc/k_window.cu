@@ -14,6 +14,7 @@
 // valid index poisons every later output of that series, an infinite input
 // every output from p steps after it (where it leaves the window: inf - inf).
 #include <algorithm>
+#include <numeric>
 
 #include "pnr_ops.cuh"
 #include "vta_internal.h"
@@ -1193,17 +1194,21 @@ __global__ void k_percentile(PnrArgs a) {
 // grid in (nearly) whole waves of the kernel's resident blocks, counting a
 // group's per-tile set-up (prefix or table rebuild) as ~4 combos of work.
 //
-// `drift`: where that makes long blocks (over 24 combos) of a series with a
-// tile per SM or more, a few waves of shorter blocks instead, the least of
-// (waves + 1) x (combos + 6).  Blocks of one full wave set up and store in
-// step, each row of the whole series at a time; shorter ones drift apart.  us
-// of a call, one wave / a few, prefix windows: 299 SMAs on 180k, 300k and 600k
-// bars 70 / 53, 100 / 73, 188 / 131, 250 Bollinger rows 129 / 103, 196 / 155,
-// 379 / 291; below a tile per SM the reverse (80k: 27.8 / 30.5, StdDev on 120k
-// 49 / 53), and for the min/max kernels throughout (100 Williams %R on 1M bars
-// 92 / 131).
+// `drift` (0: not): where that makes long blocks (over 24 combos) of a series
+// with at least `min_tiles` tiles per SM, a few waves of shorter blocks instead,
+// the least of (waves + 1) x (combos + drift), drift being a group's set-up in
+// combos.  Blocks of one full wave set up and store in step, each row of the
+// whole series at a time; shorter ones drift apart.  A long set-up (over 8
+// combos, and a fifth of a block) leaves less to gain: then from 1.9 tiles per
+// SM on.  us of a call, one wave / a few, prefix windows: 299 SMAs on 180k, 300k
+// and 600k bars 70 / 53, 100 / 73, 188 / 131, 250 Bollinger rows 129 / 103, 196 /
+// 155, 379 / 291; 100 SMAs of 25..2500 on 200k 31 / 34, 300 Bollinger rows of
+// 108..2500 156 / 143; below a tile per SM the reverse (80k: 27.8 / 30.5, StdDev
+// on 120k 49 / 53), and for the min/max kernels throughout (100 Williams %R on 1M
+// bars 92 / 131).
 template <class K>
-static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_combos, bool drift = false) {
+static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_combos, double drift = 0.,
+                       double min_tiles = 1.) {
     int per_sm = 0, dev = 0, sms = kNumSMs;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem) != cudaSuccess) {
         cudaGetLastError();
@@ -1211,7 +1216,7 @@ static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_
     }
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long slots = (long long)std::max(1, per_sm) * sms;
-    const int gmax = std::min(drift ? 24 : 16, n_combos);
+    const int gmax = std::min(drift > 0. ? 24 : 16, n_combos);
     auto pick = [&](bool waves) {
         int best_cpb = n_combos;
         double best = 1e300;
@@ -1219,7 +1224,7 @@ static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_
             const int cpb = (n_combos + g - 1) / g;
             const long long blocks = tiles * ((n_combos + cpb - 1) / cpb);
             const double cost = waves ? (double)((blocks + slots - 1) / slots) * (cpb + 4)
-                                      : ((double)blocks / slots + 1.) * (cpb + 6);
+                                      : ((double)blocks / slots + 1.) * (cpb + drift);
             if (cost < best * (waves ? 0.98 : 1.)) {
                 best = cost;
                 best_cpb = cpb;
@@ -1228,7 +1233,8 @@ static int wave_combos(K kern, int threads, size_t smem, long long tiles, int n_
         return best_cpb;
     };
     const int cpb = pick(true);
-    return drift && cpb > 24 && tiles >= sms ? pick(false) : cpb;
+    if (drift > 8. && cpb < 5. * drift) min_tiles = 1.9;
+    return drift > 0. && cpb > 24 && tiles >= min_tiles * sms ? pick(false) : cpb;
 }
 
 vta_status launch_prefix_window_batch(const PrefixWinArgs& a, int pmax, size_t smem_optin, cudaStream_t st) {
@@ -1241,13 +1247,14 @@ vta_status launch_prefix_window_batch(const PrefixWinArgs& a, int pmax, size_t s
     // 111 (200,000: 102), on 100,001 90 / 78, on 50,001 51.5 / 51.1, on 30,001
     // 31.6 / 34.3; SMA rows 404 / 270 (399 on 1,000,001 bars), 124 / 116 (299
     // on 500,001), 46 / 53 (199 on 200,001); StdDev, bound by arithmetic, 183 /
-    // 200 (299 on 500,001).
+    // 200 (299 on 500,001).  Three blocks' prefixes have to fit an SM: 100
+    // Bollinger rows of 50..5000 on 300,001 bars 154 / 169, of 35..3500 124 / 112.
     const auto at = [](const float* o) { return reinterpret_cast<uintptr_t>(o) % 32; };
     const int outs = a.kind == WK_BB ? 3 : 1;
     const bool cut = (a.kind == WK_SMA || a.kind == WK_BB) && (a.n % 4 != 0 || at(a.out0) % 16 != 0) &&
                      (outs == 1 || (at(a.out1) == at(a.out0) && at(a.out2) == at(a.out0))) &&
                      (size_t)a.n_combos * a.n * sizeof(float) * outs >= (outs == 1 ? 8 : 4) * kCutBytes &&
-                     smem + 8 * slot + fixed <= smem_optin;
+                     3 * (smem + 8 * slot + fixed) <= smem_optin;
     const auto kernel = cut ? k_prefix_window_batch<true> : k_prefix_window_batch<false>;
     if (cut) smem += 8 * slot;
     if (smem + fixed > smem_optin)
@@ -1259,7 +1266,16 @@ vta_status launch_prefix_window_batch(const PrefixWinArgs& a, int pmax, size_t s
     }
     VTA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long long tiles = ceil_div(a.n + (cut ? 7 : 0), kPwTile);
-    const int cpb = wave_combos(kernel, kPwThreads, smem, tiles, a.n_combos, true);
+    // A block's set-up scans its tile and the longest window before it, `per`
+    // consecutive slots a thread, at a bank conflict of the greatest common
+    // divisor of per and 16: 6 combos' time at windows of 300 bars (100 SMAs of
+    // 50..5000 on 300,001 bars, with it as at 300 bars / so 126 / 78 us).  Between
+    // 1 and 1.1 tiles per SM the cheaper kinds lose by the drift (100 SMAs of
+    // 3..300 on 160k bars 25 / 28, Bollinger rows 49 / 45).
+    const int span = kPwTile + pmax + (cut ? 8 : 0), per = ceil_div(span, kPwThreads);
+    const double setup = std::max(6., 3. * span / (kPwTile + 300) * std::gcd(per, 16));
+    const int cpb =
+        wave_combos(kernel, kPwThreads, smem, tiles, a.n_combos, setup, a.kind == WK_BB ? 1. : 1.1);
     ktimer_begin(st);
     kernel<<<dim3((unsigned)tiles, (unsigned)ceil_div(a.n_combos, cpb)), kPwThreads, smem, st>>>(a, pmax, cpb);
     ktimer_end(st);
