@@ -143,8 +143,9 @@ void* vta_ctx_get_stream(vta_ctx* ctx);
  *   "tm_warm"     = "auto" | <steps>   (plans; chunked ADX/SuperTrend sweeps)
  *   "timing"      = "on" | "off"
  *   "host_io"     = "cached" | "per_call": *_batch_into_host_f32 keeps its
- *                   device input/output buffer in the context between calls
- *                   (cached, the default; freed by per_call or ctx destroy) */
+ *                   device input/output buffer in the context between calls,
+ *                   *_dev calls theirs for up to 64 MiB of inputs (cached, the
+ *                   default; freed by per_call or ctx destroy) */
 vta_status vta_ctx_set_policy(vta_ctx* ctx, const char* key, const char* value);
 /* selected_batch_kernel() (alma_wrapper.rs:239-245): name of the last kernel
  * path used by this context. */
@@ -165,6 +166,9 @@ typedef struct vta_device_array {
     size_t cols;
     int device;
 } vta_device_array;
+/* Waits for the device's work; the memory may be kept for later results (at
+ * most 256 MiB a process, given back when a call needs it and with the last
+ * context). */
 vta_status vta_device_array_free(vta_device_array* arr);
 vta_status vta_device_array_copy_to_host(vta_ctx* ctx, const vta_device_array* arr,
                                          float* host, size_t n);
@@ -326,7 +330,8 @@ w("""/* ==== many-series work-list plans ====
  * time chunk) items, captured once in a CUDA graph at creation and replayed
  * by vta_tm_plan_run.  The time-chunk length of each job is picked by timing
  * candidates on the plan's own data at creation (cached per indicator,
- * period, length and series count for the process); the context policies
+ * period, length and series count for the process), a mixed plan's also
+ * together; the context policies
  * "tm_chunk" and "tm_warm" override it.  Results are bit-identical to one
  * sequential pass per series (the chunking is verified and repaired on the
  * device), and per cell they follow the crate's many-series semantics:
