@@ -25,7 +25,11 @@
  *     return once their work is queued, like the crate's x_batch_device /
  *     x_many_series_one_param_device: read their outputs after
  *     vta_ctx_synchronize (CudaX::synchronize) or from work queued behind them
- *     on the same stream.
+ *     on the same stream.  A failure of such work on the device (a weighted-
+ *     window sweep whose pipeline wait ran out: some rows are incomplete) is
+ *     reported once, as VTA_ERR_CUDA naming the sweep, by vta_ctx_synchronize
+ *     or by the next call on the context, which then does not run; a caller
+ *     that waits by an event of its own learns of it there.
  * Thread safety: a vta_ctx is used by one thread at a time (as a CudaX is).
  */
 #ifndef VTA_GB300_H

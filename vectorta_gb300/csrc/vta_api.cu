@@ -822,6 +822,8 @@ static vta_status run_batch(vta_ctx* ctx, Ind ind, const DevIn& in, size_t len, 
             const vta_status s = launch_wwma_batch_tc(a, pol == 3 ? 1 : 0, ctx, st);
             if (s == VTA_OK) {
                 ctx->last_kernel = pol == 3 ? "wwma_tc_bf16x3" : "wwma_tc_fp16x3";
+                ctx->tc_call = std::string(kInfo[ind].name) + ", " + std::to_string(nc) + " rows of " +
+                               std::to_string(n) + " bars";
                 return VTA_OK;
             }
             if (s != VTA_ERR_NOT_IMPLEMENTED || pol >= 2) return s;
@@ -1566,11 +1568,11 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
 }
 
 // ------------------------------------------------------------ drivers ------
-static vta_status tc_error(vta_ctx* ctx);
+static vta_status tc_error(vta_ctx* ctx, bool entering);
 static vta_status check_ctx(vta_ctx* ctx) {
     if (!ctx) return fail(VTA_ERR_INVALID_INPUT, "null context");
     VTA_CUDA_TRY(cudaSetDevice(ctx->device));
-    VTA_TRY(tc_error(ctx));
+    VTA_TRY(tc_error(ctx, true));
     g_cur = ctx;
     ctx->timed = false;
     // the pinned staging buffer is reused once the copies of the calls that
@@ -1585,17 +1587,20 @@ static vta_status check_ctx(vta_ctx* ctx) {
 
 // A pipeline wait of the tensor-core contraction that ran out (the kernel's
 // word in mapped host memory; server slots read theirs when a request
-// completes).  Reported once, by the call that next waits for the context's
-// work or enters it.
-static vta_status tc_error(vta_ctx* ctx) {
+// completes).  Reported once: by the call that next waits for the context's
+// work, its own or an earlier call's, or by the call that next enters the
+// context, which then does not run.
+static vta_status tc_error(vta_ctx* ctx, bool entering) {
     if (!ctx->err_host || ctx->async_alloc || *static_cast<volatile int*>(ctx->err_host) == 0) return VTA_OK;
     *ctx->err_host = 0;
-    return fail(VTA_ERR_CUDA, "tcgen05 contraction: pipeline wait timed out");
+    return fail(VTA_ERR_CUDA, "tcgen05 contraction: pipeline wait timed out; rows of a weighted-window sweep are "
+                              "incomplete (the last one queued on this context: " + ctx->tc_call + ")" +
+                              (entering ? "; reported by this call, which did not run" : ""));
 }
 
 static vta_status sync(vta_ctx* ctx) {
     VTA_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    VTA_TRY(tc_error(ctx));
+    VTA_TRY(tc_error(ctx, false));
     return check_async("stream");
 }
 

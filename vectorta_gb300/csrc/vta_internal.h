@@ -112,6 +112,7 @@ struct vta_ctx {
     // the device; the tensor-core path leaves its error word in err_host
     bool async_alloc = false;
     int* err_host = nullptr;         // pinned
+    std::string tc_call;             // the last sweep on the tensor-core path
     cudaMemPool_t pool = nullptr;    // stream-ordered allocations of async slots
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // constant cache: small per-sweep arrays (period lists, per-combo
