@@ -1258,10 +1258,10 @@ __device__ __forceinline__ float2 pair_scan(float2 v) {  // inclusive over the w
 __device__ __forceinline__ float2 pair_shfl(float2 v, int src) {
     return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
-// sum / p, from a compensated sum, correctly rounded up to the last bit
+// sum / p from a compensated sum, in f64 as the crate forms its seeds (once per
+// combo: a pair of floats would lose the residual of sums near 2^-120)
 __device__ __forceinline__ float pair_mean(float2 sum, int p) {
-    const D2 m = d2_mul(D2{sum.x, sum.y}, d2_ratio(1, p));
-    return m.hi + m.lo;
+    return (float)(((double)sum.x + (double)sum.y) / (double)p);
 }
 
 // The prefix of the terms over [f, c0) and whether every input of [f, tend) is
