@@ -1308,10 +1308,21 @@ __device__ __forceinline__ float2 pair_scan(float2 v) {  // inclusive over the w
 __device__ __forceinline__ float2 pair_shfl(float2 v, int src) {
     return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
-// sum / p from a compensated sum, in f64 as the crate forms its seeds (once per
-// combo: a pair of floats would lose the residual of sums near 2^-120)
-__device__ __forceinline__ float pair_mean(float2 sum, int p) {
-    return (float)(((double)sum.x + (double)sum.y) / (double)p);
+// sum / p from a compensated sum as f64 gives it, inv = 1 / p.  The residual of
+// the first quotient is exact by FMA, so q + c is the mean up to 2^-45 of it
+// (scaled where the residual of a small sum would underflow); where 2^-40 more
+// or less rounds alike, so does the mean, and only the others (ties of short
+// periods, one seed in 2^15) are divided in f64.  An f64 division in the chain
+// of every tile that holds a seed took RSI of 58 periods on 5,003 bars from 51
+// to 63 us.
+__device__ __forceinline__ float pair_mean(float2 sum, int p, float inv) {
+    const bool small = fabsf(sum.x) < 0x1p-40f;
+    const float k = small ? 0x1p80f : 1.f, hi = sum.x * k, lo = sum.y * k;
+    const float q = hi * inv, c = (fmaf(-q, (float)p, hi) + lo) * inv, eps = fabsf(q) * 0x1p-40f;
+    const float a = q + (c + eps), b = q + (c - eps);
+    const float m = a * (small ? 0x1p-80f : 1.f);
+    const bool sure = a == b && p < coef::kExact && (!small || fabsf(m) >= 0x1p-126f);
+    return sure ? m : (float)(((double)sum.x + (double)sum.y) / (double)p);
 }
 
 // The prefix of the terms over [f, c0) and whether every input of [f, tend) is
@@ -1416,7 +1427,7 @@ __device__ __forceinline__ void warm_tile(Op& op, int f, int tb, int nt, float x
     } else if constexpr (std::is_same<Op, OpRsi<true>>::value) {
         const float2 ga = pair_shfl(w.a, sl), la = pair_shfl(w.b, sl);
         const int p = (int)op.pf;
-        const float sg = here ? pair_mean(ga, p) : 0.f, sl_ = here ? pair_mean(la, p) : 0.f;
+        const float sg = here ? pair_mean(ga, p, op.inv_p) : 0.f, sl_ = here ? pair_mean(la, p, op.inv_p) : 0.f;
         float ag = op.ag, al = op.al;
 #pragma unroll 8
         for (int j = 0; j < 32; ++j) {
@@ -1435,7 +1446,7 @@ __device__ __forceinline__ void warm_tile(Op& op, int f, int tb, int nt, float x
         op.al = al;
     } else {  // Wilders, ATR
         const float2 sum = pair_shfl(w.a, sl);
-        const float seed = here ? pair_mean(sum, op.p) : 0.f;
+        const float seed = here ? pair_mean(sum, op.p, op.alpha) : 0.f;
         const bool copy = std::is_same<Op, OpWilders>::value && op.p == 1;
         float y = op.y;
 #pragma unroll 8
