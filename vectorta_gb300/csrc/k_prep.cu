@@ -71,7 +71,7 @@ k_first_valid_tm(const float* __restrict__ h, const float* __restrict__ l, const
 }
 
 // First NaN after each series' first valid row, and first value of magnitude
-// above 2^60 (infinite ones too): first_nan[s] and first_big[s] (may be null)
+// above `limit` (infinite ones too): first_nan[s] and first_big[s] (may be null)
 // hold `rows` (set by k_first_valid_tm) and are lowered to the row.  Blocks of
 // 128 series x 64 rows read the whole matrix once (one thread per series
 // walking its rows took 1,073 us for 3,000 x 2,520; now 11).
@@ -79,7 +79,7 @@ constexpr int kFnRows = 64, kFnBatch = 16;
 
 __global__ void __launch_bounds__(128)
 k_first_nan_tm(const float* __restrict__ x, int cols, int rows, const int* __restrict__ first, int* first_nan,
-               int* first_big) {
+               int* first_big, float limit) {
     const int s = blockIdx.x * 128 + threadIdx.x;
     if (s >= cols) return;
     const int f = first[s];
@@ -95,7 +95,7 @@ k_first_nan_tm(const float* __restrict__ x, int cols, int rows, const int* __res
 #pragma unroll
             for (int j = 0; j < kFnBatch; ++j) {
                 if (j < m && tb + j > f && isnan(v[j])) found = min(found, tb + j);
-                if (j < m && fabsf(v[j]) > 0x1p60f) big = min(big, tb + j);
+                if (j < m && fabsf(v[j]) > limit) big = min(big, tb + j);
             }
         }
     }
@@ -218,13 +218,14 @@ __global__ void k_prefix_apply(const float* __restrict__ x, int n, int first, in
 }  // namespace
 
 vta_status launch_first_valid_tm(const float* x_tm, int cols, int rows, int* first, cudaStream_t st,
-                                 int* first_nan, int* first_big) {
+                                 int* first_nan, int* first_big, float limit) {
     k_first_valid_tm<false><<<ceil_div(cols, 32), 32 * kFvWarps, 0, st>>>(nullptr, nullptr, x_tm, cols, rows, nullptr,
                                                                          first, nullptr, first_nan, first_big);
     VTA_TRY(check_launch("k_first_valid_tm"));
     if (!first_nan) return VTA_OK;
     const unsigned ny = std::min(ceil_div(rows, kFnRows), 65535u);
-    k_first_nan_tm<<<dim3(ceil_div(cols, 128), ny), 128, 0, st>>>(x_tm, cols, rows, first, first_nan, first_big);
+    k_first_nan_tm<<<dim3(ceil_div(cols, 128), ny), 128, 0, st>>>(x_tm, cols, rows, first, first_nan, first_big,
+                                                                  limit);
     return check_launch("k_first_nan_tm");
 }
 

@@ -1453,7 +1453,10 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
     const bool wsums = ind == I_WMA || ind == I_SWMA || ind == I_TRIMA;
     int* d_first_nan = sums || wsums ? d_first + C : nullptr;
     int* d_first_big = sums ? d_first_nan + C : nullptr;
-    if (kInfo[ind].in == IN_X) VTA_TRY(launch_first_valid_tm(in.p[0], C, R, d_first, st, d_first_nan, d_first_big));
+    // values up to it keep the p + 1 squares of a sliding window below 2^126
+    const float big = std::min(0x1p60f, 0x1p63f / std::sqrt((float)p + 1.f));
+    if (kInfo[ind].in == IN_X)
+        VTA_TRY(launch_first_valid_tm(in.p[0], C, R, d_first, st, d_first_nan, d_first_big, big));
     else if (ind == I_DONCHIAN) VTA_TRY(launch_first_valid_tm_hlc(in.p[0], in.p[1], in.p[1], C, R, d_first, st));
     else VTA_TRY(launch_first_valid_tm_hlc(in.p[0], in.p[1], in.p[2], C, R, d_first, st));
 

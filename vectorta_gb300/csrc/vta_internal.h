@@ -193,9 +193,9 @@ inline unsigned ceil_div(size_t a, size_t b) { return (unsigned)((a + b - 1) / b
 
 // First valid (non-NaN) index of each time-major series; rows if all NaN.
 // first_nan (may be null): the first NaN after it; rows if there is none.
-// first_big (null without first_nan): the first value of magnitude above 2^60.
+// first_big (null without first_nan): the first value of magnitude above limit.
 vta_status launch_first_valid_tm(const float* x_tm, int cols, int rows, int* first, cudaStream_t st,
-                                 int* first_nan = nullptr, int* first_big = nullptr);
+                                 int* first_nan = nullptr, int* first_big = nullptr, float limit = 0.f);
 // Same over the three HLC inputs (first index where all three are non-NaN).
 // len (may be null): per-series lengths in place of rows; first_c (may be
 // null): the first valid index of c alone.
@@ -468,7 +468,7 @@ struct PrefixWinTmArgs {
     int cols, rows;
     const int* first;
     const int* first_nan;  // first NaN after first[s] (rows: none)
-    const int* first_big;  // first value above 2^60 in magnitude (rows: none)
+    const int* first_big;  // first value whose square or sum may overflow a window (rows: none)
     int period;
     float k1, k2;
     float* out0;
