@@ -334,8 +334,8 @@ w("""/* ==== many-series work-list plans ====
  * time chunk) items, captured once in a CUDA graph at creation and replayed
  * by vta_tm_plan_run.  The time-chunk length of each job is picked by timing
  * candidates on the plan's own data at creation (cached per indicator,
- * period, length and series count for the process), a mixed plan's also
- * together; the context policies
+ * period, length and series count for the process and, with VTA_TUNE_CACHE,
+ * in its files), a mixed plan's also together; the context policies
  * "tm_chunk" and "tm_warm" override it.  Results are bit-identical to one
  * sequential pass per series (the chunking is verified and repaired on the
  * device), and per cell they follow the crate's many-series semantics:

@@ -196,7 +196,9 @@ vta_status plan_enqueue(vta_tm_plan* P, int n_jobs, cudaStream_t st, bool with_f
 // ---------------------------------------------------------------- tuning ----
 // Chunk length per (indicator, period, length bucket, series-count bucket),
 // for the process; with VTA_TUNE_CACHE=<file> also read from and appended to
-// that file ("kind period len_bucket cols_bucket chunk" per line).
+// that file ("kind period len_bucket cols_bucket chunk" per line); a mixed
+// plan's choice (tune_mix) in <file>.mixes: the number of jobs, then per job its
+// key, the chunk picked for it alone and the one kept.
 using TuneKey = std::tuple<int, int, int, int>;
 std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tune;
@@ -221,6 +223,37 @@ void tune_load_locked() {
     while (std::fscanf(f, "%d %d %d %d %d", &k, &p, &lb, &cb, &ch) == 5)
         if (ch > 0) g_tune[TuneKey{k, p, lb, cb}] = ch;
     std::fclose(f);
+    f = std::fopen((std::string(path) + ".mixes").c_str(), "r");
+    if (!f) return;
+    int n;
+    while (std::fscanf(f, "%d", &n) == 1 && n > 0 && n <= 64) {
+        std::vector<TuneKey> keys;
+        std::vector<int> own, kept;
+        int o, c;
+        while ((int)keys.size() < n && std::fscanf(f, "%d %d %d %d %d %d", &k, &p, &lb, &cb, &o, &c) == 6 && c > 0) {
+            keys.emplace_back(k, p, lb, cb);
+            own.push_back(o);
+            kept.push_back(c);
+        }
+        if ((int)keys.size() < n) break;
+        g_tune_mix[{keys, own}] = kept;
+    }
+    std::fclose(f);
+}
+
+void tune_store_mix_locked(const std::vector<TuneKey>& keys, const std::vector<int>& own,
+                           const std::vector<int>& kept) {
+    g_tune_mix[{keys, own}] = kept;
+    const char* path = std::getenv("VTA_TUNE_CACHE");
+    if (!path || !*path) return;
+    if (FILE* f = std::fopen((std::string(path) + ".mixes").c_str(), "a")) {
+        std::fprintf(f, "%d", (int)keys.size());
+        for (size_t j = 0; j < keys.size(); ++j)
+            std::fprintf(f, " %d %d %d %d %d %d", std::get<0>(keys[j]), std::get<1>(keys[j]), std::get<2>(keys[j]),
+                         std::get<3>(keys[j]), own[j], kept[j]);
+        std::fputc('\n', f);
+        std::fclose(f);
+    }
 }
 
 void tune_store_locked(const TuneKey& key, int chunk) {
@@ -261,7 +294,7 @@ vta_status time_run(vta_tm_plan* P, int n_jobs, float* ms) {
 // and both, and keeps the fastest (ATR, ADX, SuperTrend and percentile(50) of
 // ragged series, us, as picked / kept: 200 x 20,000 rows 190 / 148, 512 x 20,000
 // 295 / 260, 128 x 12,000 135 / 98).  `keys`: the jobs' tuning keys; the choice
-// is kept for the process.
+// is kept like theirs.
 vta_status tune_mix(vta_tm_plan* P, const std::vector<int>& all, const std::vector<TuneKey>& keys) {
     const int n = (int)all.size(), maxlen = *std::max_element(P->lens.begin(), P->lens.end());
     auto lengthened = [&](const std::vector<int>& own, int quarter_warm, bool windows) {
@@ -305,8 +338,9 @@ vta_status tune_mix(vta_tm_plan* P, const std::vector<int>& all, const std::vect
     }
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
-        g_tune_mix[{keys, own}] = best;
+        tune_store_mix_locked(keys, own, best);
     }
+    P->tuned = true;
     return use(best);
 }
 
