@@ -78,6 +78,9 @@ vta_status plan_states(vta_tm_plan* P, int j, int chunk) {
     plan_free(P, J.st_start);
     plan_free(P, J.st_end);
     plan_free(P, J.exact);
+    J.st_start = J.st_end = nullptr;
+    J.exact = nullptr;
+    P->state_cap[j] = 0;
     void *a = nullptr, *b = nullptr, *e = nullptr;
     const size_t words = nch * (size_t)P->cols * 8;
     VTA_TRY(plan_alloc(P, words * sizeof(float), &a));
@@ -131,6 +134,7 @@ vta_status plan_items(vta_tm_plan* P, const std::vector<int>& which) {
     if (keys.size() > (size_t)INT32_MAX) return fail(VTA_ERR_LAUNCH_CONFIG_TOO_LARGE, "tm plan: too many work items");
     if (keys.size() > P->items_cap) {
         plan_free(P, P->d_items);
+        P->items_cap = 0;
         void* p = nullptr;
         VTA_TRY(plan_alloc(P, std::max<size_t>(keys.size(), 1) * sizeof(int4), &p));
         P->d_items = static_cast<int4*>(p);
@@ -138,6 +142,7 @@ vta_status plan_items(vta_tm_plan* P, const std::vector<int>& which) {
     }
     if (lanes.size() > P->lanes_cap) {
         plan_free(P, P->d_lanes);
+        P->lanes_cap = 0;
         void* p = nullptr;
         VTA_TRY(plan_alloc(P, lanes.size() * sizeof(int), &p));
         P->d_lanes = static_cast<int*>(p);
@@ -344,6 +349,18 @@ vta_status tune_mix(vta_tm_plan* P, const std::vector<int>& all, const std::vect
     return use(best);
 }
 
+// Chunks shorter than these take states (64 bytes per series and chunk) and list
+// entries that longer ones don't: they are used only where those take less than
+// 1/64 of the free memory, so that a plan which fits without them still does.
+int safe_chunk(const PlanJob& J) { return plan_job_recurrent(J.kind) ? 1024 : 128; }
+bool chunk_fits(const vta_tm_plan* P, const PlanJob& J, int chunk) {
+    if (chunk >= safe_chunk(J)) return true;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return true;
+    const size_t cells = (size_t)P->cols * n_chunks_of(P->rows, chunk);
+    return cells * (plan_job_recurrent(J.kind) ? 70 : 5) <= free_b / 64;
+}
+
 // Times job j alone with each candidate chunk length (second of two runs)
 // and returns the fastest.
 vta_status tune_job(vta_tm_plan* P, int j, int* best) {
@@ -354,10 +371,12 @@ vta_status tune_job(vta_tm_plan* P, int j, int* best) {
     const int nc = rec ? 8 : 6;
     const int maxlen = *std::max_element(P->lens.begin(), P->lens.end());
     float best_ms = 1e30f;
-    *best = cand[0];
     vta_status s = VTA_OK;
+    int tried = 0;
     for (int i = 0; i < nc && s == VTA_OK; ++i) {
-        if (i > 0 && cand[i - 1] >= maxlen) break;  // one chunk per series already
+        if (tried && cand[i - 1] >= maxlen) break;  // one chunk per series already
+        if (!chunk_fits(P, P->jobs[j], cand[i])) continue;
+        if (!tried++) *best = cand[i];
         s = plan_states(P, j, cand[i]);
         if (s == VTA_OK) s = plan_items(P, {j});
         if (s == VTA_OK) s = plan_upload_jobs(P, {j});
@@ -468,6 +487,7 @@ vta_status plan_create(vta_ctx* ctx, const float* h, const float* l, const float
                 auto it = g_tune.find(key);
                 if (it != g_tune.end()) chunk = it->second;
             }
+            if (chunk && !chunk_fits(P, P->jobs[j], chunk)) chunk = safe_chunk(P->jobs[j]);
             if (chunk == 0) {
                 VTA_TRY(tune_job(P, (int)j, &chunk));
                 P->tuned = true;
