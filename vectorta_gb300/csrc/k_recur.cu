@@ -54,7 +54,32 @@ struct Acc {
     }
     __device__ float f() const { return hi + lo; }
     __device__ double d() const { return (double)hi + (double)lo; }
+    __device__ float mean(int p, float inv) const;  // pair_mean
 };
+
+__device__ __noinline__ float f64_mean(float2 sum, int p) { return (float)(((double)sum.x + (double)sum.y) / (double)p); }
+
+// sum / p from a compensated sum as f64 gives it, inv = 1 / p.  The residual of
+// the first quotient is exact by FMA, so q + c is the mean up to 2^-45 of it
+// (scaled where the residual of a small sum would underflow); where 2^-40 more
+// or less rounds alike, so does the mean, and only the others (ties of short
+// periods, one seed in 2^15) are divided in f64.  An f64 division in the chain
+// of every tile that holds a seed took RSI of 58 periods on 5,003 bars from 51
+// to 63 us.
+__device__ __forceinline__ float pair_mean(float2 sum, int p, float inv) {
+    const bool small = fabsf(sum.x) < 0x1p-40f;
+    const float k = small ? 0x1p80f : 1.f, hi = sum.x * k, lo = sum.y * k;
+    const float q = hi * inv, c = (fmaf(-q, (float)p, hi) + lo) * inv, eps = fabsf(q) * 0x1p-40f;
+    const float a = q + (c + eps), b = q + (c - eps);
+    const float m = a * (small ? 0x1p-80f : 1.f);
+    const bool sure = a == b && p < coef::kExact && (!small || fabsf(m) >= 0x1p-126f);
+    return sure ? m : f64_mean(sum, p);
+}
+
+__device__ __forceinline__ float Acc::mean(int p, float inv) const {
+    const float h = hi + lo;
+    return pair_mean(make_float2(h, lo - (h - hi)), p, inv);
+}
 
 // ------------------------------------------------------------ inputs -------
 struct InBatch {
@@ -482,7 +507,7 @@ struct OpWilders {
         wsum.zero();
     }
     template <class In> __device__ void accum(const In& in, int t) { wsum.add(in.X(t)); }
-    __device__ void seed() { y = (float)(wsum.d() * (1.0 / (double)p)); }
+    __device__ void seed() { y = wsum.mean(p, alpha); }
     template <class In> __device__ int step(const In& in, int t) {
         float v = in.X(t);
         y = (p == 1) ? v : fmaf(v - y, alpha, y);
@@ -1308,23 +1333,6 @@ __device__ __forceinline__ float2 pair_scan(float2 v) {  // inclusive over the w
 __device__ __forceinline__ float2 pair_shfl(float2 v, int src) {
     return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
-// sum / p from a compensated sum as f64 gives it, inv = 1 / p.  The residual of
-// the first quotient is exact by FMA, so q + c is the mean up to 2^-45 of it
-// (scaled where the residual of a small sum would underflow); where 2^-40 more
-// or less rounds alike, so does the mean, and only the others (ties of short
-// periods, one seed in 2^15) are divided in f64.  An f64 division in the chain
-// of every tile that holds a seed took RSI of 58 periods on 5,003 bars from 51
-// to 63 us.
-__device__ __forceinline__ float pair_mean(float2 sum, int p, float inv) {
-    const bool small = fabsf(sum.x) < 0x1p-40f;
-    const float k = small ? 0x1p80f : 1.f, hi = sum.x * k, lo = sum.y * k;
-    const float q = hi * inv, c = (fmaf(-q, (float)p, hi) + lo) * inv, eps = fabsf(q) * 0x1p-40f;
-    const float a = q + (c + eps), b = q + (c - eps);
-    const float m = a * (small ? 0x1p-80f : 1.f);
-    const bool sure = a == b && p < coef::kExact && (!small || fabsf(m) >= 0x1p-126f);
-    return sure ? m : (float)(((double)sum.x + (double)sum.y) / (double)p);
-}
-
 // The prefix of the terms over [f, c0) and whether every input of [f, tend) is
 // finite (whole warp)
 template <class Op>

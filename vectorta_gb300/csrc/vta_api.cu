@@ -1425,10 +1425,22 @@ static vta_status run_tm(vta_ctx* ctx, Ind ind, const DevIn& in, size_t cols, si
     // 18.5, 22.6, 26.6, 29.7, RSI(14) 41 / 24.6, 36.9 / 28.7, 36.9 / 34.8, 41 / 36.9,
     // ATR(14) of 100 series x 500, 760 and 1,000 rows 35.8 / 28.9, 33.7 / 34.4, 33.5 /
     // 38.9; 9,000 series x 500 rows: EMA 46 / 39, ATR 56.5 / 56.7.
-    const bool one = recur && ctx->policy.recur_chunk == 0 && R <= 640 && (C + 31) / 32 <= 2 * ctx->num_sms;
+    //
+    // One chunk, the emit pass alone, where the series fill the GPU without cutting
+    // their rows: from 8 warps of them per SM on, and from one on if the history is
+    // short or half of it is warm-up, which every chunk sums anew (one launch /
+    // three or one chunk: RSI(14) of 9,700 x 60 31 / 16, x 400 35 / 29, RSI(500) of
+    // 9,000 x 640 373 / 90, EMA(14) of 20,000 x 100 46 / 16, of 50,000 x 100 81 / 20, x
+    // 2,520 325 / 280; DEMA(200), which has no sums, 9,700 x 400 29 / 35).
+    const bool auto_chunk = recur && ctx->policy.recur_chunk == 0;
+    const int lane_warps = (C + 31) / 32, warm = ind == I_DEMA ? 0 : ind == I_TEMA ? 3 * std::min(p, R) : p;
+    const bool alone = auto_chunk && (lane_warps >= 8 * ctx->num_sms ||
+                                      (lane_warps > ctx->num_sms && (R <= (ind == I_DEMA ? 256 : 400) ||
+                                                                     (R <= 640 && 2LL * warm > R))));
+    const bool one = auto_chunk && !alone && R <= 640 && lane_warps <= 2 * ctx->num_sms;
     int chunk = 0, nch = 0;
     if (recur && !one) {
-        chunk = pick_chunk_tm(ctx, R, C);
+        chunk = alone ? ((R + 31) / 32) * 32 : pick_chunk_tm(ctx, R, C);
         nch = (R + chunk - 1) / chunk;
         ar.need((size_t)nch * cols * 16);
         ar.need((size_t)nch * cols * 16);
