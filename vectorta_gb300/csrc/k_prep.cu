@@ -18,12 +18,17 @@ constexpr int kScanItems = 8;
 constexpr int kScanBlock = kScanThreads * kScanItems;  // elements per block
 
 // First valid row per series: a block owns 32 series (a warp's lanes, so each
-// row is one 128-byte load) and its 32 warps examine 8 rows each, 256 rows a
+// row is one 128-byte load) and its warps examine 8 rows each, up to 256 rows a
 // round, until every series of the block is found.  Bound by memory latency: a
 // NaN lead of up to 256 rows costs one round trip (one thread per series, 16
 // rows a trip, took 22 us for 3,000 series with leads up to 250, 50 us over
-// high / low / close; now 3.6 and 5.7).
-constexpr int kFvWarps = 32, kFvRows = 8;
+// high / low / close; now 3.6 and 5.7).  Where the series alone fill the GPU, past
+// two blocks of 32 warps per SM, 4 warps: the rows behind short leads are read
+// for nothing (50,000 series x 250 rows, 32 warps / 4: ALMA(14) 73 / 62 us,
+// Donchian(14) 78 / 56).
+constexpr int kFvWarps = 32, kFvWideWarps = 4, kFvRows = 8;
+
+int first_valid_threads(int cols) { return 32 * (ceil_div(cols, 32) > 2u * kNumSMs ? kFvWideWarps : kFvWarps); }
 
 // ALL: c together with h and l (first), beside c alone (first_c, may be null).
 template <bool ALL>
@@ -31,12 +36,12 @@ __global__ void __launch_bounds__(32 * kFvWarps)
 k_first_valid_tm(const float* __restrict__ h, const float* __restrict__ l, const float* __restrict__ c, int cols,
                  int rows, const int* len, int* first, int* first_c, int* first_nan, int* first_big) {
     __shared__ int fa[32], fc[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, round = (blockDim.x >> 5) * kFvRows;
     const int s = blockIdx.x * 32 + lane;
     const int L = s < cols ? (len ? len[s] : rows) : 0;
     if (warp == 0) fa[lane] = fc[lane] = L;
     __syncthreads();
-    for (int t0 = 0;; t0 += kFvWarps * kFvRows) {
+    for (int t0 = 0;; t0 += round) {
         if (L - t0 > warp * kFvRows) {
             const int tb = t0 + warp * kFvRows, m = L - tb;  // m rows left
             float hv[kFvRows], lv[kFvRows], cv[kFvRows];
@@ -59,7 +64,7 @@ k_first_valid_tm(const float* __restrict__ h, const float* __restrict__ l, const
         }
         __syncthreads();
         // done once found or past the end (a round's finds are below the next one's)
-        const bool more = fa[lane] == L && L - t0 > kFvWarps * kFvRows;
+        const bool more = fa[lane] == L && L - t0 > round;
         if (!__syncthreads_or(more)) break;
     }
     if (warp == 0 && s < cols) {
@@ -219,7 +224,7 @@ __global__ void k_prefix_apply(const float* __restrict__ x, int n, int first, in
 
 vta_status launch_first_valid_tm(const float* x_tm, int cols, int rows, int* first, cudaStream_t st,
                                  int* first_nan, int* first_big, float limit) {
-    k_first_valid_tm<false><<<ceil_div(cols, 32), 32 * kFvWarps, 0, st>>>(nullptr, nullptr, x_tm, cols, rows, nullptr,
+    k_first_valid_tm<false><<<ceil_div(cols, 32), first_valid_threads(cols), 0, st>>>(nullptr, nullptr, x_tm, cols, rows, nullptr,
                                                                          first, nullptr, first_nan, first_big);
     VTA_TRY(check_launch("k_first_valid_tm"));
     if (!first_nan) return VTA_OK;
@@ -231,7 +236,7 @@ vta_status launch_first_valid_tm(const float* x_tm, int cols, int rows, int* fir
 
 vta_status launch_first_valid_tm_hlc(const float* h, const float* l, const float* c, int cols,
                                      int rows, int* first, cudaStream_t st, const int* len, int* first_c) {
-    k_first_valid_tm<true><<<ceil_div(cols, 32), 32 * kFvWarps, 0, st>>>(h, l, c, cols, rows, len, first, first_c,
+    k_first_valid_tm<true><<<ceil_div(cols, 32), first_valid_threads(cols), 0, st>>>(h, l, c, cols, rows, len, first, first_c,
                                                                         nullptr, nullptr);
     return check_launch("k_first_valid_tm_hlc");
 }
