@@ -77,8 +77,8 @@ __device__ __forceinline__ float pair_mean(float2 sum, int p, float inv) {
 }
 
 __device__ __forceinline__ float Acc::mean(int p, float inv) const {
-    const float h = hi + lo;
-    return pair_mean(make_float2(h, lo - (h - hi)), p, inv);
+    const float h = hi + lo, e = lo - (h - hi);
+    return pair_mean(make_float2(h, isfinite(e) ? e : 0.f), p, inv);  // (an infinite sum is its own mean)
 }
 
 // ------------------------------------------------------------ inputs -------
