@@ -1954,6 +1954,23 @@ __device__ void trans_pow(long long n, int p, D2 (&m)[Op::NS][Op::NS]) {
     }
 }
 
+// Ops whose state, once infinite, stays infinite (many-series RSI: an infinite
+// move; the batch form turns it into NaN).  A product of float pairs would make
+// it NaN, so the composition leaves infinite records out and holds, per
+// component, whether one has passed.
+template <class Op> struct InfHeld { static constexpr bool v = false; };
+template <> struct InfHeld<OpRsi<false>> { static constexpr bool v = true; };
+__device__ __forceinline__ unsigned take_inf(float4& g) {
+    const bool x = isinf(g.x), y = isinf(g.y);
+    if (x) g.x = 0.f;
+    if (y) g.y = 0.f;
+    return (x ? 1u : 0u) | (y ? 2u : 0u);
+}
+__device__ __forceinline__ void put_inf(float4& cv, unsigned held) {
+    if (held & 1u) cv.x = INFINITY;
+    if (held & 2u) cv.y = INFINITY;
+}
+
 // The map of one chunk from its AGG record (state, applied steps or marker).
 template <class Op>
 __device__ void chunk_map(const float4 g, int p, int chunk, const D2 (&ml)[Op::NS][Op::NS], AffD<Op::NS>& a) {
@@ -2061,13 +2078,15 @@ __global__ void k_recur_carry(RecurArgs a, int n_chunks) {
     const float4 kNone = make_float4(0.f, 0.f, 0.f, 0.f);
     auto rec = [&](int k) { return k < k1 ? __ldg(agg + (size_t)k * a.n_lanes + li) : kNone; };
     float4 q0 = rec(k0), q1 = rec(k0 + 1), q2 = rec(k0 + 2), q3 = rec(k0 + 3);
+    unsigned held = 0;
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
-        const float4 g = q0;
+        float4 g = q0;
         q0 = q1;
         q1 = q2;
         q2 = q3;
         q3 = rec(k + 4);
+        if (InfHeld<Op>::v) held |= take_inf(g);
         if (g.w == full) {
             full_step(run.b, g);
             ++cnt;
@@ -2080,6 +2099,11 @@ __global__ void k_recur_carry(RecurArgs a, int n_chunks) {
         }
     }
     flush();
+    if (InfHeld<Op>::v) {  // what the threads before this one hold
+        const unsigned below = (1u << lane) - 1u;
+        const bool x = __ballot_sync(0xffffffffu, held & 1u) & below, y = __ballot_sync(0xffffffffu, held & 2u) & below;
+        held = (x ? 1u : 0u) | (y ? 2u : 0u);
+    }
 #pragma unroll 1
     for (int d = 1; d < 32; d <<= 1) {
         const AffD<N> up = affd_shfl_up<N, SH>(run, d);
@@ -2096,7 +2120,7 @@ __global__ void k_recur_carry(RecurArgs a, int n_chunks) {
     q3 = rec(k0 + 3);
 #pragma unroll 1
     for (int k = k0; k < k1; ++k) {
-        const float4 g = q0;
+        float4 g = q0;
         q0 = q1;
         q1 = q2;
         q2 = q3;
@@ -2106,6 +2130,10 @@ __global__ void k_recur_carry(RecurArgs a, int n_chunks) {
             cv.x = S[0].hi + S[0].lo;
             if (N > 1) cv.y = S[N > 1 ? 1 : 0].hi + S[N > 1 ? 1 : 0].lo;
             if (N > 2) cv.z = S[N > 2 ? 2 : 0].hi + S[N > 2 ? 2 : 0].lo;
+            if (InfHeld<Op>::v) {
+                put_inf(cv, held);
+                held |= take_inf(g);
+            }
             carry[(size_t)k * a.n_lanes + li] = cv;
             if (g.w == full) {
                 full_step(S, g);
@@ -2151,10 +2179,12 @@ __device__ __forceinline__ float4 entry_state(const float4* rec, int q, int lane
     D2 S[N];
 #pragma unroll
     for (int r = 0; r < N; ++r) S[r] = {0.f, 0.f};
+    unsigned held = 0;
 #pragma unroll 1
     for (int k = 0; k < q; ++k) {
-        const float4 e = rec[k * 32 + lane];
+        float4 e = rec[k * 32 + lane];
         if (e.w == kBeforeSeed) continue;
+        if (InfHeld<Op>::v) held |= take_inf(e);
         AffD<N> m;
         chunk_map<Op>(e, p, chunk, ml, m);
         D2 t[N];
@@ -2173,6 +2203,7 @@ __device__ __forceinline__ float4 entry_state(const float4* rec, int q, int lane
     cv.x = S[0].hi + S[0].lo;
     if (N > 1) cv.y = S[N > 1 ? 1 : 0].hi + S[N > 1 ? 1 : 0].lo;
     if (N > 2) cv.z = S[N > 2 ? 2 : 0].hi + S[N > 2 ? 2 : 0].lo;
+    if (InfHeld<Op>::v) put_inf(cv, held);
     return cv;
 }
 
