@@ -1,5 +1,6 @@
-"""Weighted windows of thousands of bars: around the lengths up to which a
-preparation block stages four weight rows (7,232), and up to the longest strip
+"""Weighted windows of thousands of bars: around the lengths whose preparation
+fits the shared memory of a plain launch (1,504), up to which a block stages
+four weight rows (7,232), and up to the longest strip
 (28,656), against the oracle; longer ones are refused and leave no error behind.
 
 Tolerance: with S the series' span, the values centred on a tile's reference lie
@@ -19,7 +20,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("name", ["alma", "wma", "srwma"])
-@pytest.mark.parametrize("rng", [(3384, 3400, 8), (7232, 7312, 16), (5, 12005, 3000), (28000, 28656, 656)],
+@pytest.mark.parametrize("rng", [(1488, 1552, 8), (3384, 3400, 8), (7232, 7312, 16), (5, 12005, 3000), (28000, 28656, 656)],
                          ids=lambda r: f"{r[0]}-{r[1]}")
 def test_long_windows(name, rng):
     x = datagen.random_walk(29_500, seed=4, nan_lead=3).astype(np.float32)

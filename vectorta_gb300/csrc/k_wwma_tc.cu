@@ -920,7 +920,7 @@ vta_status launch_wwma_batch_tc(const WwmaBatchArgs& a, int variant, vta_ctx* ct
                (int)ceil_div(rows, per_block), kbig, per_block, perm ? 1 : 0};
     StripArgs sa{a.x, a.n, a.first, kbig, jmax, step, d_sh, d_sl, d_ref, d_xs, d_tnan, d_nbits};
     auto prep = variant == 1 ? k_wwma_prep<1> : k_wwma_prep<0>;
-    if (psmem > 48 * 1024)
+    if (psmem + kPrepStatic > 48 * 1024)
         VTA_CUDA_TRY(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem));
     prep<<<ra.blocks + n_time_tiles, kPrepThreads, psmem, st>>>(ra, sa, rows);
     VTA_TRY(check_launch("k_wwma_prep"));
