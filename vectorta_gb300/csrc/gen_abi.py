@@ -242,7 +242,10 @@ vta_status vta_ma_select_into_host_f32(vta_ctx* ctx, const char* ma_type, const 
  * Inputs: one series in a (b, c NULL); Donchian (high, low) in (a, b); ATR,
  * WillR, ADX, SuperTrend (high, low, close).  Outputs: out holds n_outputs
  * rows of n_streams values: Bollinger and Donchian upper / middle / lower,
- * SuperTrend trend / changed. */
+ * SuperTrend trend / changed.
+ * Both updates return when theirs is done: the device one too waits for the
+ * context's stream, unlike the batch calls on device pointers, so that its
+ * outputs may be read from any stream. */
 typedef struct vta_streams vta_streams;
 vta_status vta_streams_create(vta_ctx* ctx, const char* indicator, const char* const* param_keys,
     const double* param_values, size_t n_params, size_t n_streams, vta_streams** out);
